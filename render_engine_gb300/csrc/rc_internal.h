@@ -18,11 +18,17 @@ struct DState {
     const int* dims;           // nu, nv per quad
     const int* off;            // first point of each quad
     const float4* tri;         // dynamic triangles, 3 float4 each (v0 + quad id bits, e1, e2)
-    const float4* grp;         // plane-culling groups, 3 float4 each, then the pair records (grp_float4s)
+    const float4* grp;         // plane-culling groups, 3 float4 each, then the pair, box and quad records (grp_float4s)
     const int* misc;           // dynamic triangles outside any group (always tested exactly)
     const float* ref;          // converged reference per point (scenes with references)
     const uint8_t* valid;
     int nt, ng, nmisc;
+    int nbox;                  // boxes that the groups are sides of, besides the enclosing one (an even
+                               // number, the last may be empty); -1 = the plane filter alone
+    int outer;                 // 1: an enclosing box
+    int nquad;                 // quad records (0 = none)
+    float box_scale;           // largest coordinate of an origin that the box margins cover
+    float box_m;               // the boxes' margin
     GroupRanges gr;
 };
 
@@ -208,10 +214,23 @@ inline bool supported_nl_nw(int NL, int NW) {
 #define X(n) extern template struct Ops<n>;
 RC_NL_VALUES(X)
 #undef X
-// The group buffer: 3 float4 per group, then 3 float4 per pair of groups (pass-1 records).
-__host__ __device__ inline int grp_float4s(int ng) { return 3 * ng + 3 * (ng / 2); }
+// The group buffer: 3 float4 per group, 3 float4 per pair of groups (pass-1 records); with boxes,
+// their slabs (2 float4 of the enclosing box, 3 per pair of the others), their planes (2 float4
+// each, the enclosing box last) and 3 float4 per group (the rectangles); 2 float4 per quad.
+constexpr int MAX_BOXES = 32;
+__host__ __device__ inline int box_float4s(const DState& s) {
+    return s.nbox < 0 ? 0 : 2 * s.outer + 3 * (s.nbox / 2) + 2 * (s.nbox + s.outer);
+}
+__host__ __device__ inline int grp_float4s(const DState& s) {
+    return 3 * s.ng + 3 * (s.ng / 2) + box_float4s(s) + (s.nbox < 0 ? 0 : 3 * s.ng) + 2 * s.nquad;
+}
+// What a block stages of it (stage_smem), and the triangles beside it.
+__host__ __device__ inline int staged_rec(const DState& s) {
+    return s.nbox < 0 ? grp_float4s(s) : box_float4s(s) + 3 * s.ng + 2 * s.nquad;
+}
+__host__ __device__ inline int staged_tri(const DState& s) { return s.nbox < 0 ? 3 * s.nt : 0; }
 __host__ __device__ inline size_t frame_smem_bytes(const DState& s) {
-    return sizeof(float4) * (3 * (size_t)s.nt + (size_t)grp_float4s(s.ng)) + sizeof(int) * (size_t)s.nmisc + 16;
+    return sizeof(float4) * (size_t)(staged_rec(s) + staged_tri(s)) + (s.nbox < 0 ? sizeof(int) * (size_t)s.nmisc : 0) + 16;
 }
 __host__ __device__ constexpr int lcs_of(int NL) { return (NL + 3) / 4 * 4; }
 __host__ __device__ constexpr int aes_of(int NL) { return (NL + 1 + 3) / 4 * 4; }

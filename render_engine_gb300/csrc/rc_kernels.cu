@@ -5,9 +5,9 @@
 //  * a frame without verification, projection or DDGI is ONE kernel: trace + blend +
 //    history + Sum 1/(n+1) + error sums, so the per-point rays' result never goes through
 //    HBM (the reference writes kk and m, then k_update reads them back);
-//  * dynamic triangles are culled by a plane filter over axis-aligned rectangles before the
-//    exact Möller-Trumbore test; the exact test runs only on the few rectangles that can
-//    hold the closest hit, so hit ids and distances are those of the reference's full scan;
+//  * dynamic triangles are culled by slab tests of the boxes that they are sides of (or by a plane
+//    filter over axis-aligned rectangles) before the exact test; the exact test runs only on
+//    what can hold the closest hit, so hit ids and distances are those of the reference's full scan;
 //  * per-point gathers at the hit point are 16-byte vectors (albedo + direct light in one
 //    record, the cache padded to 4 lights);
 //  * reductions are order-free or fixed-order (Sum 1/(n+1) exactly in 64-bit fixed point,
@@ -205,7 +205,9 @@ __device__ __forceinline__ void proj_region_add(float* __restrict__ neq, int rg,
 struct TraceSmem {
     const float4* tri;
     const float4* grp;
-    const float4* gpair;   // pass-1 records, 3 float4 per pair of groups
+    const float4* box;     // the boxes' slabs and planes (box_float4s)
+    const float4* rect;    // 3 float4 per group, for trace_boxes
+    const float4* quad;    // 2 float4 per quad (resolve_hit)
     const int* misc;
 };
 
@@ -250,15 +252,17 @@ __device__ __forceinline__ void filter_axis(const float4* __restrict__ gp, int a
 }
 
 template <typename MaskT>
-__device__ __forceinline__ void trace_groups(const TraceSmem& sm, const DState& s, f3 o, f3 d, float& tmin, int& q, int& jb) {
+__device__ __forceinline__ void trace_groups(const float4* __restrict__ tri, const float4* __restrict__ grp, int ng, GroupRanges gr, f3 o,
+                                             f3 d, float& tmin, int& q, int& jb) {
+    const float4* gpair = grp + 3 * ng;
     // pass 1: bit ng - 1 - g of mask <=> group g is a candidate
     MaskT mask = 0;
     const float idx = __fdividef(1.f, d.x), idy = __fdividef(1.f, d.y), idz = __fdividef(1.f, d.z);
-    filter_axis(sm.gpair, s.gr.g0[0], s.gr.g0[1], o.x, idx, o.y, d.y, o.z, d.z, mask);
-    filter_axis(sm.gpair, s.gr.g0[1], s.gr.g0[2], o.y, idy, o.x, d.x, o.z, d.z, mask);
-    filter_axis(sm.gpair, s.gr.g0[2], s.gr.g0[3], o.z, idz, o.x, d.x, o.y, d.y, mask);
+    filter_axis(gpair, gr.g0[0], gr.g0[1], o.x, idx, o.y, d.y, o.z, d.z, mask);
+    filter_axis(gpair, gr.g0[1], gr.g0[2], o.y, idy, o.x, d.x, o.z, d.z, mask);
+    filter_axis(gpair, gr.g0[2], gr.g0[3], o.z, idz, o.x, d.x, o.y, d.y, mask);
     // pass 2: candidates nearest first, exact test, stop past the best hit plus the slack
-    const int top = s.ng - 1;
+    const int top = ng - 1;
     float thr = tmin * 1.0001f + 1e-5f;
     while (mask) {
         float best = __int_as_float(0x7f800000);
@@ -266,48 +270,214 @@ __device__ __forceinline__ void trace_groups(const TraceSmem& sm, const DState& 
         for (MaskT m = mask; m; m &= m - 1) {
             const int b = sizeof(MaskT) == 8 ? __ffsll((long long)m) - 1 : __ffs((int)m) - 1;
             const int g = top - b;
-            const float ok = g < s.gr.g0[1] ? o.x : (g < s.gr.g0[2] ? o.y : o.z);
-            const float idk = g < s.gr.g0[1] ? idx : (g < s.gr.g0[2] ? idy : idz);
-            const float tk = (sm.grp[3 * g].x - ok) * idk;
+            const float ok = g < gr.g0[1] ? o.x : (g < gr.g0[2] ? o.y : o.z);
+            const float idk = g < gr.g0[1] ? idx : (g < gr.g0[2] ? idy : idz);
+            const float tk = (grp[3 * g].x - ok) * idk;
             if (tk < best) { best = tk; bb = b; }
         }
         if (!(best <= thr)) break;
         mask &= ~((MaskT)1 << bb);
         const int g = top - bb;
-        const float4 G1 = sm.grp[3 * g + 1];
+        const float4 G1 = grp[3 * g + 1];
         int j = __float_as_int(G1.y), jend = j + __float_as_int(G1.z);
         if (jend - j == 2) {
             // exact test on the triangle whose side of the diagonal holds the crossing (both
             // within eps of the diagonal): the other one cannot hold the hit
-            const float4 GL = sm.grp[3 * g + 2];
-            const bool ax0 = g < s.gr.g0[1], ax1 = !ax0 && g < s.gr.g0[2];
+            const float4 GL = grp[3 * g + 2];
+            const bool ax0 = g < gr.g0[1], ax1 = !ax0 && g < gr.g0[2];
             const float oa = ax0 ? o.y : o.x, da = ax0 ? d.y : d.x;
             const float ob = ax0 || ax1 ? o.z : o.y, db = ax0 || ax1 ? d.z : d.y;
             const float sd = GL.x * (oa + best * da) + GL.y * (ob + best * db) + GL.z;
             if (sd > GL.w) jend = j + 1;
             else if (sd < -GL.w) j = j + 1;
         }
-        for (; j < jend; ++j) mt_tri(sm.tri, j, o, d, tmin, q, jb);
+        for (; j < jend; ++j) mt_tri(tri, j, o, d, tmin, q, jb);
         thr = tmin * 1.0001f + 1e-5f;
     }
 }
 
+__device__ __forceinline__ float median3(float a, float b, float c) { return fmaxf(fminf(a, b), fminf(fmaxf(a, b), c)); }
+
+// Closest hit of a state whose groups are sides of axis-aligned boxes (build_boxes in
+// rc_runtime.cu): an enclosing box that the origin lies in, and boxes (a lone rectangle is one of
+// no thickness) that the ray enters from outside, or leaves when it starts in one.
+//
+// A slab test of every box, two boxes at once in paired FP32, gives the nearest one's entry
+// distance, and one face of it (or the enclosing box's exit face) is the only candidate.  Its
+// distance is the reference's own Moeller-Trumbore value: for a rectangle whose edges lie along
+// the axes every cross and dot product has one term, so both its triangles give
+//     t = (e2 * (e1 * (o_k - c))) * (1 / (e1 * (d_k * e2)))
+// with those roundings, and their u, v tests hold when the crossing lies inside the rectangle and
+// off its diagonal by a margin m.  The answer stands only when it is certain: inside by m, ahead,
+// |det| > 1e-9, t > 1e-4, and every other surface's distance bound beyond the hit by 1e-5 of it +
+// 2e-6.  m = 1e-5 + 2e-6 x the largest coordinate is over ten times the rounding of a crossing
+// point, and the slack twenty times that of a distance.  The slabs of the boxes are grown by m (the
+// enclosing one's shrunk), so a box that its slab misses holds no hit, and a slab's distance is a
+// lower bound however grazing the ray.  A component of d that is zero gives NaN slabs, which the
+// minima and maxima leave out: a bound that is too low.  Anything uncertain (rays within m of an
+// edge or a diagonal, origins in two boxes or within m of one: below 1e-4 of a room's rays)
+// returns false, and the full scan decides.
+//
+// Bound by instruction issue (min / max on the half-rate ALU pipe), so it replaces tests by fewer:
+// a box takes about 16 instructions where its five or six faces took 15 each in the plane filter,
+// and the one exact test 45 instead of 240.  17.3 M rays of a room of 31 rectangles (k_frozen):
+// 486 us with the plane filter, 297 us; a fused frame of 1,082,802 points: 63.1 -> 48.2 us, with
+// tracking 89.0 -> 76.5 us.  The slabs pack (x, y) of one box and z of two, 12 registers of ray
+// constants; packed by axis over two boxes (18 registers) the frame took 8 % longer.
+__device__ __forceinline__ bool trace_boxes(const TraceSmem& sm, const DState& s, f3 o, f3 d, float& tmin, int& q) {
+    const float inf = __int_as_float(0x7f800000);
+    const float ix = __fdividef(1.f, d.x), iy = __fdividef(1.f, d.y), iz = __fdividef(1.f, d.z);
+    const float mx = -o.x * ix, my = -o.y * iy, mz = -o.z * iz;
+    const float ax = fabsf(ix), ay = fabsf(iy), az = fabsf(iz);
+    const float4* rec = sm.box;
+    float room = inf;              // exit distance of the enclosing box
+    if (s.outer) {
+        const float4 R0 = rec[0];
+        const float2 R1 = *reinterpret_cast<const float2*>(rec + 1);
+        const float cx = fmaf(R0.x, ix, mx), cy = fmaf(R0.y, iy, my), cz = fmaf(R0.z, iz, mz);
+        // every plane that the ray enters by lies behind: none of those faces can be hit
+        if (!(fmaxf(fmaxf(fmaf(-R0.w, ax, cx), fmaf(-R1.x, ay, cy)), fmaf(-R1.y, az, cz)) <= 5e-5f)) return false;
+        room = fminf(fminf(fmaf(R0.w, ax, cx), fmaf(R1.x, ay, cy)), fmaf(R1.y, az, cz));
+        rec += 2;
+    } else if (!(fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z)) <= s.box_scale)) {
+        return false;
+    }
+    // the two smallest entry distances of the grown boxes, the box's number in the low 5 bits (the
+    // distance is lowered by at most 4e-6 of itself, raised by as much; far below the slack)
+    constexpr unsigned MISS = 0x7f000000u;
+    unsigned k1 = MISS, k2 = MISS;
+    {
+        const float2 i2 = make_float2(ix, iy), m2 = make_float2(mx, my), a2 = make_float2(ax, ay), n2 = make_float2(-ax, -ay);
+        const float2 iz2 = make_float2(iz, iz), mz2 = make_float2(mz, mz), az2 = make_float2(az, az), nz2 = make_float2(-az, -az);
+        auto visit = [&](float nx, float ny, float nz, float fx, float fy, float fz, unsigned b) {
+            const float key = fmaxf(fmaxf(fmaxf(nx, ny), nz), 0.f);
+            const float out = fminf(fminf(fx, fy), fz);
+            const unsigned k = key <= out ? (__float_as_uint(key) & ~31u) | b : MISS;
+            k2 = min(k2, max(k1, k));
+            k1 = min(k1, k);
+        };
+        for (int b = 0; b < s.nbox; b += 2, rec += 3) {
+            // boxes b and b + 1: (centre x, y of each) (centre z of each, half x, y of b) (half x, y of b + 1, half z of each)
+            const float4 C0 = rec[0], C1 = rec[1], C2 = rec[2];
+            const float2 h0 = make_float2(C1.z, C1.w), h1 = make_float2(C2.x, C2.y), hz = make_float2(C2.z, C2.w);
+            const float2 c0 = __ffma2_rn(make_float2(C0.x, C0.y), i2, m2), c1 = __ffma2_rn(make_float2(C0.z, C0.w), i2, m2);
+            const float2 cz = __ffma2_rn(make_float2(C1.x, C1.y), iz2, mz2);
+            const float2 f0 = __ffma2_rn(h0, a2, c0), f1 = __ffma2_rn(h1, a2, c1), fz = __ffma2_rn(hz, az2, cz);
+            const float2 q0 = __ffma2_rn(h0, n2, c0), q1 = __ffma2_rn(h1, n2, c1), qz = __ffma2_rn(hz, nz2, cz);
+            visit(q0.x, q0.y, qz.x, f0.x, f0.y, fz.x, (unsigned)b);
+            visit(q1.x, q1.y, qz.y, f1.x, f1.y, fz.y, (unsigned)b + 1u);
+        }
+    }
+    const float near1 = __uint_as_float(k1);
+    const bool solid = k1 < MISS && near1 < room;
+    if (!solid && !s.outer) return true;   // no box ahead
+    // the candidate's planes: where the ray enters it, or leaves it when it starts inside
+    const float4* pick = rec + 2 * (solid ? (int)(k1 & 31u) : s.nbox);
+    const float4 T0 = pick[0], T1 = pick[1];
+    const float tx0 = (T0.x - o.x) * ix, tx1 = (T0.y - o.x) * ix, ty0 = (T0.z - o.y) * iy, ty1 = (T0.w - o.y) * iy;
+    const float tz0 = (T1.x - o.z) * iz, tz1 = (T1.y - o.z) * iz;
+    const float nx = fminf(tx0, tx1), ny = fminf(ty0, ty1), nz = fminf(tz0, tz1);
+    const float fx = fmaxf(tx0, tx1), fy = fmaxf(ty0, ty1), fz = fmaxf(tz0, tz1);
+    const float tin = fmaxf(fmaxf(nx, ny), nz), tout = fminf(fminf(fx, fy), fz);
+    const bool inside = tin <= 5e-5f;
+    const float at = inside ? tout : tin;
+    const float ex = inside ? fx : nx, ey = inside ? fy : ny, ez = inside ? fz : nz;
+    const float second = median3(ex, ey, ez);
+    const int axis = ex == at ? 0 : (ey == at ? 1 : 2);
+    const float ok = axis == 0 ? o.x : (axis == 1 ? o.y : o.z), dk = axis == 0 ? d.x : (axis == 1 ? d.y : d.z);
+    const int face = 2 * axis + ((dk > 0.f) == inside ? 1 : 0);
+    const unsigned w1 = __float_as_uint(T1.w);
+    const int g = (int)((face < 4 ? __float_as_uint(T1.z) : w1) >> (8 * (face & 3))) & 0xff;
+    // the other surfaces: the next box, the enclosing one, this one's other faces
+    float bound = fminf(__uint_as_float(solid ? k2 : k1), solid ? room : inf);
+    bool sure = g != 0xff;
+    if (inside) {
+        bound = fminf(bound, second);
+    } else if (!(w1 >> 16 & 1u)) {      // not a lone rectangle: its exit, and the entry's edge
+        bound = fminf(bound, tout);
+        sure = sure && (tin - second) * fabsf(dk) > s.box_m;
+    }
+    if (!sure) return false;
+    const float4 F0 = sm.rect[3 * g], F1 = sm.rect[3 * g + 1], F2 = sm.rect[3 * g + 2];
+    const float pa = fmaf(at, axis == 0 ? d.y : d.x, axis == 0 ? o.y : o.x);
+    const float pb = fmaf(at, axis == 2 ? d.y : d.z, axis == 2 ? o.y : o.z);
+    const float det = fabsf(__fmul_rn(F0.y, __fmul_rn(dk, F0.z)));
+    const float num = fabsf(__fmul_rn(F0.z, __fmul_rn(F0.y, __fsub_rn(ok, F0.x))));
+    const float t = __fmul_rn(num, __frcp_rn(det));
+    const float side = fabsf(fmaf(F2.x, pa, fmaf(F2.y, pb, F2.z)));
+    if (fabsf(pa - F1.x) < F1.y && fabsf(pb - F1.z) < F1.w && side > s.box_m && det > 1e-9f && at > 0.f && t > 1e-4f &&
+        t * 1.00001f + 2e-6f < bound) {
+        tmin = t;
+        q = __float_as_int(F0.w);
+        return true;
+    }
+    return false;
+}
+
+// The full in-order scan for the lanes of `need`, one after another, by all the lanes of `act` (the
+// lanes that reached the call together): each tests every popc(act)-th triangle, and the smallest
+// distance, then the smallest index at that distance, is the scan's answer.  One such ray costs its
+// warp about 200 instructions; on its own lane, through the plane filter, it made the warp the
+// last of a small frame by 8 us (10,728 points: 20 us instead of 12).
+static __device__ __forceinline__ float2 scan_lanes(const float4* __restrict__ tri, int nt, unsigned act, unsigned need, f3 o, f3 d, float tmin,
+                                                 int q) {
+    const unsigned lane = threadIdx.x & 31u;
+    const int rank = __popc(act & ((1u << lane) - 1u)), n = __popc(act);
+    while (need) {
+        const int src = __ffs(need) - 1;
+        need &= need - 1u;
+        const f3 so = mk(__shfl_sync(act, o.x, src), __shfl_sync(act, o.y, src), __shfl_sync(act, o.z, src));
+        const f3 sd = mk(__shfl_sync(act, d.x, src), __shfl_sync(act, d.y, src), __shfl_sync(act, d.z, src));
+        float t = __int_as_float(0x7f800000);
+        int tq = -1, j1 = 0x7fffffff;
+        for (int j = rank; j < nt; j += n) mt_tri(tri, j, so, sd, t, tq, j1);
+        const unsigned best = __reduce_min_sync(act, __float_as_uint(t));
+        const unsigned at = __reduce_min_sync(act, __float_as_uint(t) == best ? (unsigned)j1 : 0x7fffffffu);
+        if ((int)lane == src) {
+            tmin = __uint_as_float(best);
+            q = at == 0x7fffffffu ? -1 : __float_as_int(tri[3 * at].w);
+        }
+    }
+    return make_float2(tmin, __int_as_float(q));
+}
+
+// The plane filter over all groups, and the triangles outside any.
+static __device__ __forceinline__ float2 trace_filter(const float4* tri, const float4* grp, const int* misc, int ng, int nmisc, GroupRanges gr,
+                                                   f3 o, f3 d) {
+    float tmin = __int_as_float(0x7f800000);
+    int q = -1, jb = 0x7fffffff;
+    for (int k = 0; k < nmisc; ++k) mt_tri(tri, misc[k], o, d, tmin, q, jb);
+    if (ng <= 32) trace_groups<unsigned>(tri, grp, ng, gr, o, d, tmin, q, jb);
+    else trace_groups<unsigned long long>(tri, grp, ng, gr, o, d, tmin, q, jb);
+    return make_float2(tmin, __int_as_float(q));
+}
+
 // Closest dynamic-triangle hit, equal to the reference's in-order scan (poc_gpu.cu:199-220).
-// Pass 1 marks the groups whose plane crossing falls in their outer box; pass 2 visits the
-// marked groups nearest first, runs the exact Möller-Trumbore on their triangles, and stops
-// once the next crossing lies beyond the best exact hit by more than the filter's error.
-__device__ __forceinline__ void trace_dyn(const TraceSmem& sm, const DState& s, bool brute, f3 o, f3 d, float& tmin, int& q,
-                                          int& jb) {
+// States made of boxes go through trace_boxes, and the few rays that it cannot decide through the
+// scan itself.  The plane filter takes other states: pass 1 marks the groups whose plane crossing
+// falls in their outer box; pass 2 visits the marked groups nearest first, runs the exact
+// Möller-Trumbore on their triangles, and stops once the next crossing lies beyond the best exact
+// hit by more than the filter's error.
+__device__ __forceinline__ void trace_dyn(const TraceSmem& sm, const DState& s, bool brute, f3 o, f3 d, float& tmin, int& q) {
     tmin = __int_as_float(0x7f800000);
     q = -1;
-    jb = 0x7fffffff;
     if (brute || s.ng == 0) {
+        int jb = 0x7fffffff;
         for (int j = 0; j < s.nt; ++j) mt_tri(sm.tri, j, o, d, tmin, q, jb);
         return;
     }
-    for (int k = 0; k < s.nmisc; ++k) mt_tri(sm.tri, sm.misc[k], o, d, tmin, q, jb);
-    if (s.ng <= 32) trace_groups<unsigned>(sm, s, o, d, tmin, q, jb);
-    else trace_groups<unsigned long long>(sm, s, o, d, tmin, q, jb);
+    float2 r;
+    if (s.nbox >= 0) {
+        const bool ok = trace_boxes(sm, s, o, d, tmin, q);
+        const unsigned act = __activemask();
+        const unsigned need = __ballot_sync(act, !ok);
+        if (need == 0u) return;
+        r = scan_lanes(s.tri, s.nt, act, need, o, d, tmin, q);
+    } else {
+        r = trace_filter(sm.tri, sm.grp, sm.misc, s.ng, s.nmisc, s.gr, o, d);
+    }
+    tmin = r.x;
+    q = __float_as_int(r.y);
 }
 
 // poc_gpu.cu:288-295.  fs scales the exit distance: 1 reproduces the reference exactly (a
@@ -463,15 +633,26 @@ __device__ __forceinline__ void trace_bvh(const DStatic& g, f3 o, f3 d, float& t
 }
 
 // poc_gpu.cu:239-246
-__device__ __forceinline__ int point_index(const DState& s, f3 H, int q) {
-    const float* Q = s.Q + 12 * q;
+static __device__ __forceinline__ int point_index(const float* __restrict__ quads, const int* __restrict__ dims, const int* __restrict__ off,
+                                               f3 H, int q) {
+    const float* Q = quads + 12 * q;
     f3 o = mk(__ldg(Q), __ldg(Q + 1), __ldg(Q + 2)), u = mk(__ldg(Q + 3), __ldg(Q + 4), __ldg(Q + 5));
     f3 v = mk(__ldg(Q + 6), __ldg(Q + 7), __ldg(Q + 8));
     f3 dd = H - o;
     float a = dot(dd, u) / dot(u, u), b = dot(dd, v) / dot(v, v);
-    int nu = __ldg(s.dims + 2 * q), nv = __ldg(s.dims + 2 * q + 1);
+    int nu = __ldg(dims + 2 * q), nv = __ldg(dims + 2 * q + 1);
     int iu = min(max(int(a * nu), 0), nu - 1), iv = min(max(int(b * nv), 0), nv - 1);
-    return __ldg(s.off + q) + iv * nu + iu;
+    return __ldg(off + q) + iv * nu + iu;
+}
+// One axis of point_index for an edge along one coordinate (u has a single component u_k):
+// int(dd_k u_k / u_k^2 * nu) from qf = dd_k * s, s = nu / u_k rounded.  The reference's value carries
+// four roundings and qf two, so they differ by at most 3.6e-7 relative; where qf is at least 1e-6
+// of its size from an integer (or below one, where both truncate to 0), truncating it gives the
+// same index.  `ok` is false where it is not, or not a number.
+__device__ __forceinline__ int cell_axis(float x, float o, float s, int n, bool& ok) {
+    const float qf = (x - o) * s;
+    ok = ok && (fabsf(qf - rintf(qf)) > 1e-6f * fabsf(qf) || fabsf(qf) < 0.5f);
+    return min(max(int(qf), 0), n - 1);
 }
 // poc_gpu.cu:263-287
 __device__ __forceinline__ int hash_find(const DStatic& g, unsigned long long key) {
@@ -509,12 +690,29 @@ struct Hit {
 
 // The cache point a traced ray reached (poc_gpu.cu:345-358, 466-469): with h.t and h.q set,
 // fills the hit point, the point index and whether the hit counts.
-__device__ __forceinline__ void resolve_hit(const DState& s, const DStatic& g, const Grid& grid, f3 O, f3 D, int i, Hit& h) {
+// The point index of a quad whose edges and normal lie along the axes comes from its record in
+// shared memory (two 16-byte loads and no division) instead of 15 gathered words; see cell_axis.
+__device__ __forceinline__ void resolve_hit(const TraceSmem& sm, const DState& s, const DStatic& g, const Grid& grid, f3 O, f3 D, int i,
+                                            Hit& h) {
     const bool hit = h.q != -1;
     h.H = hit ? O + D * h.t : O;
     if (!hit) { h.pi = i; h.back = true; return; }
     if (h.q >= 0) {
-        h.pi = point_index(s, h.H, h.q);
+        if (s.nquad) {
+            const float4 R0 = sm.quad[2 * h.q], R1 = sm.quad[2 * h.q + 1];
+            const int code = __float_as_int(R1.w);   // axes of u, v, n (2 bits each), n's sign, 1 = aligned
+            if (code & 128) {
+                const int nu = __float_as_int(R1.x), nv = __float_as_int(R1.y);
+                bool ok = true;
+                const int iu = cell_axis(sel3(h.H, code & 3), R0.x, R0.y, nu, ok);
+                const int iv = cell_axis(sel3(h.H, (code >> 2) & 3), R0.z, R0.w, nv, ok);
+                const float dn = sel3(D, (code >> 4) & 3);
+                h.back = (code & 64) ? dn > 0.f : dn < 0.f;
+                h.pi = ok ? __float_as_int(R1.z) + iv * nu + iu : point_index(s.Q, s.dims, s.off, h.H, h.q);
+                return;
+            }
+        }
+        h.pi = point_index(s.Q, s.dims, s.off, h.H, h.q);
         const float* Q = s.Q + 12 * h.q;
         h.back = dot(mk(__ldg(Q + 9), __ldg(Q + 10), __ldg(Q + 11)), D) > 0.f;
         return;
@@ -534,34 +732,45 @@ __device__ __forceinline__ void resolve_hit(const DState& s, const DStatic& g, c
 __device__ __forceinline__ Hit trace_resolve(const TraceSmem& sm, const DState& s, const DStatic& g, const Grid& grid,
                                              const FrameParams& p, const DevCache& c, f3 O, f3 D, int i) {
     Hit h;
-    int jb;
-    trace_dyn(sm, s, p.brute != 0, O, D, h.t, h.q, jb);
+    trace_dyn(sm, s, p.brute != 0, O, D, h.t, h.q);
     if (p.check) {
-        float tb; int qb, jbb;
-        trace_dyn(sm, s, true, O, D, tb, qb, jbb);
+        float tb; int qb;
+        trace_dyn(sm, s, true, O, D, tb, qb);
         atomicAdd(c.check + 1, 1ull);
         if (qb != h.q || __float_as_int(tb) != __float_as_int(h.t)) atomicAdd(c.check, 1ull);
     }
     if (g.has_bvh) trace_bvh(g, O, D, h.t, h.q, c.flags);
-    resolve_hit(s, g, grid, O, D, i, h);
+    resolve_hit(sm, s, g, grid, O, D, i, h);
     return h;
 }
 
+// What the trace reads of a state's geometry goes to shared memory once per block: with boxes their
+// records alone (the full scan takes few rays and reads the triangles through L1), otherwise the triangles, the groups and the triangles outside any; the quad records with both.
 __device__ __forceinline__ void stage_smem(float4* sm, const DState& s) {
-    float4* st = sm;
-    float4* sg = sm + 3 * s.nt;
-    const int ngf = grp_float4s(s.ng);
-    int* smi = (int*)(sg + ngf);
-    for (int j = threadIdx.x; j < 3 * s.nt; j += blockDim.x) st[j] = s.tri[j];
-    for (int j = threadIdx.x; j < ngf; j += blockDim.x) sg[j] = s.grp[j];
-    for (int j = threadIdx.x; j < s.nmisc; j += blockDim.x) smi[j] = s.misc[j];
+    const int nt = staged_tri(s), nr = staged_rec(s);
+    const float4* rec = s.grp + (grp_float4s(s) - nr);
+    for (int j = threadIdx.x; j < nr; j += blockDim.x) sm[j] = rec[j];
+    for (int j = threadIdx.x; j < nt; j += blockDim.x) sm[nr + j] = s.tri[j];
+    int* smi = (int*)(sm + nr + nt);
+    if (s.nbox < 0)
+        for (int j = threadIdx.x; j < s.nmisc; j += blockDim.x) smi[j] = s.misc[j];
 }
 __device__ __forceinline__ TraceSmem smem_view(float4* sm, const DState& s) {
     TraceSmem t;
-    t.tri = sm;
-    t.grp = sm + 3 * s.nt;
-    t.gpair = t.grp + 3 * s.ng;
-    t.misc = (const int*)(t.grp + grp_float4s(s.ng));
+    const int nt = staged_tri(s), nr = staged_rec(s);
+    t.quad = sm + (nr - 2 * s.nquad);
+    if (s.nbox >= 0) {
+        t.box = sm;
+        t.rect = sm + box_float4s(s);
+        t.grp = s.grp;
+        t.tri = s.tri;
+        t.misc = s.misc;
+    } else {
+        t.box = t.rect = nullptr;
+        t.grp = sm;
+        t.tri = sm + nr;
+        t.misc = (const int*)(sm + nr + nt);
+    }
     return t;
 }
 
@@ -616,8 +825,8 @@ __global__ void __launch_bounds__(BLOCK) k_build(const DState s, const DStatic g
         float r = sqrtf(dot(d, d));
         f3 D = d * (1.f / r);
         float cc = dot(N, D), t;
-        int q, jb;
-        trace_dyn(tsm, s, false, O, D, t, q, jb);
+        int q;
+        trace_dyn(tsm, s, false, O, D, t, q);
         if (g.has_bvh) trace_bvh(g, O, D, t, q, flags);
         bool vis = t >= r - 1e-3f;
         float rr = fmaxf(r, 0.05f);
@@ -1060,12 +1269,11 @@ __global__ void __launch_bounds__(WQ_BLOCK) k_trace_queue(const DState s, const 
                     slot = __float_as_int(a.w);
                     D = mk(b.x, b.y, b.z);
                     pt = __float_as_int(b.w);
-                    int jb;
-                    trace_dyn(tsm, s, p.brute != 0, O, D, tmin, q, jb);
+                    trace_dyn(tsm, s, p.brute != 0, O, D, tmin, q);
                     if (p.check) {
                         float tb;
-                        int qb, jbb;
-                        trace_dyn(tsm, s, true, O, D, tb, qb, jbb);
+                        int qb;
+                        trace_dyn(tsm, s, true, O, D, tb, qb);
                         atomicAdd(c.check + 1, 1ull);
                         if (qb != q || __float_as_int(tb) != __float_as_int(tmin)) atomicAdd(c.check, 1ull);
                     }
@@ -1153,7 +1361,7 @@ __global__ void __launch_bounds__(WQ_BLOCK) k_trace_queue(const DState s, const 
                 Hit h;
                 h.t = tmin;
                 h.q = q;
-                resolve_hit(s, g, grid, O, D, pt, h);
+                resolve_hit(tsm, s, g, grid, O, D, pt, h);
                 out[slot] = make_float4(h.H.x, h.H.y, h.H.z, __int_as_float(h.back ? -1 : h.pi));
             } else {
                 atomicOr(c.flags, (unsigned)FLAG_BAD_INDEX);   // a malformed queue record: skipped
@@ -1494,8 +1702,8 @@ __device__ __forceinline__ void store_vertex(rc_hg_vertex* dst, const rc_hg_vert
 // closest hit distance along a shadow ray (no cache-point resolution)
 __device__ __forceinline__ float shadow_t(const TraceSmem& sm, const DState& s, const DStatic& g, f3 O, f3 D, unsigned* flags) {
     float t;
-    int q, jb;
-    trace_dyn(sm, s, false, O, D, t, q, jb);
+    int q;
+    trace_dyn(sm, s, false, O, D, t, q);
     if (g.has_bvh) trace_bvh(g, O, D, t, q, flags);
     return q == -1 ? INFINITY : t;
 }
@@ -2122,8 +2330,8 @@ __global__ void __launch_bounds__(BLOCK) k_trace_rays(const DState s, const DSta
     const float* r = rays + 6 * (size_t)i;
     const f3 o = mk(r[0], r[1], r[2]), d = mk(r[3], r[4], r[5]);
     float t;
-    int q, jb;
-    trace_dyn(tsm, s, brute != 0, o, d, t, q, jb);
+    int q;
+    trace_dyn(tsm, s, brute != 0, o, d, t, q);
     if (g.has_bvh) trace_bvh(g, o, d, t, q, flags);
     prim[i] = q;
     tout[i] = q != -1 ? t : __int_as_float(0x7f800000);

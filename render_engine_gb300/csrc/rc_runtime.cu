@@ -379,9 +379,234 @@ struct Groups {
     std::vector<float4> grp;
     std::vector<int> misc;
     GroupRanges gr{};
+    int nbox = -1, outer = 0;
+    float box_scale = 0.f, box_m = 0.f;
 };
-Groups build_groups(const std::vector<float>& T, const std::vector<int>& TQ, int nt) {
-    struct G { int axis, j0, cnt; float c, lo[2], hi[2]; float line[4]; };
+
+// A plane-culling group: `cnt` triangles from j0 in the plane `c` of one axis, their rectangle in
+// the two other axes (increasing), and the line between the two.
+struct PlaneGroup { int axis, j0, cnt; float c, lo[2], hi[2]; float line[4]; };
+
+// The groups as sides of axis-aligned boxes, for trace_boxes: the largest box whose six sides are
+// all groups encloses the scene (if there is one); then, greedily, the box with the most sides
+// among the groups left that two adjacent sides span; a group that is left over is a box of no
+// thickness.  Appends the box and rectangle records and sets nbox / outer / box_scale / box_m.  The
+// plane filter tests a pair of groups in about 30 instructions and a box costs about 16, so boxes
+// are used when there are no more of them than pairs of groups (and at most MAX_BOXES).
+void build_boxes(const std::vector<PlaneGroup>& gs, const std::vector<float>& T, const std::vector<int>& TQ, float scene_scale,
+                 Groups& out) {
+    struct Box { float lo[3], hi[3]; int face[6]; bool flat; };
+    const int n = (int)gs.size();
+    float scale = scene_scale;
+    auto ax = [](int k, int u) { return u == 0 ? (k == 0 ? 1 : 0) : (k == 2 ? 1 : 2); };
+    auto full = [&](int g, float lo[3], float hi[3]) {   // the rectangle as a box of no thickness
+        const int k = gs[g].axis;
+        lo[k] = hi[k] = gs[g].c;
+        for (int u = 0; u < 2; ++u) { lo[ax(k, u)] = gs[g].lo[u]; hi[ax(k, u)] = gs[g].hi[u]; }
+    };
+    std::vector<char> used(n, 0);
+    for (int g = 0; g < n; ++g) {
+        if (gs[g].cnt == 0) { used[g] = 1; continue; }   // padding
+        float lo[3], hi[3];
+        full(g, lo, hi);
+        for (int k = 0; k < 3; ++k) scale = std::max(scale, std::max(fabsf(lo[k]), fabsf(hi[k])));
+    }
+    const float tol = 1e-6f * scale;
+    auto same = [&](float a, float b) { return fabsf(a - b) <= tol; };
+    // sides of box b among the unused groups (face[2 k + side])
+    auto sides = [&](Box& b) {
+        int found = 0;
+        for (int f = 0; f < 6; ++f) b.face[f] = -1;
+        for (int g = 0; g < n; ++g) {
+            if (used[g]) continue;
+            float lo[3], hi[3];
+            full(g, lo, hi);
+            const int k = gs[g].axis;
+            bool fit = true;
+            for (int a = 0; a < 3; ++a)
+                if (a != k) fit = fit && same(lo[a], b.lo[a]) && same(hi[a], b.hi[a]);
+            if (!fit) continue;
+            const int f = same(lo[k], b.lo[k]) ? 2 * k : (same(lo[k], b.hi[k]) ? 2 * k + 1 : -1);
+            if (f < 0 || b.face[f] >= 0) continue;
+            b.face[f] = g;
+            ++found;
+        }
+        return found;
+    };
+    // the best box that two unused groups of different axes span
+    auto best = [&](bool enclosing, Box& res) {
+        int most = 1;
+        double vol = -1.0;
+        for (int x = 0; x < n; ++x)
+            for (int y = x + 1; y < n; ++y) {
+                if (used[x] || used[y] || gs[x].axis == gs[y].axis) continue;
+                Box b{};
+                float l0[3], h0[3], l1[3], h1[3];
+                full(x, l0, h0);
+                full(y, l1, h1);
+                const int kx = gs[x].axis, ky = gs[y].axis, kz = 3 - kx - ky;
+                if (!same(l0[kz], l1[kz]) || !same(h0[kz], h1[kz])) continue;
+                if (!(same(l0[kx], l1[kx]) || same(l0[kx], h1[kx])) || !(same(l1[ky], l0[ky]) || same(l1[ky], h0[ky]))) continue;
+                for (int a = 0; a < 3; ++a) { b.lo[a] = std::min(l0[a], l1[a]); b.hi[a] = std::max(h0[a], h1[a]); }
+                const int f = sides(b);
+                const double v = (double)(b.hi[0] - b.lo[0]) * (b.hi[1] - b.lo[1]) * (b.hi[2] - b.lo[2]);
+                if (enclosing ? (f == 6 && v > vol) : (f > most || (f == most && v > vol && f > 1))) {
+                    most = f;
+                    vol = v;
+                    res = b;
+                }
+            }
+        return enclosing ? vol > 0.0 : most > 1;
+    };
+    auto take = [&](const Box& b) {
+        for (int f = 0; f < 6; ++f)
+            if (b.face[f] >= 0) used[b.face[f]] = 1;
+    };
+    Box outer{};
+    bool have_outer = best(true, outer);
+    if (have_outer) {   // seen from inside: most of its sides' first triangles wind around an inward normal
+        int inward = 0;
+        for (int f = 0; f < 6; ++f) {
+            const float* t = &T[9 * (size_t)gs[outer.face[f]].j0];
+            const int k = f / 2, a = (k + 1) % 3, b = (k + 2) % 3;
+            const float nk = t[3 + a] * t[6 + b] - t[3 + b] * t[6 + a];
+            inward += (f & 1) ? nk < 0.f : nk > 0.f;
+        }
+        have_outer = inward >= 4;
+    }
+    if (have_outer) take(outer);
+    std::vector<Box> boxes;
+    Box b{};
+    while (best(false, b)) {
+        b.flat = false;
+        take(b);
+        boxes.push_back(b);
+    }
+    for (int g = 0; g < n; ++g) {
+        if (used[g]) continue;
+        Box f{};
+        full(g, f.lo, f.hi);
+        for (int k = 0; k < 6; ++k) f.face[k] = -1;
+        f.face[2 * gs[g].axis] = f.face[2 * gs[g].axis + 1] = g;
+        f.flat = true;
+        boxes.push_back(f);
+    }
+    if (boxes.size() > (size_t)n / 2 || boxes.size() > (size_t)MAX_BOXES || !out.misc.empty()) return;
+    const float m = 1e-5f + 2e-6f * scale;
+    out.nbox = ((int)boxes.size() + 1) / 2 * 2;
+    out.outer = have_outer ? 1 : 0;
+    out.box_scale = 4.f * scale;
+    out.box_m = m;
+    if (have_outer) {
+        float c[3], h[3];
+        for (int k = 0; k < 3; ++k) { c[k] = 0.5f * (outer.lo[k] + outer.hi[k]); h[k] = 0.5f * (outer.hi[k] - outer.lo[k]) - m; }
+        out.grp.push_back(make_float4(c[0], c[1], c[2], h[0]));
+        out.grp.push_back(make_float4(h[1], h[2], 0.f, 0.f));
+    }
+    // slabs: centre and half extent grown by m; an empty box is missed by every ray
+    for (int x = 0; x < out.nbox; x += 2) {
+        float c[3][2], h[3][2];
+        for (int u = 0; u < 2; ++u)
+            for (int k = 0; k < 3; ++k) {
+                const bool real = x + u < (int)boxes.size();
+                c[k][u] = real ? 0.5f * (boxes[x + u].lo[k] + boxes[x + u].hi[k]) : 0.f;
+                h[k][u] = real ? 0.5f * (boxes[x + u].hi[k] - boxes[x + u].lo[k]) + m : -1e30f;
+            }
+        out.grp.push_back(make_float4(c[0][0], c[1][0], c[0][1], c[1][1]));
+        out.grp.push_back(make_float4(c[2][0], c[2][1], h[0][0], h[1][0]));
+        out.grp.push_back(make_float4(h[0][1], h[1][1], h[2][0], h[2][1]));
+    }
+    // A group as a rectangle: two triangles (p, e1, e2) and (p', -e1, -e2) in one plane whose edges
+    // have one component each.  (c, |e1|, |e2|, quad) (centre a, half a less m, centre b, half b
+    // less m) (the diagonal); other groups have no rectangle and go to the plane filter.
+    auto comp = [](const float* v) {
+        int k = -1;
+        for (int a = 0; a < 3; ++a)
+            if (v[a] != 0.f) {
+                if (k >= 0) return -1;
+                k = a;
+            }
+        return k;
+    };
+    std::vector<char> rect_ok(n, 0);
+    std::vector<float4> rect;
+    for (int g = 0; g < n; ++g) {
+        const PlaneGroup& G = gs[g];
+        float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0;
+        if (G.cnt == 2 && std::isfinite(G.line[3])) {
+            const float *t0 = &T[9 * (size_t)G.j0], *t1 = t0 + 9;
+            const int a = comp(t0 + 3), b = comp(t0 + 6);
+            bool ok = a >= 0 && b >= 0 && a != b && a != G.axis && b != G.axis && t1[G.axis] == G.c;
+            for (int k = 0; k < 6; ++k) ok = ok && t1[3 + k] == -t0[3 + k];
+            const float ha = 0.5f * (G.hi[0] - G.lo[0]) - m, hb = 0.5f * (G.hi[1] - G.lo[1]) - m;
+            if (ok && ha > 0.f && hb > 0.f) {
+                rect_ok[g] = 1;
+                float qb;
+                memcpy(&qb, &TQ[G.j0], 4);
+                r0 = make_float4(G.c, fabsf(t0[3 + a]), fabsf(t0[6 + b]), qb);
+                r1 = make_float4(0.5f * (G.lo[0] + G.hi[0]), ha, 0.5f * (G.lo[1] + G.hi[1]), hb);
+                r2 = make_float4(G.line[0], G.line[1], G.line[2], 0.f);
+            }
+        }
+        rect.push_back(r0);
+        rect.push_back(r1);
+        rect.push_back(r2);
+    }
+    auto planes = [&](const Box& x) {
+        uint32_t v[2] = {0xffffffffu, 0xff00ffffu | (x.flat ? 0x10000u : 0u)};
+        for (int f = 0; f < 6; ++f)
+            if (x.face[f] >= 0 && rect_ok[x.face[f]]) v[f / 4] = (v[f / 4] & ~(0xffu << (8 * (f & 3)))) | (uint32_t)x.face[f] << (8 * (f & 3));
+        float w0, w1;
+        memcpy(&w0, &v[0], 4);
+        memcpy(&w1, &v[1], 4);
+        out.grp.push_back(make_float4(x.lo[0], x.hi[0], x.lo[1], x.hi[1]));
+        out.grp.push_back(make_float4(x.lo[2], x.hi[2], w0, w1));
+    };
+    Box empty{};
+    for (int f = 0; f < 6; ++f) empty.face[f] = -1;
+    boxes.resize((size_t)out.nbox, empty);
+    for (const Box& x : boxes) planes(x);
+    if (have_outer) planes(outer);
+    out.grp.insert(out.grp.end(), rect.begin(), rect.end());
+}
+
+// Quad records for resolve_hit: (o_u, nu / u, o_v, nv / v) (nu, nv, first point, axes and flags),
+// u, v, n the single components of edges and normal that lie along the axes; a quad with other
+// edges gets flags 0.  None above 64 quads (2 KB of shared memory).
+int build_quads(const std::vector<float>& Q, const std::vector<int>& dims, const std::vector<int>& off, std::vector<float4>& out) {
+    const int nq = (int)off.size();
+    if (nq > 64) return 0;
+    auto axis = [](const float* v) {
+        int k = -1;
+        for (int a = 0; a < 3; ++a)
+            if (v[a] != 0.f) {
+                if (k >= 0 || !std::isfinite(v[a])) return -1;
+                k = a;
+            }
+        return k;
+    };
+    for (int q = 0; q < nq; ++q) {
+        const float* p = &Q[12 * (size_t)q];
+        const int ku = axis(p + 3), kv = axis(p + 6), kn = axis(p + 9);
+        float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
+        // the components' squares and quotients stay normal numbers
+        auto plain = [](float v) { return fabsf(v) > 1e-12f && fabsf(v) < 1e12f; };
+        if (ku >= 0 && kv >= 0 && kn >= 0 && fabsf(p[9 + kn]) == 1.f && plain(p[3 + ku]) && plain(p[6 + kv])) {
+            const int code = ku | kv << 2 | kn << 4 | (p[9 + kn] > 0.f ? 64 : 0) | 128;
+            r0 = make_float4(p[ku], (float)dims[2 * q] / p[3 + ku], p[kv], (float)dims[2 * q + 1] / p[6 + kv]);
+            memcpy(&r1.x, &dims[2 * q], 4);
+            memcpy(&r1.y, &dims[2 * q + 1], 4);
+            memcpy(&r1.z, &off[q], 4);
+            memcpy(&r1.w, &code, 4);
+        }
+        out.push_back(r0);
+        out.push_back(r1);
+    }
+    return nq;
+}
+
+Groups build_groups(const std::vector<float>& T, const std::vector<int>& TQ, int nt, float scene_scale) {
+    using G = PlaneGroup;
     std::vector<G> gs;
     std::vector<int> misc;
     auto axis_of = [&](int j) {
@@ -526,6 +751,7 @@ Groups build_groups(const std::vector<float>& T, const std::vector<int>& TQ, int
     }
     std::sort(misc.begin(), misc.end());
     out.misc = misc;
+    build_boxes(gs, T, TQ, scene_scale, out);
     return out;
 }
 
@@ -646,9 +872,17 @@ rc_status load_scene(rc_ctx* ctx, const uint8_t* data, size_t n) {
             tri[3 * j + 1] = make_float4(t[3], t[4], t[5], 0.f);
             tri[3 * j + 2] = make_float4(t[6], t[7], t[8], 0.f);
         }
-        Groups G = build_groups(T, TQ, S.Nt);
+        float scene_scale = 0.f;
+        for (int a = 0; a < 3; ++a)
+            scene_scale = std::max(scene_scale, std::max(fabsf(S.grid.lo[a]), fabsf(S.grid.lo[a] + S.grid.ext[a])));
+        Groups G = build_groups(T, TQ, S.Nt, scene_scale);
         DState& d = hs.d;
         memset(&d, 0, sizeof d);
+        d.nquad = build_quads(Q, dims, off, G.grp);
+        d.nbox = G.nbox;
+        d.outer = G.outer;
+        d.box_scale = G.box_scale;
+        d.box_m = G.box_m;
         stage.add(&d.Q, Q);
         stage.add(&d.dims, dims);
         stage.add(&d.off, off);
