@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -55,6 +56,10 @@ struct HgDev {
     int depth;
     int acc_frames, stale_frames;
     float td;
+    float ext[3];        // zone box extents zhi - zlo
+    float half;          // half of the smallest zone edge (the segments' sampling step)
+    float gs[3];         // zones per unit length, G / ext
+    float gm[3];         // 2^-19 (|zlo| G / ext + G) + 2e-7 G / ext, see mark_segment
 };
 
 rc_status fail(rc_hg* hg, rc_status s, const char* fmt, ...) {
@@ -86,6 +91,15 @@ HgDev dev_of(const rc_hg* hg) {
     d.acc_frames = hg->cfg.acc_frames;
     d.stale_frames = hg->cfg.stale_frames;
     d.td = hg->cfg.tracing_distance;
+    const float G[3] = {(float)ZX, (float)ZY, (float)ZZ};
+    float c[3];
+    for (int k = 0; k < 3; ++k) {
+        d.ext[k] = d.zhi[k] - d.zlo[k];
+        c[k] = d.ext[k] / G[k];
+        d.gs[k] = G[k] / d.ext[k];
+        d.gm[k] = 1.9073486e-6f * (std::fabs(d.zlo[k]) * d.gs[k] + G[k]) + 2e-7f * d.gs[k];
+    }
+    d.half = 0.5f * std::min(c[0], std::min(c[1], c[2]));
     return d;
 }
 
@@ -95,26 +109,66 @@ int grid_for(size_t n, int block) { return (int)std::min<size_t>((n + block - 1)
 __device__ __forceinline__ float mn(float a, float b) { return a < b ? a : b; }
 __device__ __forceinline__ float mx(float a, float b) { return a > b ? a : b; }
 
+// bit b of a 96-bit mask (no bit for b >= 96): shl.b32 gives 0 for a shift of 32 or more, so each
+// word takes the shift by b less its own offset, wrapped around below it
+__device__ __forceinline__ uint32_t shl1(uint32_t n) {
+    uint32_t r;
+    asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(n));
+    return r;
+}
+__device__ __forceinline__ void zone_bit(uint32_t (&m)[3], uint32_t b) {
+    m[0] |= shl1(b);
+    m[1] |= shl1(b - 32u);
+    m[2] |= shl1(b - 64u);
+}
+
 // rtxgi_bench.patch:825-837 DepMarkPoint
-__device__ __forceinline__ void mark_point(const HgDev& c, uint32_t (&m)[3], float px, float py, float pz) {
-    const float p[3] = {px, py, pz};
+__device__ __noinline__ uint32_t zone_exact(const float zlo0, const float zlo1, const float zlo2, const float e0, const float e1,
+                                            const float e2, float px, float py, float pz) {
+    const float p[3] = {px, py, pz}, lo[3] = {zlo0, zlo1, zlo2}, e[3] = {e0, e1, e2};
     const float G[3] = {(float)ZX, (float)ZY, (float)ZZ};
     float cc[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) cc[k] = __fmul_rn(__fdiv_rn(__fsub_rn(p[k], c.zlo[k]), __fsub_rn(c.zhi[k], c.zlo[k])), G[k]);
+    for (int k = 0; k < 3; ++k) cc[k] = __fmul_rn(__fdiv_rn(__fsub_rn(p[k], lo[k]), e[k]), G[k]);
 #pragma unroll
     for (int k = 0; k < 3; ++k)
-        if (cc[k] < 0.0f || cc[k] >= G[k]) return;
-    const uint32_t b = (uint32_t)cc[0] + ZX * ((uint32_t)cc[1] + ZY * (uint32_t)cc[2]);
-    const uint32_t bit = 1u << (b & 31u);
-    if (b < 32u) m[0] |= bit;
-    else if (b < 64u) m[1] |= bit;
-    else m[2] |= bit;
+        if (cc[k] < 0.0f || cc[k] >= G[k]) return 96u;
+    return (uint32_t)cc[0] + ZX * ((uint32_t)cc[1] + ZY * (uint32_t)cc[2]);
+}
+__device__ __forceinline__ void mark_point(const HgDev& c, uint32_t (&m)[3], float px, float py, float pz) {
+    // (p - lo) * (G / ext): two roundings where the exact quotient and product have two, 2.4e-7
+    // relative in all; off an integer by four times that, the integer part is the same
+    const float cc[3] = {__fmul_rn(__fsub_rn(px, c.zlo[0]), c.gs[0]), __fmul_rn(__fsub_rn(py, c.zlo[1]), c.gs[1]),
+                         __fmul_rn(__fsub_rn(pz, c.zlo[2]), c.gs[2])};
+    const float fx = floorf(cc[0]), fy = floorf(cc[1]), fz = floorf(cc[2]);
+    // (1e-30: a quotient that underflows where this product does not)
+    auto far = [](float x, float f) { return fminf(x - f, f + 1.f - x) > 1e-6f * fabsf(x) + 1e-30f; };
+    uint32_t b;
+    if (far(cc[0], fx) && far(cc[1], fy) && far(cc[2], fz)) {
+        const bool in = fx >= 0.f && fx < (float)ZX && fy >= 0.f && fy < (float)ZY && fz >= 0.f && fz < (float)ZZ;
+        b = in ? (uint32_t)fx + ZX * ((uint32_t)fy + ZY * (uint32_t)fz) : 96u;
+    } else {
+        b = zone_exact(c.zlo[0], c.zlo[1], c.zlo[2], c.ext[0], c.ext[1], c.ext[2], px, py, pz);
+    }
+    zone_bit(m, b);
 }
 
 // rtxgi_bench.patch:839-858 DepMarkSegment: the segment clipped to the zone box, sampled every
 // half of the smallest zone edge (at most 49 points); lerp(a, b, s) = a + s (b - a).
-__device__ void mark_segment(const HgDev& c, uint32_t (&m)[3], const float (&a)[3], const float (&b)[3]) {
+//
+// Bound by instruction issue.  The HLSL's samples take four IEEE divisions each (about 100
+// instructions); here the samples' zone coordinates (p - lo) G / ext are stepped in fixed point, 27
+// fraction bits, about 25 instructions a sample, and a sample that lies within a margin of a zone's
+// face is computed as the HLSL writes it.  The margin: with u = 2^-24, A = (a - lo) G / ext, D = (b -
+// a) G / ext and t at most tmax, the HLSL's own position is off by u (10 |D| tmax + |A| + |lo| G /
+// ext) and its quotient and product by 3 u G; the stepped one by u (3 |A| + 9 |D| tmax + G) and 48
+// roundings of 2^-28; so 2^-19 (|D| tmax + |A| + |lo| G / ext + G) covers both, and 2e-7 G / ext
+// the HLSL's 1e-7 in place of a smaller component in the clip.  The clipped samples lie inside the
+// box, so one that is not within the margin of a face is inside a zone.  1920 x 1080 camera paths of
+// two bounces (k_hg_mark): 736 -> 486 us.
+// START_MARKED: the zone of a is in m already, so a first sample at t = 0 (a itself) is left out.
+template <bool START_MARKED>
+__device__ __forceinline__ void mark_segment(const HgDev& c, uint32_t (&m)[3], const float (&a)[3], const float (&b)[3]) {
     float d[3], tn[3], tf[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -128,21 +182,84 @@ __device__ void mark_segment(const HgDev& c, uint32_t (&m)[3], const float (&a)[
     const float tmin = mx(mx(tn[0], tn[1]), mx(tn[2], 0.0f));
     const float tmax = mn(mn(tf[0], tf[1]), mn(tf[2], 1.0f));
     if (tmin > tmax) return;
-    const float c0 = __fdiv_rn(__fsub_rn(c.zhi[0], c.zlo[0]), (float)ZX);
-    const float c1 = __fdiv_rn(__fsub_rn(c.zhi[1], c.zlo[1]), (float)ZY);
-    const float c2 = __fdiv_rn(__fsub_rn(c.zhi[2], c.zlo[2]), (float)ZZ);
     const float dd = __fadd_rn(__fmul_rn(d[0], d[0]), __fmul_rn(d[1], d[1]));
-    const float len = __fmul_rn(__fsqrt_rn(__fadd_rn(dd, __fmul_rn(d[2], d[2]))), __fsub_rn(tmax, tmin));
-    const float q = ceilf(__fdiv_rn(len, __fmul_rn(0.5f, mn(c0, mn(c1, c2)))));
-    const uint32_t n = q >= 47.0f ? 48u : (uint32_t)q + 1u;
     const float span = __fsub_rn(tmax, tmin);
-    for (uint32_t i = 0; i <= n; ++i) {
-        const float s = __fdiv_rn((float)i, (float)n);
-        const float t = __fadd_rn(tmin, __fmul_rn(s, span));
-        mark_point(c, m, __fadd_rn(a[0], __fmul_rn(d[0], t)), __fadd_rn(a[1], __fmul_rn(d[1], t)),
-                   __fadd_rn(a[2], __fmul_rn(d[2], t)));
+    const float len = __fmul_rn(__fsqrt_rn(__fadd_rn(dd, __fmul_rn(d[2], d[2]))), span);
+    const float q = ceilf(__fdiv_rn(len, c.half));
+    const uint32_t n = q >= 47.0f ? 48u : (uint32_t)q + 1u;
+    const float step = __fdividef(span, (float)n);
+    constexpr float ONE = 134217728.f;   // 2^27
+    int z[3], dz[3];
+    float mg = 0.f;
+    bool fixed = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float A = __fmul_rn(__fsub_rn(a[k], c.zlo[k]), c.gs[k]), D = __fmul_rn(d[k], c.gs[k]);
+        z[k] = __float2int_rn(__fmaf_rn(D, tmin, A) * ONE);
+        dz[k] = __float2int_rn(D * step * ONE);
+        const float mk = __fmaf_rn(1.9073486e-6f, __fadd_rn(fabsf(A), fabsf(D) * tmax), c.gm[k]);
+        mg = fmaxf(mg, mk);
+        fixed = fixed && mk < 0.25f;   // (false for a NaN)
+    }
+    // within the margin of a face: (z + M) mod 2^27 <= 2 M, read in the top 27 bits of a word; all
+    // samples when the margin is no margin
+    const uint32_t M = fixed ? (uint32_t)(mg * ONE) + 1u : 0u, lim = fixed ? M << 6 : 0xffffffffu;
+    uint32_t late0 = 0u, late1 = 0u;   // the samples left to the exact evaluation, n <= 48
+    uint32_t i0 = 0u;
+    if (START_MARKED && tmin == 0.f) {
+        i0 = 1u;
+        z[0] += dz[0];
+        z[1] += dz[1];
+        z[2] += dz[2];
+    }
+    for (uint32_t i = i0; i <= n; ++i) {
+        const uint32_t f0 = ((uint32_t)z[0] + M) << 5, f1 = ((uint32_t)z[1] + M) << 5, f2 = ((uint32_t)z[2] + M) << 5;
+        const bool late = min(min(f0, f1), f2) <= lim;
+        const uint32_t zone = (uint32_t)(z[0] >> 27) + ZX * ((uint32_t)(z[1] >> 27) + ZY * (uint32_t)(z[2] >> 27));
+        zone_bit(m, late ? 96u : zone);
+        if (late) {
+            late0 |= shl1(i);
+            late1 |= shl1(i - 32u);
+        }
+        z[0] += dz[0];
+        z[1] += dz[1];
+        z[2] += dz[2];
+    }
+    // hits lie on walls, which often are faces of the zones: a segment's last sample is one of
+    // these, and evaluating it inside the loop would send the warp through it at every step
+    while (late0 | late1) {
+        uint32_t i;
+        if (late0) {
+            i = (uint32_t)__ffs((int)late0) - 1u;
+            late0 &= late0 - 1u;
+        } else {
+            i = 31u + (uint32_t)__ffs((int)late1);
+            late1 &= late1 - 1u;
+        }
+        const float t = __fadd_rn(tmin, __fmul_rn(__fdiv_rn((float)i, (float)n), span));
+        zone_bit(m, zone_exact(c.zlo[0], c.zlo[1], c.zlo[2], c.ext[0], c.ext[1], c.ext[2], __fadd_rn(a[0], __fmul_rn(d[0], t)),
+                               __fadd_rn(a[1], __fmul_rn(d[1], t)), __fadd_rn(a[2], __fmul_rn(d[2], t))));
     }
 }
+
+// A vertex record in four 16-byte loads; WIDE needs 16-byte aligned records (the launch looks).
+template <bool WIDE>
+__device__ __forceinline__ rc_hg_vertex load_vertex(const rc_hg_vertex* __restrict__ v) {
+    if (!WIDE) return *v;
+    rc_hg_vertex x;
+    const float4* s = reinterpret_cast<const float4*>(v);
+    const float4 a = __ldg(s), b = __ldg(s + 1), e = __ldg(s + 2), f = __ldg(s + 3);
+    x.origin[0] = a.x; x.origin[1] = a.y; x.origin[2] = a.z;
+    x.dir[0] = a.w; x.dir[1] = b.x; x.dir[2] = b.y;
+    x.hit[0] = b.z; x.hit[1] = b.w; x.hit[2] = e.x;
+    x.to_light[0] = e.y; x.to_light[1] = e.z; x.to_light[2] = e.w;
+    x.light_dist = f.x;
+    x.light_index = __float_as_int(f.y);
+    x.entry = __float_as_uint(f.z);
+    x.flags = __float_as_uint(f.w);
+    return x;
+}
+bool wide_vertices(const rc_hg_vertex* v) { return (reinterpret_cast<uintptr_t>(v) & 15u) == 0; }
 
 // rtxgi_bench.patch:860-880 DepOr: OR into the bank being filled, only the words with new bits
 __device__ __forceinline__ void dep_or(uint4* bank, uint32_t e, uint4 m) {
@@ -162,6 +279,7 @@ __device__ __forceinline__ void dep_or(uint4* bank, uint32_t e, uint4 m) {
 // bw is one of b0 / b1 (no __restrict__ on them: they alias).
 // Paths are either contiguous (ps = npaths + 1 offsets) or in fixed slots (ps = NULL, path p is
 // v[p * stride .. p * stride + plen[p])).
+template <bool WIDE>
 __global__ void __launch_bounds__(HG_BLOCK) k_hg_mark(const HgDev c, const rc_hg_vertex* __restrict__ v,
                                                       const int* __restrict__ ps, const int* __restrict__ plen, int stride, int npaths,
                                                       uint4* bw, const uint4* b0, const uint4* b1) {
@@ -173,26 +291,26 @@ __global__ void __launch_bounds__(HG_BLOCK) k_hg_mark(const HgDev c, const rc_hg
     const long long j0 = ps ? ps[p] : (long long)p * stride;
     const long long j1 = ps ? ps[p + 1] : j0 + plen[p];
     for (long long j = j0; j < j1; ++j) {
-        const rc_hg_vertex x = v[j];
+        const rc_hg_vertex x = load_vertex<WIDE>(v + j);
         const float o[3] = {x.origin[0], x.origin[1], x.origin[2]};
         if (x.flags & RC_HG_MISS) {
             uint32_t sm[3] = {0u, 0u, 0u};
             const float e[3] = {__fadd_rn(o[0], __fmul_rn(x.dir[0], c.td)), __fadd_rn(o[1], __fmul_rn(x.dir[1], c.td)),
                                 __fadd_rn(o[2], __fmul_rn(x.dir[2], c.td))};
-            mark_segment(c, sm, o, e);
+            mark_segment<false>(c, sm, o, e);
             const uint4 dm = make_uint4(sm[0], sm[1], sm[2], RC_HG_SKY_BIT);
             for (int di = 0; di < len; ++di) dep_or(bw, idx[di], dm);
             break;
         }
         const float h[3] = {x.hit[0], x.hit[1], x.hit[2]};
         uint32_t din[3] = {0u, 0u, 0u}, dloc[3] = {0u, 0u, 0u}, lights = 0u;
-        mark_segment(c, din, o, h);
+        mark_segment<false>(c, din, o, h);
         mark_point(c, dloc, h[0], h[1], h[2]);
         if (x.light_index >= 0) {
             const float r = mn(x.light_dist, c.td);
             const float e[3] = {__fadd_rn(h[0], __fmul_rn(x.to_light[0], r)), __fadd_rn(h[1], __fmul_rn(x.to_light[1], r)),
                                 __fadd_rn(h[2], __fmul_rn(x.to_light[2], r))};
-            mark_segment(c, dloc, h, e);
+            mark_segment<true>(c, dloc, h, e);
             if (x.flags & RC_HG_LIGHT_VISIBLE) lights |= 1u << min(x.light_index, 30);
         }
         const int prev = len;
@@ -242,35 +360,48 @@ __constant__ float c_seg19[20] = {0.f / 19.f,  1.f / 19.f,  2.f / 19.f,  3.f / 1
 // Bit l of every voxel on the shadow segment of a vertex whose sampled light l (< 64) was
 // visible: 20 evenly spaced samples from the hit to the light (at most tracing_distance), as
 // k_build rasterises its shadow rays (poc_gpu.cu:192-197).  A bit already set is not written.
+// One thread per vertex slot (path p, vertex j < plen[p]): bound by the latency of the samples'
+// reads (64-bit words of the L2), so ten of them are in flight at a time.  1920 x 1080 paths, three
+// slots each, 128^3 voxels: 336 us with a thread per path and four reads in flight, 293 us (L2 70 % busy).
+template <bool WIDE>
 __global__ void __launch_bounds__(HG_BLOCK) k_vox_mark(const HgDev c, const VoxDev g, const rc_hg_vertex* __restrict__ v,
-                                                       const int* __restrict__ plen, int stride, int npaths,
+                                                       const int* __restrict__ plen, int stride, long long nslots,
                                                        unsigned long long* __restrict__ vox) {
     const int res = g.res;
-    const int p = blockIdx.x * HG_BLOCK + threadIdx.x;
-    if (p >= npaths) return;
-    const long long j0 = (long long)p * stride;
-    for (long long j = j0; j < j0 + plen[p]; ++j) {
-        const rc_hg_vertex x = v[j];
+    for (long long j = blockIdx.x * (long long)HG_BLOCK + threadIdx.x; j < nslots; j += (long long)gridDim.x * HG_BLOCK) {
+        const long long p = j / stride;
+        if (j - p * stride >= plen[p]) continue;
+        const rc_hg_vertex x = load_vertex<WIDE>(v + j);
         if ((x.flags & RC_HG_MISS) || x.light_index < 0 || x.light_index >= 64 || !(x.flags & RC_HG_LIGHT_VISIBLE)) continue;
         const unsigned long long bit = 1ull << x.light_index;
         const float r = mn(x.light_dist, c.td);
         float a[3], d[3];
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
             a[k] = x.hit[k];
             d[k] = __fmul_rn(x.to_light[k], r);
         }
-        size_t last = ~(size_t)0;   // consecutive samples in one voxel mark it once
-#pragma unroll 4
-        for (int k = 0; k < 20; ++k) {
-            const float t = c_seg19[k];
-            const int ix = vox_axis(__fadd_rn(a[0], __fmul_rn(d[0], t)), g.lo[0], g.scale[0], res);
-            const int iy = vox_axis(__fadd_rn(a[1], __fmul_rn(d[1], t)), g.lo[1], g.scale[1], res);
-            const int iz = vox_axis(__fadd_rn(a[2], __fmul_rn(d[2], t)), g.lo[2], g.scale[2], res);
-            const size_t vi = ((size_t)iz * res + iy) * res + ix;
-            if (vi == last) continue;
-            last = vi;
-            unsigned long long* w = vox + vi;
-            if (!(__ldcg(w) & bit)) atomicOr(w, bit);
+        unsigned last = ~0u;   // consecutive samples in one voxel mark it once (res <= 256: 24-bit indexes)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            unsigned vi[10];
+            bool on[10];
+            unsigned long long w[10];
+#pragma unroll
+            for (int k = 0; k < 10; ++k) {
+                const float t = c_seg19[10 * h + k];
+                const int ix = vox_axis(__fadd_rn(a[0], __fmul_rn(d[0], t)), g.lo[0], g.scale[0], res);
+                const int iy = vox_axis(__fadd_rn(a[1], __fmul_rn(d[1], t)), g.lo[1], g.scale[1], res);
+                const int iz = vox_axis(__fadd_rn(a[2], __fmul_rn(d[2], t)), g.lo[2], g.scale[2], res);
+                vi[k] = (unsigned)((iz * res + iy) * res + ix);
+                on[k] = vi[k] != last;
+                last = vi[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 10; ++k) w[k] = on[k] ? __ldcg(vox + vi[k]) : bit;
+#pragma unroll
+            for (int k = 0; k < 10; ++k)
+                if (!(w[k] & bit)) atomicOr(vox + vi[k], bit);
         }
     }
 }
@@ -708,8 +839,9 @@ rc_status rc_hg_begin_frame(rc_hg* hg, uint32_t dep_frame, uint32_t period) {
 rc_status rc_hg_mark_paths(rc_hg* hg, const rc_hg_vertex* d_vertices, const int* d_path_start, int npaths) {
     if (!hg || npaths < 0 || (npaths > 0 && (!d_vertices || !d_path_start))) return RC_ERR_ARG;
     if (npaths == 0) return RC_OK;
-    k_hg_mark<<<grid_for(npaths, HG_BLOCK), HG_BLOCK, 0, hg->stream>>>(dev_of(hg), d_vertices, d_path_start, nullptr, 0, npaths,
-                                                                        hg->bank[hg->bank_sel], hg->bank[0], hg->bank[1]);
+    auto kern = wide_vertices(d_vertices) ? k_hg_mark<true> : k_hg_mark<false>;
+    kern<<<grid_for(npaths, HG_BLOCK), HG_BLOCK, 0, hg->stream>>>(dev_of(hg), d_vertices, d_path_start, nullptr, 0, npaths,
+                                                                  hg->bank[hg->bank_sel], hg->bank[0], hg->bank[1]);
     HGCK(cudaGetLastError());
     return RC_OK;
 }
@@ -717,8 +849,9 @@ rc_status rc_hg_mark_paths(rc_hg* hg, const rc_hg_vertex* d_vertices, const int*
 rc_status rc_hg_mark_paths_strided(rc_hg* hg, const rc_hg_vertex* d_vertices, const int* d_len, int stride, int npaths) {
     if (!hg || npaths < 0 || stride < 1 || (npaths > 0 && (!d_vertices || !d_len))) return RC_ERR_ARG;
     if (npaths == 0) return RC_OK;
-    k_hg_mark<<<grid_for(npaths, HG_BLOCK), HG_BLOCK, 0, hg->stream>>>(dev_of(hg), d_vertices, nullptr, d_len, stride, npaths,
-                                                                        hg->bank[hg->bank_sel], hg->bank[0], hg->bank[1]);
+    auto kern = wide_vertices(d_vertices) ? k_hg_mark<true> : k_hg_mark<false>;
+    kern<<<grid_for(npaths, HG_BLOCK), HG_BLOCK, 0, hg->stream>>>(dev_of(hg), d_vertices, nullptr, d_len, stride, npaths,
+                                                                  hg->bank[hg->bank_sel], hg->bank[0], hg->bank[1]);
     HGCK(cudaGetLastError());
     return RC_OK;
 }
@@ -749,8 +882,9 @@ rc_status rc_hg_voxels_mark(rc_hg* hg, const rc_hg_vertex* d_vertices, const int
     if (!hg || npaths < 0 || stride < 1 || (npaths > 0 && (!d_vertices || !d_len))) return RC_ERR_ARG;
     if (!hg->vres) return fail(hg, RC_ERR_STATE, "no voxel masks (rc_hg_voxels_init)");
     if (npaths == 0) return RC_OK;
-    k_vox_mark<<<grid_for(npaths, HG_BLOCK), HG_BLOCK, 0, hg->stream>>>(dev_of(hg), vox_dev(hg), d_vertices, d_len, stride, npaths,
-                                                                         hg->vox);
+    const long long nslots = (long long)npaths * stride;
+    auto kern = wide_vertices(d_vertices) ? k_vox_mark<true> : k_vox_mark<false>;
+    kern<<<grid_for((size_t)nslots, HG_BLOCK), HG_BLOCK, 0, hg->stream>>>(dev_of(hg), vox_dev(hg), d_vertices, d_len, stride, nslots, hg->vox);
     HGCK(cudaGetLastError());
     return RC_OK;
 }
