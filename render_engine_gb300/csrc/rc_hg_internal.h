@@ -9,6 +9,6 @@ namespace rc {
 cudaStream_t hg_stream(rc_hg* hg);   // the stream the cache's work is issued on
 const rc_hg_config& hg_config(const rc_hg* hg);
 bool hg_has_voxels(const rc_hg* hg);
-// v[i].entry = entry[i], on the cache's stream
-cudaError_t hg_set_entries(rc_hg* hg, rc_hg_vertex* v, const uint32_t* entry, long long n);
+// rc_hg_insert on the cache's stream, the entries also into v[i].entry
+cudaError_t hg_insert_vertices(rc_hg* hg, const float* pos, const float* nrm, int n, uint32_t* entry, rc_hg_vertex* v);
 }  // namespace rc

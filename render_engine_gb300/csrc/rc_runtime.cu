@@ -2537,8 +2537,7 @@ rc_status rc_hg_camera_paths(rc_hg* hg, rc_ctx* ctx, int state, const rc_hg_path
     p.NR = S.NR;
     CKR(RC_DISPATCH(S.NL, paths(S.st[state].d, S.g, S.grid, ctx->c, p, cd, pd, C.pos, C.nrm, C.rgb, C.vtx, C.len, d_image, hs)));
     const int n = (int)nslots, np = (int)npix;
-    if ((st = rc_hg_insert(hg, C.pos, C.nrm, n, C.entry))) return fail(ctx, st, "insert: %s", rc_hg_last_error(hg));
-    CKR(rc::hg_set_entries(hg, C.vtx, C.entry, (long long)nslots));
+    CKR(rc::hg_insert_vertices(hg, C.pos, C.nrm, n, C.entry, C.vtx));
     if ((st = rc_hg_accumulate(hg, C.entry, C.rgb, n))) return fail(ctx, st, "accumulate: %s", rc_hg_last_error(hg));
     if ((st = rc_hg_mark_paths_strided(hg, C.vtx, C.len, (int)S1, np))) return fail(ctx, st, "mark: %s", rc_hg_last_error(hg));
     if (rc::hg_has_voxels(hg) && (st = rc_hg_voxels_mark(hg, C.vtx, C.len, (int)S1, np)))
@@ -2548,7 +2547,7 @@ rc_status rc_hg_camera_paths(rc_hg* hg, rc_ctx* ctx, int state, const rc_hg_path
     CKR(cudaStreamWaitEvent(ctx->stream, C.ready, 0));
     C.stride = (int)S1;
     C.npaths = np;
-    ctx->launches += 6;
+    ctx->launches += rc::hg_has_voxels(hg) ? 5 : 4;
     return RC_OK;
 }
 
