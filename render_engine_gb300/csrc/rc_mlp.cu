@@ -90,28 +90,19 @@ __global__ void k_wait_check(uint32_t polls, int arrive, unsigned* __restrict__ 
 // ---------------------------------------------------------------- the network
 // 168 input features (padded to 176) -> 64 -> 64 -> 64 -> 64 -> 16 outputs (the first n_out
 // used), ReLU between layers, no biases.  Weights live as FP32 masters with their Adam
-// moments, and as bf16 tiles in the K-major core-matrix layout the MMAs read: W_l (rows =
-// outputs, K = inputs) for the forward products and W_l^T (rows = inputs, K = outputs) for
-// the gradients that flow back.
+// moments, and as bf16 tiles W_l (rows = outputs, K = inputs) in the K-major core-matrix layout the
+// forward products read; the gradients that flow back read the same tiles with the other index as
+// K (rc_umma.cuh).
 constexpr int K0 = 176, HID = 64, OUTP = 16, NLAYER = 5;
 __host__ __device__ constexpr int in_dim(int l) { return l == 0 ? K0 : HID; }
 __host__ __device__ constexpr int out_dim(int l) { return l == NLAYER - 1 ? OUTP : HID; }
 __host__ __device__ constexpr int master_off(int l) { return l == 0 ? 0 : HID * K0 + (l - 1) * HID * HID; }
 constexpr int NWEIGHT = HID * K0 + 3 * HID * HID + OUTP * HID;   // 24,576
-// bf16 tile byte offsets: forward tiles, then the transposed ones of layers 1..4
-__host__ __device__ constexpr int wf_off(int l) { return 2 * master_off(l); }
-constexpr int WF_BYTES = 2 * NWEIGHT;                                 // 49,152
-__host__ __device__ constexpr int wb_off(int l) { return WF_BYTES + 2 * (master_off(l) - master_off(1)); }
-constexpr int WB_BYTES = 2 * (3 * HID * HID + OUTP * HID);            // 26,624
-// activation tiles of one 128-sample tile kept for the backward pass (training)
-constexpr int ACT_X0T = 0;                                            // X0^T: 176 x 128
-__host__ __device__ constexpr int act_ht(int l) { return K0 * 128 * 2 + (l - 1) * HID * 128 * 2; }   // H_l^T, l = 1..4
-constexpr int ACT_DY = K0 * 128 * 2 + 4 * HID * 128 * 2;              // dY: 128 x 16 (K-major)
-constexpr int ACT_DYT = ACT_DY + 128 * OUTP * 2;                      // dY^T: 16 x 128
-constexpr int ACT_BYTES = ACT_DYT + OUTP * 128 * 2;                   // 122,880 per tile
+__host__ __device__ constexpr int wf_off(int l) { return 2 * master_off(l); }   // byte offset of W_l's tile
+constexpr int WF_BYTES = 2 * NWEIGHT;                                           // 49,152
 
 struct MlpArgs {
-    const uint8_t* wbf;        // bf16 tiles (forward, then transposed)
+    const uint8_t* wbf;        // bf16 weight tiles
     const float4* P;           // point position (xyz)
     const float4* N;           // point normal (xyz)
     const float4* aux;         // albedo, direct light of lights 0..2
@@ -123,8 +114,7 @@ struct MlpArgs {
     int ostride;
     int n_out;
     float lo[3], inv_ext[3];   // encoding box
-    uint8_t* act;              // training: activation tiles, ACT_BYTES per tile
-    float* dwpart;             // training: weight gradients of each backward CTA, NWEIGHT per CTA
+    float* dwpart;             // training: weight gradients of each CTA, NWEIGHT per CTA
     float* loss;               // training: sum of the relative L2 loss (for reporting)
     float loss_scale;          // 1 / (samples x n_out)
     const float* scale;        // training: the loss scale of this step (device, MlpState::SCALE)
@@ -134,9 +124,6 @@ struct MlpArgs {
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
-}
-__device__ __forceinline__ float bf16_at(const uint8_t* base, uint32_t off) {
-    return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + off));
 }
 __device__ __forceinline__ void st_bf16(uint8_t* base, uint32_t off, float v) {
     *reinterpret_cast<__nv_bfloat16*>(base + off) = __float2bfloat16_rn(v);
@@ -215,38 +202,47 @@ __device__ __forceinline__ void encode(const MlpArgs& a, int pt, int half, Emit&
     emit(21, f);
 }
 
-// Forward pass over tiles of 128 samples.  A CTA holds the bf16 weights once and runs GROUPS
-// tiles at a time, each on its own group of two warpgroups (thread t of a group works on sample
+// Inference over tiles of 128 queries.  A CTA holds the bf16 weights once and runs GROUPS
+// tiles at a time, each on its own group of two warpgroups (thread t of a group works on query
 // row t % 128; the two threads of a row split the input features and the columns of each
 // accumulator, warp w reading the tensor-memory lanes of its quarter w % 4), with its own
 // activation tile, mbarrier, named barrier and 64 tensor-memory columns; the groups overlap
 // one tile's products with another's encoding and epilogues.
-// TRAIN: also keeps X0^T, H_l^T and dY (with dY^T) of each tile in global memory and adds the
-// loss; otherwise writes the n_out outputs.
 constexpr int FWD_THREADS = 256;                               // threads of one group
-constexpr int INFER_GROUPS = 4;                                // tiles in flight per inference CTA
-constexpr size_t GROUP_SMEM_INFER = (size_t)128 * K0 * 2;      // activation tile
-constexpr size_t GROUP_SMEM_TRAIN = GROUP_SMEM_INFER + (size_t)K0 * 128 * 2;   // + transposed staging
-template <bool TRAIN, int GROUPS>
-__global__ void __launch_bounds__(FWD_THREADS * GROUPS) k_mlp_forward(const MlpArgs a) {
-    const float sc = TRAIN ? __ldg(a.scale) : 1.f;   // loss scale (a power of two)
+constexpr int INFER_GROUPS = 4;                                // tiles in flight per CTA
+constexpr size_t GROUP_SMEM = (size_t)128 * K0 * 2;            // activation tile
+// 16 accumulator columns -> ReLU -> bf16, as two 16-byte pieces of a K-major tile
+__device__ __forceinline__ void relu_pack(const float (&v)[16], uint4& lo4, uint4& hi4) {
+    lo4.x = pack_bf16(fmaxf(v[0], 0.f), fmaxf(v[1], 0.f));
+    lo4.y = pack_bf16(fmaxf(v[2], 0.f), fmaxf(v[3], 0.f));
+    lo4.z = pack_bf16(fmaxf(v[4], 0.f), fmaxf(v[5], 0.f));
+    lo4.w = pack_bf16(fmaxf(v[6], 0.f), fmaxf(v[7], 0.f));
+    hi4.x = pack_bf16(fmaxf(v[8], 0.f), fmaxf(v[9], 0.f));
+    hi4.y = pack_bf16(fmaxf(v[10], 0.f), fmaxf(v[11], 0.f));
+    hi4.z = pack_bf16(fmaxf(v[12], 0.f), fmaxf(v[13], 0.f));
+    hi4.w = pack_bf16(fmaxf(v[14], 0.f), fmaxf(v[15], 0.f));
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+    return make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+}
+__global__ void __launch_bounds__(FWD_THREADS * INFER_GROUPS) k_mlp_infer(const MlpArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t mbar[GROUPS];
+    __shared__ uint64_t mbar[INFER_GROUPS];
     __shared__ uint32_t tmem_base;
-    __shared__ int gflag[GROUPS];
-    constexpr uint32_t TCOLS = GROUPS == 1 ? 64u : (GROUPS == 2 ? 128u : 256u);
-    uint8_t* sw = smem;                               // forward weight tiles, WF_BYTES
+    __shared__ int gflag[INFER_GROUPS];
+    constexpr uint32_t TCOLS = 64u * INFER_GROUPS;
+    uint8_t* sw = smem;                               // weight tiles, WF_BYTES
     const int grp = threadIdx.x / FWD_THREADS, tid = threadIdx.x % FWD_THREADS;
     // this group's activation tile: X0 (128 x 176) and then each H_l (128 x 64) in its place,
     // H_{l+1} written once the product that reads H_l has completed
-    uint8_t* sx = smem + WF_BYTES + (size_t)grp * (TRAIN ? GROUP_SMEM_TRAIN : GROUP_SMEM_INFER);
-    uint8_t* st = sx + 128 * K0 * 2;                  // TRAIN: transposed staging, 176 x 128
+    uint8_t* sx = smem + WF_BYTES + (size_t)grp * GROUP_SMEM;
     const int warp = tid >> 5, lane = tid & 31;
     const int row = tid & 127, half = tid >> 7, quarter = warp & 3;
-    for (int i = threadIdx.x; i < WF_BYTES / 16; i += FWD_THREADS * GROUPS)
+    for (int i = threadIdx.x; i < WF_BYTES / 16; i += FWD_THREADS * INFER_GROUPS)
         reinterpret_cast<uint4*>(sw)[i] = reinterpret_cast<const uint4*>(a.wbf)[i];
-    if (threadIdx.x < GROUPS) mbar_init(&mbar[threadIdx.x], 1);
+    if (threadIdx.x < INFER_GROUPS) mbar_init(&mbar[threadIdx.x], 1);
     if (threadIdx.x < 32) tmem_alloc(&tmem_base, TCOLS);
+    fence_proxy_async();
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -256,33 +252,19 @@ __global__ void __launch_bounds__(FWD_THREADS * GROUPS) k_mlp_forward(const MlpA
     uint32_t phase = 0;
     bool ok = true;
     const int ntiles = (a.n + 127) / 128;
-    for (int tile = blockIdx.x * GROUPS + grp; tile < ntiles && ok; tile += gridDim.x * GROUPS) {
+    for (int tile = blockIdx.x * INFER_GROUPS + grp; tile < ntiles && ok; tile += gridDim.x * INFER_GROUPS) {
         const int s = tile * 128 + row;
         const bool live = s < a.n;
         const int pt = live ? (a.idx ? a.idx[s] : s) : 0;
         encode(a, pt, half, [&](int k8, const float (&f)[8]) {
-            uint4 v;
-            v.x = pack_bf16(f[0], f[1]);
-            v.y = pack_bf16(f[2], f[3]);
-            v.z = pack_bf16(f[4], f[5]);
-            v.w = pack_bf16(f[6], f[7]);
-            *reinterpret_cast<uint4*>(sx + kmajor_offset(row, 8 * k8, K0)) = v;
-            if (TRAIN)
-                for (int j = 0; j < 8; ++j) st_bf16(st, kmajor_offset(8 * k8 + j, row, 128), f[j]);
+            *reinterpret_cast<uint4*>(sx + kmajor_offset(row, 8 * k8, K0)) = pack8(f);
         });
         fence_proxy_async();
         gsync();
-        if (TRAIN) {
-            uint4* dst = reinterpret_cast<uint4*>(a.act + (size_t)tile * ACT_BYTES + ACT_X0T);
-            for (int i = tid; i < K0 * 128 * 2 / 16; i += FWD_THREADS) dst[i] = reinterpret_cast<const uint4*>(st)[i];
-            gsync();
-        }
         for (int l = 0; l < NLAYER && ok; ++l) {
             const int K = in_dim(l), N = out_dim(l);
-            uint8_t* A = sx;
-            uint8_t* Hn = sx;
             if (tid == 0) {
-                const uint32_t a0 = smem_u32(A), b0 = smem_u32(sw + wf_off(l));
+                const uint32_t a0 = smem_u32(sx), b0 = smem_u32(sw + wf_off(l));
                 for (int kk = 0; kk < K / 16; ++kk)
                     mma_bf16(tmem, smem_desc(a0 + 256u * kk, 128u, 16u * K), smem_desc(b0 + 256u * kk, 128u, 16u * K),
                              idesc_bf16_f32(128, N), kk > 0);
@@ -312,49 +294,16 @@ __global__ void __launch_bounds__(FWD_THREADS * GROUPS) k_mlp_forward(const MlpA
                 tmem_wait_ld();
                 if (l < NLAYER - 1) {
                     uint4 lo4, hi4;
-                    lo4.x = pack_bf16(fmaxf(v[0], 0.f), fmaxf(v[1], 0.f));
-                    lo4.y = pack_bf16(fmaxf(v[2], 0.f), fmaxf(v[3], 0.f));
-                    lo4.z = pack_bf16(fmaxf(v[4], 0.f), fmaxf(v[5], 0.f));
-                    lo4.w = pack_bf16(fmaxf(v[6], 0.f), fmaxf(v[7], 0.f));
-                    hi4.x = pack_bf16(fmaxf(v[8], 0.f), fmaxf(v[9], 0.f));
-                    hi4.y = pack_bf16(fmaxf(v[10], 0.f), fmaxf(v[11], 0.f));
-                    hi4.z = pack_bf16(fmaxf(v[12], 0.f), fmaxf(v[13], 0.f));
-                    hi4.w = pack_bf16(fmaxf(v[14], 0.f), fmaxf(v[15], 0.f));
-                    *reinterpret_cast<uint4*>(Hn + kmajor_offset(row, c, HID)) = lo4;
-                    *reinterpret_cast<uint4*>(Hn + kmajor_offset(row, c + 8, HID)) = hi4;
-                    if (TRAIN)
-                        for (int j = 0; j < 16; ++j) st_bf16(st, kmajor_offset(c + j, row, 128), fmaxf(v[j], 0.f));
-                } else if (!TRAIN) {
-                    if (live)
-                        for (int j = 0; j < a.n_out; ++j) a.out[(size_t)s * a.ostride + j] = v[j];
-                } else {
-                    // relative L2 loss (y - t)^2 / (sg(y)^2 + 0.01) and its gradient
-                    float lsum = 0.f;
-                    uint8_t* dy = a.act + (size_t)tile * ACT_BYTES + ACT_DY;
-                    uint8_t* dyt = a.act + (size_t)tile * ACT_BYTES + ACT_DYT;
-                    for (int j = 0; j < OUTP; ++j) {
-                        float g = 0.f;
-                        if (live && j < a.n_out) {
-                            const float t = a.target[(size_t)pt * a.tstride + j];   // the target of the sample's point
-                            const float d = v[j] - t, den = v[j] * v[j] + 0.01f;
-                            lsum += d * d / den;
-                            g = 2.f * d / den * a.loss_scale * sc;
-                        }
-                        st_bf16(dy, kmajor_offset(row, j, OUTP), g);
-                        st_bf16(dyt, kmajor_offset(j, row, 128), g);
-                    }
-                    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-                    if (lane == 0 && lsum != 0.f) atomicAdd(a.loss, lsum);
+                    relu_pack(v, lo4, hi4);
+                    *reinterpret_cast<uint4*>(sx + kmajor_offset(row, c, HID)) = lo4;
+                    *reinterpret_cast<uint4*>(sx + kmajor_offset(row, c + 8, HID)) = hi4;
+                } else if (live) {
+                    for (int j = 0; j < a.n_out; ++j) a.out[(size_t)s * a.ostride + j] = v[j];
                 }
             }
             fence_before_sync();
             fence_proxy_async();
             gsync();
-            if (TRAIN && l < NLAYER - 1) {
-                uint4* dst = reinterpret_cast<uint4*>(a.act + (size_t)tile * ACT_BYTES + act_ht(l + 1));
-                for (int i = tid; i < HID * 128 * 2 / 16; i += FWD_THREADS) dst[i] = reinterpret_cast<const uint4*>(st)[i];
-                gsync();
-            }
             fence_after_sync();
         }
     }
@@ -368,146 +317,268 @@ __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(sdst)), "l"(gsrc) : "memory");
 }
 
-// Backward pass (128 threads per CTA, one CTA per SM, tiles blockIdx.x, blockIdx.x + gridDim.x,
-// ... in that order): for each tile and l = 4 .. 0, dW_l += dZ_l^T A_l over the tile's samples
-// (rows of dZ^T beyond the layer's outputs are zero) and, for l >= 1,
-// dZ_{l-1} = (dZ_l W_l) masked by ReLU'(H_l).  The weight gradients of all five layers stay in
-// tensor memory across the CTA's tiles (the MMAs accumulate into them; columns bw_dw_col(l),
-// 432 in all) and leave once, as the CTA's slot of dwpart; dZ_l W_l goes to columns BW_DA ..
-// BW_DA + 63, per tile.  The transposed weights stay in shared memory for the whole kernel;
-// each step's activation tile A_l^T is loaded into one of two buffers while the step before
-// runs its products and its epilogue (and the next tile's dY, dY^T while its layers 3 .. 0
-// run).  The tile order within a CTA and the number of CTAs are fixed, so the sums are
-// reproducible.
-constexpr uint32_t BW_COLS = 512;
-constexpr uint32_t BW_DA = 448;
-__host__ __device__ constexpr uint32_t bw_dw_col(int l) { return l == 0 ? 0u : (uint32_t)(K0 + (l - 1) * HID); }
-static_assert(bw_dw_col(NLAYER - 1) + HID <= BW_DA && BW_DA + HID <= BW_COLS, "tensor-memory columns of the backward pass");
-// shared-memory carve-up (bytes)
-constexpr int BS_SAT = K0 * 128 * 2;                 // one A_l^T buffer (the largest, layer 0)
-constexpr int BS_SWT = 2 * BS_SAT;                   // W_l^T of layers 1..4 (WB_BYTES)
-constexpr int BS_SDZ = BS_SWT + WB_BYTES;            // dZ, 128 x 64 (K-major)
-constexpr int BS_SDZT = BS_SDZ + 128 * HID * 2;      // dZ^T, 128 x 128 (rows 64.. zero)
-constexpr int BS_SDY = BS_SDZT + 128 * 128 * 2;      // dY, 128 x 16 (K-major)
-constexpr int BS_SDYT = BS_SDY + 128 * OUTP * 2;     // dY^T, 128 x 128 (rows 16.. zero)
-constexpr int BS_END = BS_SDYT + 128 * 128 * 2;      // 202,752
-__global__ void __launch_bounds__(128) k_mlp_backward(const MlpArgs a, int ntiles) {
+// n MMAs along K from base descriptors that advance by astep / bstep bytes each: an addition to the
+// start address field (shared memory ends below its 2^18), so the one issuing thread spends a few
+// instructions per MMA.  Rolled, like the loops over the layers below: a tile runs this code a few
+// times only, and unrolled the instruction fetches cost more than the loops (60 us a step, not 49).
+__device__ __forceinline__ void mma_chain(uint32_t d, uint64_t adesc, uint32_t astep, uint64_t bdesc, uint32_t bstep, int n, uint32_t idesc,
+                                          bool fresh) {
+    uint32_t acc = fresh ? 0u : 1u;
+#pragma unroll 1
+    for (int kk = 0; kk < n; ++kk) {
+        mma_bf16(d, adesc, bdesc, idesc, acc);
+        adesc += astep >> 4;
+        bdesc += bstep >> 4;
+        acc = 1u;
+    }
+}
+
+// One training step's forward and backward pass: one CTA per SM over the tiles blockIdx.x,
+// blockIdx.x + gridDim.x, ... of 128 samples, in that order, each tile forward and then backward
+// while its activations are in shared memory.
+//
+// Warps 0..7 are the chain: they take each product out of tensor memory, form the next operand and
+// hand it over (row = sample; the two threads of a row split the columns).  One thread of warp 16
+// issues the products as the operands arrive, so that no warp of the chain spends its time on
+// that; warps 8..15 encode the next tile's features meanwhile, into the other of two X0 buffers.
+// Layer l's forward product goes to columns TR_DA .. of the tensor memory and back to shared memory
+// as H_{l+1} = bf16(ReLU).  Backward, for l = 4 .. 0:
+//     dZ_{l-1} = (dZ_l W_l) masked by ReLU'(H_l)   (issued first, its result waited for)
+//     dW_l += dZ_l^T A_l over the tile's samples   (issued behind it, runs during the epilogue)
+// dZ_l is stored as its rows (samples) by columns (features); the first product reads it K-major, the
+// second with the samples as K, M-major, and likewise A_l and W_l with the other index as K, so no
+// transposed copy of anything is made.  (dZ_l^T has out_dim(l) rows of the 128 the instruction
+// takes: the rows beyond read whatever follows in shared memory and land in lanes that nothing
+// reads.)  The weight gradients stay in tensor memory across the CTA's tiles (columns tr_dw_col(l))
+// and leave once, as the CTA's slot of dwpart; the tile order within a CTA and the number of CTAs
+// are fixed, so the sums are reproducible.
+//
+// Buffers: dZ_3 has one of its own, then dZ_2, dZ_1, dZ_0 take the places of H_4, H_3, H_2, whose
+// last readers (dW_4, dW_3, dW_2) come before the product that the epilogue has just waited for.
+//
+// Bound by the latency of the chain (nine products, each waited for and passed through registers) at
+// one tile per SM: the weights, two X0 buffers and the activations take 222 KB.
+// 65,536 samples (512 tiles, four rounds): 42 us, 7.6 us a tile; as a forward kernel that wrote
+// activations and their transposes to global memory and a backward kernel that read them, 45 + 54 us.
+// With the chain's first warp issuing the products it took 50 us.
+constexpr int TR_CHAIN = 256;                        // threads of the chain
+constexpr int TR_ENCODE = 256;                       // threads that encode
+constexpr int TR_THREADS = TR_CHAIN + TR_ENCODE + 32;
+constexpr uint32_t TR_COLS = 512, TR_DA = 448;
+__host__ __device__ constexpr uint32_t tr_dw_col(int l) { return l == 0 ? 0u : (uint32_t)(K0 + (l - 1) * HID); }
+static_assert(tr_dw_col(NLAYER - 1) + HID <= TR_DA && TR_DA + HID <= TR_COLS, "tensor-memory columns of a training step");
+constexpr int TS_X = WF_BYTES;                       // X0, two buffers of 128 x 176
+constexpr int TS_H = TS_X + 2 * 128 * K0 * 2;        // H_1 .. H_4, 128 x 64 each
+constexpr int TS_E = TS_H + 4 * 128 * HID * 2;       // dZ_3
+constexpr int TS_DY = TS_E + 128 * HID * 2;          // dZ_4, 128 x 16
+constexpr int TS_END = TS_DY + 128 * OUTP * 2 + 2048;   // 2 KB that the rows beyond dZ_4^T's 16 may read
+constexpr size_t TRAIN_SMEM = (size_t)TS_END;
+static_assert(TRAIN_SMEM > 114 * 1024 && TRAIN_SMEM <= 226 * 1024, "one training CTA per SM, all of its tensor memory");
+// named barriers: an operand handed over by the chain; an X0 buffer full, empty (one of each per buffer)
+enum TrainBar { TB_CHAIN = 1, TB_FULL = 2, TB_EMPTY = 4 };
+
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+__global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int ntiles) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tmem_base;
-    uint8_t* sat[2] = {smem, smem + BS_SAT};
-    uint8_t* swt = smem + BS_SWT;
-    uint8_t* sdz = smem + BS_SDZ;
-    uint8_t* sdzt = smem + BS_SDZT;
-    uint8_t* sdy = smem + BS_SDY;
-    uint8_t* sdyt = smem + BS_SDYT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < 128 * 128 * 2 / 16; i += 128) {
-        reinterpret_cast<uint4*>(sdzt)[i] = make_uint4(0u, 0u, 0u, 0u);
-        reinterpret_cast<uint4*>(sdyt)[i] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    __syncthreads();
-    // the transposed weights, once; the first tile's dY, dY^T and A_4^T
-    for (int i = tid; i < WB_BYTES / 16; i += 128) cp_async16(reinterpret_cast<uint4*>(swt) + i, reinterpret_cast<const uint4*>(a.wbf + WF_BYTES) + i);
-    auto load_dy = [&](int tile) {
-        const uint8_t* act = a.act + (size_t)tile * ACT_BYTES;
-        for (int i = tid; i < 128 * OUTP * 2 / 16; i += 128) cp_async16(reinterpret_cast<uint4*>(sdy) + i, reinterpret_cast<const uint4*>(act + ACT_DY) + i);
-        for (int i = tid; i < OUTP * 128 * 2 / 16; i += 128) cp_async16(reinterpret_cast<uint4*>(sdyt) + i, reinterpret_cast<const uint4*>(act + ACT_DYT) + i);
-    };
-    auto load_at = [&](int tile, int l, uint8_t* dst) {
-        const uint4* src = reinterpret_cast<const uint4*>(a.act + (size_t)tile * ACT_BYTES + (l == 0 ? ACT_X0T : act_ht(l)));
-        for (int i = tid; i < in_dim(l) * 128 * 2 / 16; i += 128) cp_async16(reinterpret_cast<uint4*>(dst) + i, src + i);
-    };
-    load_dy(blockIdx.x);
-    load_at(blockIdx.x, NLAYER - 1, sat[0]);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    constexpr int W_ENCODE = TR_CHAIN / 32, W_ISSUE = (TR_CHAIN + TR_ENCODE) / 32;
     if (tid == 0) mbar_init(&mbar, 1);
-    if (warp == 0) tmem_alloc(&tmem_base, BW_COLS);
+    if (warp == W_ISSUE) tmem_alloc(&tmem_base, TR_COLS);
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    const uint32_t tmem = tmem_base;
-    uint32_t phase = 0;
-    int step = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const bool first = tile == (int)blockIdx.x;
-        for (int l = NLAYER - 1; l >= 0; --l, ++step) {
-            const int Kin = in_dim(l), Nout = out_dim(l);
-            uint8_t* cur = sat[step & 1];
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const uint32_t tmem = tmem_base, sm0 = smem_u32(smem);
+    const int count = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // tiles of this CTA
+    auto hbuf = [](int l) { return (uint32_t)(TS_H + (l - 1) * (128 * HID * 2)); };
+    auto xbuf = [](int it) { return (uint32_t)(TS_X + (it & 1) * (128 * K0 * 2)); };
+    if (warp == W_ISSUE) {
+        // the products, in the order of their operands; never waits for a product itself
+        for (int it = 0; it < count; ++it) {
+            if (it == 0) bar_sync(TB_CHAIN, TR_CHAIN + 32);   // the weights
+            bar_sync(TB_FULL + (it & 1), TR_ENCODE + 32);
+#pragma unroll 1
+            for (int l = 0; l < NLAYER; ++l) {
+                if (l > 0) bar_sync(TB_CHAIN, TR_CHAIN + 32);
+                fence_after_sync();
+                if (lane == 0) {
+                    const uint32_t K = (uint32_t)in_dim(l);
+                    mma_chain(tmem + TR_DA, smem_desc(sm0 + (l == 0 ? xbuf(it) : hbuf(l)), 128u, 16u * K), 256u,
+                              smem_desc(sm0 + wf_off(l), 128u, 16u * K), 256u, (int)K / 16, idesc_bf16_f32(128, out_dim(l)), true);
+                    mma_commit(&mbar);
+                }
+                __syncwarp();
+            }
+#pragma unroll 1
+            for (int l = NLAYER - 1; l >= 0; --l) {
+                bar_sync(TB_CHAIN, TR_CHAIN + 32);
+                fence_after_sync();
+                if (lane == 0) {
+                    const uint32_t Kin = (uint32_t)in_dim(l), Nout = (uint32_t)out_dim(l);
+                    const uint32_t z = sm0 + (l == 4 ? (uint32_t)TS_DY : (l == 3 ? (uint32_t)TS_E : hbuf(l + 2)));
+                    if (l >= 1) {
+                        mma_chain(tmem + TR_DA, smem_desc(z, 128u, 16u * Nout), 256u, smem_desc(sm0 + wf_off(l), 16u * HID, 128u), 32u * HID,
+                                  (int)Nout / 16, idesc_bf16_f32(128, HID, false, true), true);
+                        mma_commit(&mbar);
+                    }
+                    mma_chain(tmem + tr_dw_col(l), smem_desc(z, 16u * Nout, 128u), 32u * Nout,
+                              smem_desc(sm0 + (l == 0 ? xbuf(it) : hbuf(l)), 16u * Kin, 128u), 32u * Kin, 8, idesc_bf16_f32(128, (int)Kin, true, true),
+                              it == 0);
+                    if (l == 0 && it == count - 1) mma_commit(&mbar);   // the last dW_0
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp >= W_ENCODE) {
+        const int et = tid - TR_CHAIN, row = et & 127, half = et >> 7;
+        for (int it = 0; it < count; ++it) {
+            const int s = ((int)blockIdx.x + it * (int)gridDim.x) * 128 + row;
+            const int pt = a.idx ? a.idx[s] : s;
+            uint8_t* sx = smem + xbuf(it);
+            if (it >= 2) bar_sync(TB_EMPTY + (it & 1), TR_CHAIN + TR_ENCODE);
+            encode(a, pt, half, [&](int k8, const float (&f)[8]) {
+                *reinterpret_cast<uint4*>(sx + kmajor_offset(row, 8 * k8, K0)) = pack8(f);
+            });
             fence_proxy_async();
-            __syncthreads();
-            if (tid == 0) {
-                const uint32_t zt = smem_u32(l == NLAYER - 1 ? sdyt : sdzt), at = smem_u32(cur);
-                for (int kk = 0; kk < 8; ++kk)
-                    mma_bf16(tmem + bw_dw_col(l), smem_desc(zt + 256u * kk, 128u, 16u * 128), smem_desc(at + 256u * kk, 128u, 16u * 128),
-                             idesc_bf16_f32(128, Kin), (kk > 0 || !first) ? 1u : 0u);
-                if (l >= 1) {
-                    const uint32_t z = smem_u32(l == NLAYER - 1 ? sdy : sdz), w = smem_u32(swt + (wb_off(l) - WF_BYTES));
-                    for (int kk = 0; kk < Nout / 16; ++kk)
-                        mma_bf16(tmem + BW_DA, smem_desc(z + 256u * kk, 128u, 16u * Nout), smem_desc(w + 256u * kk, 128u, 16u * Nout),
-                                 idesc_bf16_f32(128, HID), kk > 0);
-                }
-                mma_commit(&mbar);
+            bar_arrive(TB_FULL + (it & 1), TR_ENCODE + 32);
+        }
+    } else {
+        const int quarter = warp & 3, half = warp >> 2, row = quarter * 32 + lane;
+        const uint32_t acc = tmem + TR_DA + ((uint32_t)(quarter * 32) << 16);
+        uint32_t phase = 0;
+        bool ok = true;
+        // Every warp watches the barrier itself.  A wait that gives up is the last one: the chain goes
+        // on through its barriers, so that nobody waits for it, and the error flag stays set.
+        auto wait = [&]() {
+            if (ok && !mbar_wait(&mbar, phase, WAIT_LIMIT)) {
+                ok = false;
+                if (lane == 0) atomicOr(a.err, 1u);
             }
-            // the next step's operands, into the other buffer, while this one runs
-            if (l > 0) {
-                load_at(tile, l - 1, sat[(step + 1) & 1]);
-            } else if (tile + (int)gridDim.x < ntiles) {
-                load_dy(tile + gridDim.x);
-                load_at(tile + gridDim.x, NLAYER - 1, sat[(step + 1) & 1]);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            bool seen = true;
-            if (warp == 0) {   // one warp watches the barrier (see k_mlp_forward)
-                seen = mbar_wait(&mbar, phase, WAIT_LIMIT);
-                fence_before_sync();
-            }
-            ok = __syncthreads_and(seen);
             phase ^= 1u;
-            if (!ok) {
-                if (tid == 0) atomicOr(a.err, 1u);
-                break;
-            }
             fence_after_sync();
-            if (l >= 1) {
-                // dZ_{l-1} = (dZ_l W_l) * [H_l > 0], row = sample
-                const int m = tid;
-                for (int c = 0; c < HID; c += 16) {
-                    float v[16];
-                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + BW_DA + (uint32_t)c, v);
-                    tmem_wait_ld();
-                    for (int j = 0; j < 16; ++j) {
-                        const int k = c + j;
-                        const float h = bf16_at(cur, kmajor_offset(k, m, 128));
-                        v[j] = h > 0.f ? v[j] : 0.f;
-                    }
-                    for (int j = 0; j < 16; ++j) {
-                        st_bf16(sdz, kmajor_offset(m, c + j, HID), v[j]);
-                        st_bf16(sdzt, kmajor_offset(c + j, m, 128), v[j]);
-                    }
-                }
-            }
+        };
+        auto handover = [&]() {   // this thread's writes to shared memory, and its reads of the accumulator, before the next product
             fence_before_sync();
             fence_proxy_async();
-            __syncthreads();
-            fence_after_sync();
+            bar_arrive(TB_CHAIN, TR_CHAIN + 32);
+        };
+        for (int i = tid; i < WF_BYTES / 16; i += TR_CHAIN) cp_async16(smem + 16 * i, a.wbf + 16 * i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float sc = __ldg(a.scale);   // loss scale (a power of two)
+        auto point = [&](int it) {
+            const int s = ((int)blockIdx.x + it * (int)gridDim.x) * 128 + row;
+            return a.idx ? a.idx[s] : s;
+        };
+        int pt = point(0);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        handover();
+        for (int it = 0; it < count; ++it) {
+            // the sample's targets and the next tile's points, fetched ahead of their use
+            const float* tg = a.target + (size_t)pt * a.tstride;
+            float t4[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t4[j] = half == 0 && j < a.n_out ? tg[j] : 0.f;
+            if (it + 1 < count) pt = point(it + 1);
+#pragma unroll 1
+            for (int l = 0; l < NLAYER; ++l) {
+                wait();
+                // (this product came behind everything before it: the other X0 buffer has been read)
+                if (l == 0 && it > 0 && it + 1 < count) bar_arrive(TB_EMPTY + ((it + 1) & 1), TR_CHAIN + TR_ENCODE);
+                if (l < NLAYER - 1) {
+                    float v[2][16];
+                    tmem_ld16(acc + 32u * half, v[0]);
+                    tmem_ld16(acc + 32u * half + 16u, v[1]);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint4 lo4, hi4;
+                        relu_pack(v[h], lo4, hi4);
+                        uint8_t* dst = smem + hbuf(l + 1) + kmajor_offset(row, 32 * half + 16 * h, HID);
+                        *reinterpret_cast<uint4*>(dst) = lo4;
+                        *reinterpret_cast<uint4*>(dst + 128) = hi4;
+                    }
+                    handover();
+                } else {
+                    // relative L2 loss (y - t)^2 / (sg(y)^2 + 0.01) and its gradient
+                    float lsum = 0.f;
+                    if (half == 0) {
+                        float v[16];
+                        tmem_ld16(acc, v);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < OUTP; ++j) {
+                            float g = 0.f;
+                            if (j < a.n_out) {
+                                const float t = j < 4 ? t4[j & 3] : tg[j];
+                                const float d = v[j] - t, den = v[j] * v[j] + 0.01f;
+                                lsum += d * d / den;
+                                g = 2.f * d / den * a.loss_scale * sc;
+                            }
+                            v[j] = g;
+                        }
+                        uint8_t* dst = smem + TS_DY + kmajor_offset(row, 0, OUTP);
+                        *reinterpret_cast<uint4*>(dst) =
+                            make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+                        *reinterpret_cast<uint4*>(dst + 128) =
+                            make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]), pack_bf16(v[14], v[15]));
+                    }
+                    handover();
+                    if (half == 0) {
+                        for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+                        if (lane == 0 && lsum != 0.f) atomicAdd(a.loss, lsum);
+                    }
+                }
+            }
+#pragma unroll 1
+            for (int l = NLAYER - 1; l >= 1; --l) {
+                const uint32_t off = kmajor_offset(row, 32 * half, HID);
+                uint4 h[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) h[q] = *reinterpret_cast<const uint4*>(smem + hbuf(l) + off + 128 * q);
+                wait();
+                const uint32_t zn = l == 4 ? (uint32_t)TS_E : hbuf(l + 1);
+                float v[2][16];
+                tmem_ld16(acc + 32u * half, v[0]);
+                tmem_ld16(acc + 32u * half + 16u, v[1]);
+                tmem_wait_ld();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint32_t hw[4] = {h[q].x, h[q].y, h[q].z, h[q].w};
+                    uint32_t zw[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162*>(&hw[j]);
+                        const float lo = v[q >> 1][8 * (q & 1) + 2 * j], hi = v[q >> 1][8 * (q & 1) + 2 * j + 1];
+                        zw[j] = pack_bf16(__low2float(b) > 0.f ? lo : 0.f, __high2float(b) > 0.f ? hi : 0.f);
+                    }
+                    *reinterpret_cast<uint4*>(smem + zn + off + 128 * q) = make_uint4(zw[0], zw[1], zw[2], zw[3]);
+                }
+                handover();
+            }
         }
+        wait();   // the last dW_0
+        fence_before_sync();
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // the CTA's weight gradients: rows = outputs (warps 0 and 1 hold rows 0..63), 16-byte stores
-    if (ok && warp < 2) {
-        const int row = warp * 32 + lane;
+    __syncthreads();
+    fence_after_sync();
+    // the CTA's weight gradients: rows = outputs 0..63, in the lanes of the warps 0 and 1 of each four
+    if (warp < W_ISSUE && (warp & 3) < 2) {
+        const int row = (warp & 3) * 32 + lane;
         float* dw = a.dwpart + (size_t)blockIdx.x * NWEIGHT;
+        int piece = 0;
         for (int l = 0; l < NLAYER; ++l) {
             const int Kin = in_dim(l), Nout = out_dim(l);
-            for (int c = 0; c < Kin; c += 16) {
+            for (int c = 0; c < Kin; c += 16, ++piece) {
+                if ((piece & 3) != warp >> 2) continue;
                 float v[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + bw_dw_col(l) + (uint32_t)c, v);
+                tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + tr_dw_col(l) + (uint32_t)c, v);
                 tmem_wait_ld();
                 if (row < Nout) {
                     float4* d4 = reinterpret_cast<float4*>(dw + master_off(l) + row * Kin + c);
+#pragma unroll
                     for (int j = 0; j < 4; ++j) d4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
                 }
             }
@@ -515,100 +586,110 @@ __global__ void __launch_bounds__(128) k_mlp_backward(const MlpArgs a, int ntile
     }
     fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, BW_COLS);
+    if (warp == W_ISSUE) tmem_dealloc(tmem, TR_COLS);
 }
 
-// Master weights (FP32, [out][in] per layer) -> bf16 tiles: W_l (rows out, K in) and, for
-// layers 1..4, W_l^T (rows in, K out).
-__global__ void k_mlp_pack(const float* __restrict__ w, uint8_t* __restrict__ wbf) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NWEIGHT) return;
+// byte offset of master weight i in the bf16 tiles
+__device__ __forceinline__ uint32_t tile_offset(int i) {
     int l = 0;
     while (l + 1 < NLAYER && i >= master_off(l + 1)) ++l;
     const int K = in_dim(l), r = (i - master_off(l)) / K, k = (i - master_off(l)) % K;
-    const float v = w[i];
-    st_bf16(wbf + wf_off(l), kmajor_offset(r, k, K), v);
-    if (l >= 1) st_bf16(wbf + wb_off(l), kmajor_offset(k, r, out_dim(l)), v);
+    return wf_off(l) + kmajor_offset(r, k, K);
 }
 
-// Gradient of each weight = the tile gradients added in a fixed order (reproducible): slice s
-// of GSLICES adds tiles s, s + GSLICES, ... in order, then the slices are added in order; then
-// one Adam step on the FP32 master weight, and its bf16 copies.
-constexpr int GSLICES = 16;
-__global__ void k_mlp_gsum(const float* __restrict__ part, int ntiles, float* __restrict__ slices) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.y;
-    if (i >= NWEIGHT) return;
-    float g = 0.f;
-    for (int t = s; t < ntiles; t += GSLICES) g += part[(size_t)t * NWEIGHT + i];
-    slices[(size_t)s * NWEIGHT + i] = g;
+// Master weights (FP32, [out][in] per layer) -> bf16 tiles.
+__global__ void k_mlp_pack(const float* __restrict__ w, uint8_t* __restrict__ wbf) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < NWEIGHT) st_bf16(wbf, tile_offset(i), w[i]);
 }
+
 // Loss scaling.  The output gradient is multiplied by a power-of-two scale before it goes
 // through the bf16 backward pass and divided out of the summed weight gradient (exact for a power
 // of two, barring overflow).  A step whose summed gradient is not finite is skipped and the
 // scale halved; after SCALE_RUN finite steps in a row it doubles, up to SCALE_MAX.
-// Device state, floats: scale for the next step, steps applied, finite steps in a row, steps
-// skipped, Adam's bias corrections c1 and c2 of this step, 1 / the scale of this step.
-enum MlpState { ST_SCALE = 0, ST_STEPS, ST_RUN, ST_SKIPPED, ST_C1, ST_C2, ST_INV, ST_COUNT };
+// Device state, floats: scale for the next step, steps applied, finite steps in a row, steps skipped.
+enum MlpState { ST_SCALE = 0, ST_STEPS, ST_RUN, ST_SKIPPED, ST_COUNT };
 constexpr float SCALE_MAX = 65536.f;
 constexpr int SCALE_RUN = 1000;
-__global__ void k_mlp_gcheck(const float* __restrict__ slices, unsigned* __restrict__ nonfinite) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NWEIGHT) return;
-    float g = 0.f;
-    for (int s = 0; s < GSLICES; ++s) g += slices[(size_t)s * NWEIGHT + i];
-    if (!isfinite(g)) atomicOr(nonfinite, 1u);
-}
-__global__ void k_mlp_step(float* __restrict__ st, const unsigned* __restrict__ nonfinite, float b1, float b2) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    st[ST_INV] = 1.f / st[ST_SCALE];
-    if (*nonfinite) {
-        st[ST_SCALE] = fmaxf(st[ST_SCALE] * 0.5f, 1.f);
-        st[ST_RUN] = 0.f;
-        st[ST_SKIPPED] += 1.f;
-        return;
+// words beside the state: a gradient of this step is not finite; blocks that have read the state
+enum MlpWord { WD_NONFINITE = 0, WD_TICKET, WD_COUNT };
+
+// Gradient of each weight = the CTAs' gradients added in a fixed order (reproducible): slice s
+// of GSLICES adds CTAs s, s + GSLICES, ... in order, then the slices are added in order.  A block
+// sums 64 weights, one thread per four weights and slice, all of a thread's loads in flight.
+// 152 CTAs' gradients, 15 MB in the L2: 6.7 us (with the loss scale's step at its end 9 us).
+constexpr int GSLICES = 16, GWEIGHTS = 64;
+static_assert(NWEIGHT % GWEIGHTS == 0, "whole blocks of weights");
+__global__ void __launch_bounds__(GSLICES * GWEIGHTS / 4) k_mlp_gsum(const float* __restrict__ part, int nctas, float* __restrict__ gsum,
+                                                                     unsigned* __restrict__ words) {
+    __shared__ float slice[GSLICES][GWEIGHTS];
+    const int w4 = threadIdx.x % (GWEIGHTS / 4), s = threadIdx.x / (GWEIGHTS / 4);
+    const float4* p = reinterpret_cast<const float4*>(part) + blockIdx.x * (GWEIGHTS / 4) + w4;
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 5
+    for (int t = s; t < nctas; t += GSLICES) {
+        const float4 x = p[(size_t)t * (NWEIGHT / 4)];
+        g.x += x.x;
+        g.y += x.y;
+        g.z += x.z;
+        g.w += x.w;
     }
-    // Adam's bias corrections 1 / (1 - b^t), in FP32 (a double pow is a long chain of the GPU's
-    // slow FP64 operations on one thread: about 9 us per step)
-    const float t = st[ST_STEPS] + 1.f;
-    st[ST_STEPS] = t;
-    st[ST_C1] = 1.f / (1.f - powf(b1, t));
-    st[ST_C2] = 1.f / (1.f - powf(b2, t));
-    st[ST_RUN] += 1.f;
-    if (st[ST_RUN] >= (float)SCALE_RUN) {
-        st[ST_SCALE] = fminf(st[ST_SCALE] * 2.f, SCALE_MAX);
-        st[ST_RUN] = 0.f;
-    }
-}
-__global__ void k_mlp_adam(const float* __restrict__ slices, float* __restrict__ w, float* __restrict__ m1, float* __restrict__ m2,
-                           float* __restrict__ grad, uint8_t* __restrict__ wbf, float lr, float b1, float b2, float eps,
-                           const float* __restrict__ st, const unsigned* __restrict__ nonfinite) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NWEIGHT || *nonfinite) return;
-    const float c1 = st[ST_C1], c2 = st[ST_C2];
-    float g = 0.f;
-    for (int s = 0; s < GSLICES; ++s) g += slices[(size_t)s * NWEIGHT + i];
-    g *= st[ST_INV];
-    grad[i] = g;
-    const float m = b1 * m1[i] + (1.f - b1) * g;
-    const float v = b2 * m2[i] + (1.f - b2) * g * g;
-    m1[i] = m;
-    m2[i] = v;
-    const float x = w[i] - lr * (m * c1) / (sqrtf(v * c2) + eps);
-    w[i] = x;
-    int l = 0;
-    while (l + 1 < NLAYER && i >= master_off(l + 1)) ++l;
-    const int K = in_dim(l), r = (i - master_off(l)) / K, k = (i - master_off(l)) % K;
-    st_bf16(wbf + wf_off(l), kmajor_offset(r, k, K), x);
-    if (l >= 1) st_bf16(wbf + wb_off(l), kmajor_offset(k, r, out_dim(l)), x);
+    *reinterpret_cast<float4*>(&slice[s][4 * w4]) = g;
+    __syncthreads();
+    if (threadIdx.x >= GWEIGHTS) return;
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < GSLICES; ++k) sum += slice[k][threadIdx.x];
+    gsum[blockIdx.x * GWEIGHTS + threadIdx.x] = sum;
+    if (!isfinite(sum)) atomicOr(words + WD_NONFINITE, 1u);
 }
 
-constexpr size_t FWD_SMEM_INFER = (size_t)WF_BYTES + INFER_GROUPS * GROUP_SMEM_INFER;   // 224 KB: one CTA per SM
-constexpr int TRAIN_GROUPS = 2;                                  // tiles in flight per training-forward CTA
-constexpr size_t FWD_SMEM_TRAIN = (size_t)WF_BYTES + TRAIN_GROUPS * GROUP_SMEM_TRAIN;   // 224 KB
-// operands of the backward pass (more than half an SM's shared memory: one CTA per SM, each
-// holding all 512 tensor-memory columns)
-constexpr size_t BWD_SMEM = (size_t)BS_END;
-static_assert(BWD_SMEM > 114 * 1024 && BWD_SMEM <= 227 * 1024, "backward shared memory");
+// One Adam step on the FP32 master weights, and their bf16 copies; the loss scale's step.  Every
+// thread reads the state of before the step and forms Adam's bias corrections 1 / (1 - b^t) itself,
+// in FP32 (a double pow is a long chain of the GPU's slow FP64 operations); the last block to have
+// read the state writes the next one.
+__global__ void __launch_bounds__(128) k_mlp_adam(const float* __restrict__ gsum, float* __restrict__ w, float* __restrict__ m1,
+                                                  float* __restrict__ m2, float* __restrict__ grad, uint8_t* __restrict__ wbf, float lr, float b1,
+                                                  float b2, float eps, float* st, unsigned* words) {
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    const float4 s = __ldcg(reinterpret_cast<const float4*>(st));
+    const bool skip = __ldcg(words + WD_NONFINITE) != 0u;
+    const float scale = s.x, t = s.y + 1.f;
+    if (i < NWEIGHT && !skip) {
+        const float c1 = 1.f / (1.f - powf(b1, t)), c2 = 1.f / (1.f - powf(b2, t));
+        const float g = gsum[i] * (1.f / scale);
+        grad[i] = g;
+        const float m = b1 * m1[i] + (1.f - b1) * g;
+        const float v = b2 * m2[i] + (1.f - b2) * g * g;
+        m1[i] = m;
+        m2[i] = v;
+        const float x = w[i] - lr * (m * c1) / (sqrtf(v * c2) + eps);
+        w[i] = x;
+        st_bf16(wbf, tile_offset(i), x);
+    }
+    __syncthreads();   // the block's threads have read the state
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(words + WD_TICKET, 1u) != gridDim.x - 1) return;
+    words[WD_TICKET] = 0u;
+    words[WD_NONFINITE] = 0u;   // ready for the next step
+    float4 n = s;
+    if (skip) {
+        n.x = fmaxf(scale * 0.5f, 1.f);
+        n.z = 0.f;
+        n.w += 1.f;
+    } else {
+        n.y = t;
+        n.z += 1.f;
+        if (n.z >= (float)SCALE_RUN) {
+            n.x = fminf(scale * 2.f, SCALE_MAX);
+            n.z = 0.f;
+        }
+    }
+    *reinterpret_cast<float4*>(st) = n;
+}
+
+constexpr size_t INFER_SMEM = (size_t)WF_BYTES + INFER_GROUPS * GROUP_SMEM;   // 224 KB: one CTA per SM
 }  // namespace
 
 extern "C" rc_status rc_mlp_tile_product(const uint16_t* d_a, const uint16_t* d_b, float* d_d, int K, int N, unsigned* d_err,
@@ -634,32 +715,14 @@ struct rc_mlp {
     rc_mlp_config cfg{};
     cudaStream_t stream = nullptr;
     bool own_stream = false;
-    float *w = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr, *part = nullptr, *slices = nullptr, *loss = nullptr;
+    float *w = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr, *part = nullptr, *gsum = nullptr, *loss = nullptr;
     float* state = nullptr;     // loss scale and Adam step state (MlpState)
-    uint8_t *wbf = nullptr, *act = nullptr;
+    uint8_t* wbf = nullptr;
     unsigned* err = nullptr;
-    unsigned* nonfinite = nullptr;
+    unsigned* words = nullptr;  // MlpWord
     int cap_tiles = 0, sms = 0;
     long long step = 0;
     std::string msg;
-    // A training step's launches (2 memsets, 6 kernels) as CUDA graphs, one per set of arguments
-    // that came twice in a row (a caller that trains on the same buffers every frame replays one
-    // graph per call; arguments seen once are launched directly)
-    struct StepArgs {
-        const void *P = nullptr, *N = nullptr, *aux = nullptr, *target = nullptr, *idx = nullptr;
-        int tstride = 0, n = 0;
-        const float* loss = nullptr;
-        bool operator==(const StepArgs& o) const {
-            return P == o.P && N == o.N && aux == o.aux && target == o.target && idx == o.idx && tstride == o.tstride && n == o.n &&
-                   loss == o.loss;
-        }
-    };
-    struct StepGraph {
-        StepArgs args;
-        cudaGraphExec_t exec;
-    };
-    std::vector<StepGraph> graphs;
-    StepArgs last;
 };
 
 namespace {
@@ -711,11 +774,9 @@ rc_status rc_mlp_create(const rc_mlp_config* cfg, rc_mlp** out) {
     cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, cfg->device);
     m->cap_tiles = (cfg->max_batch + 127) / 128;
     if (cudaMalloc(&m->w, 4 * NWEIGHT) || cudaMalloc(&m->m1, 4 * NWEIGHT) || cudaMalloc(&m->m2, 4 * NWEIGHT) ||
-        cudaMalloc(&m->grad, 4 * NWEIGHT) || cudaMalloc(&m->wbf, WF_BYTES + WB_BYTES) || cudaMalloc(&m->err, 4) ||
+        cudaMalloc(&m->grad, 4 * NWEIGHT) || cudaMalloc(&m->wbf, WF_BYTES) || cudaMalloc(&m->err, 4) ||
         cudaMalloc(&m->loss, 4) || cudaMalloc(&m->part, (size_t)4 * NWEIGHT * std::max(1, std::min(m->cap_tiles, m->sms))) ||
-        cudaMalloc(&m->slices, (size_t)4 * NWEIGHT * GSLICES) ||
-        cudaMalloc(&m->act, (size_t)ACT_BYTES * m->cap_tiles) || cudaMalloc(&m->state, 4 * ST_COUNT) ||
-        cudaMalloc(&m->nonfinite, 4))
+        cudaMalloc(&m->gsum, 4 * NWEIGHT) || cudaMalloc(&m->state, 4 * ST_COUNT) || cudaMalloc(&m->words, 4 * WD_COUNT))
         return bad(RC_ERR_NOMEM);
     {
         float st0[ST_COUNT] = {0};
@@ -739,11 +800,11 @@ rc_status rc_mlp_create(const rc_mlp_config* cfg, rc_mlp** out) {
     rc_status s = rc_mlp_weights(m, w.data(), w.size(), 1);
     if (s != RC_OK) return bad(s);
     if (cudaMemsetAsync(m->m1, 0, 4 * NWEIGHT, m->stream) || cudaMemsetAsync(m->m2, 0, 4 * NWEIGHT, m->stream) ||
-        cudaMemsetAsync(m->err, 0, 4, m->stream) || cudaStreamSynchronize(m->stream))
+        cudaMemsetAsync(m->err, 0, 4, m->stream) || cudaMemsetAsync(m->words, 0, 4 * WD_COUNT, m->stream) ||
+        cudaStreamSynchronize(m->stream))
         return bad(RC_ERR_CUDA);
-    if (cudaFuncSetAttribute(k_mlp_forward<true, TRAIN_GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FWD_SMEM_TRAIN) ||
-        cudaFuncSetAttribute(k_mlp_forward<false, INFER_GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FWD_SMEM_INFER) ||
-        cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BWD_SMEM))
+    if (cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRAIN_SMEM) ||
+        cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INFER_SMEM))
         return bad(RC_ERR_CUDA);
     *out = m;
     return RC_OK;
@@ -752,9 +813,8 @@ rc_status rc_mlp_create(const rc_mlp_config* cfg, rc_mlp** out) {
 void rc_mlp_destroy(rc_mlp* m) {
     if (!m) return;
     if (m->stream) cudaStreamSynchronize(m->stream);
-    cudaFree(m->w); cudaFree(m->m1); cudaFree(m->m2); cudaFree(m->grad); cudaFree(m->part); cudaFree(m->slices);
-    cudaFree(m->loss); cudaFree(m->wbf); cudaFree(m->act); cudaFree(m->err); cudaFree(m->state); cudaFree(m->nonfinite);
-    for (auto& g : m->graphs) cudaGraphExecDestroy(g.exec);
+    cudaFree(m->w); cudaFree(m->m1); cudaFree(m->m2); cudaFree(m->grad); cudaFree(m->part);
+    cudaFree(m->loss); cudaFree(m->wbf); cudaFree(m->err); cudaFree(m->state); cudaFree(m->words); cudaFree(m->gsum);
     if (m->own_stream && m->stream) cudaStreamDestroy(m->stream);
     delete m;
 }
@@ -765,7 +825,6 @@ rc_status rc_mlp_weights(rc_mlp* m, float* host, size_t n, int to_device) {
     if (!m || !host || n != (size_t)NWEIGHT) return mfail(m, RC_ERR_ARG, "weights: 24576 floats");
     if (to_device) {
         if (cudaMemcpyAsync(m->w, host, 4 * NWEIGHT, cudaMemcpyHostToDevice, m->stream) != cudaSuccess) return mfail(m, RC_ERR_CUDA, "copy");
-        if (cudaMemsetAsync(m->wbf, 0, WF_BYTES + WB_BYTES, m->stream) != cudaSuccess) return mfail(m, RC_ERR_CUDA, "clear");
         k_mlp_pack<<<(NWEIGHT + 255) / 256, 256, 0, m->stream>>>(m->w, m->wbf);
         if (cudaGetLastError() != cudaSuccess) return mfail(m, RC_ERR_CUDA, "pack");
     } else if (cudaMemcpyAsync(host, m->w, 4 * NWEIGHT, cudaMemcpyDeviceToHost, m->stream) != cudaSuccess) {
@@ -782,26 +841,6 @@ rc_status rc_mlp_gradients(rc_mlp* m, float* host, size_t n) {
     return RC_OK;
 }
 
-namespace {
-// The launches of one training step on the network's stream.
-cudaError_t issue_train(rc_mlp* m, const MlpArgs& a, int ntiles, bool own_loss) {
-    cudaError_t e;
-    if (own_loss && (e = cudaMemsetAsync(m->loss, 0, 4, m->stream)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(m->nonfinite, 0, 4, m->stream)) != cudaSuccess) return e;
-    k_mlp_forward<true, TRAIN_GROUPS><<<std::min((ntiles + TRAIN_GROUPS - 1) / TRAIN_GROUPS, m->sms), FWD_THREADS * TRAIN_GROUPS,
-                                        FWD_SMEM_TRAIN, m->stream>>>(a);
-    const int bwd_ctas = std::min(ntiles, m->sms);
-    k_mlp_backward<<<bwd_ctas, 128, BWD_SMEM, m->stream>>>(a, ntiles);
-    const float b1 = 0.9f, b2 = 0.99f;
-    k_mlp_gsum<<<dim3((NWEIGHT + 255) / 256, GSLICES), 256, 0, m->stream>>>(m->part, bwd_ctas, m->slices);
-    k_mlp_gcheck<<<(NWEIGHT + 255) / 256, 256, 0, m->stream>>>(m->slices, m->nonfinite);
-    k_mlp_step<<<1, 32, 0, m->stream>>>(m->state, m->nonfinite, b1, b2);
-    k_mlp_adam<<<(NWEIGHT + 255) / 256, 256, 0, m->stream>>>(m->slices, m->w, m->m1, m->m2, m->grad, m->wbf, m->cfg.lr, b1, b2,
-                                                              1e-8f, m->state, m->nonfinite);
-    return cudaGetLastError();
-}
-}  // namespace
-
 rc_status rc_mlp_train(rc_mlp* m, const float* d_pos4, const float* d_nrm4, const float* d_aux4, const float* d_target, int tstride,
                        const int* d_idx, int n, float* d_loss) {
     if (!m || !d_pos4 || !d_nrm4 || !d_aux4 || !d_target || n < 128 || n % 128 || n > 128 * m->cap_tiles || tstride < m->cfg.n_out)
@@ -814,40 +853,18 @@ rc_status rc_mlp_train(rc_mlp* m, const float* d_pos4, const float* d_nrm4, cons
     a.tstride = tstride;
     a.idx = d_idx;
     a.n = n;
-    a.act = m->act;
     a.dwpart = m->part;
     a.loss = d_loss ? d_loss : m->loss;
     a.loss_scale = 1.f / ((float)n * (float)m->cfg.n_out);
     a.scale = m->state + ST_SCALE;
-    const int ntiles = n / 128;
+    const int ntiles = n / 128, ctas = std::min(ntiles, m->sms);
     m->step++;
-    rc_mlp::StepArgs key;
-    key.P = d_pos4; key.N = d_nrm4; key.aux = d_aux4; key.target = d_target; key.idx = d_idx;
-    key.tstride = tstride; key.n = n; key.loss = d_loss;
-    for (const auto& g : m->graphs)
-        if (g.args == key) return cudaGraphLaunch(g.exec, m->stream) == cudaSuccess ? RC_OK : mfail(m, RC_ERR_CUDA, "graph launch");
-    // the same arguments twice in a row: capture the step (unless the stream is being captured
-    // already or cannot be); otherwise launch it directly
-    const bool repeat = key == m->last;
-    m->last = key;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (!repeat || m->graphs.size() >= 16 || cudaStreamIsCapturing(m->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
-        cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-        cudaGetLastError();
-        return issue_train(m, a, ntiles, !d_loss) == cudaSuccess ? RC_OK : mfail(m, RC_ERR_CUDA, "launch");
-    }
-    const cudaError_t le = issue_train(m, a, ntiles, !d_loss);
-    cudaGraph_t graph = nullptr;
-    const cudaError_t ce = cudaStreamEndCapture(m->stream, &graph);
-    cudaGraphExec_t exec = nullptr;
-    const bool ok = le == cudaSuccess && ce == cudaSuccess && graph && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
-    if (graph) cudaGraphDestroy(graph);
-    if (!ok) {   // the step did not run: launch it directly
-        cudaGetLastError();
-        return issue_train(m, a, ntiles, !d_loss) == cudaSuccess ? RC_OK : mfail(m, RC_ERR_CUDA, "launch");
-    }
-    m->graphs.push_back({key, exec});
-    return cudaGraphLaunch(exec, m->stream) == cudaSuccess ? RC_OK : mfail(m, RC_ERR_CUDA, "graph launch");
+    const float b1 = 0.9f, b2 = 0.99f;
+    if (!d_loss && cudaMemsetAsync(m->loss, 0, 4, m->stream) != cudaSuccess) return mfail(m, RC_ERR_CUDA, "clear");
+    k_mlp_train<<<ctas, TR_THREADS, TRAIN_SMEM, m->stream>>>(a, ntiles);
+    k_mlp_gsum<<<NWEIGHT / GWEIGHTS, GSLICES * GWEIGHTS / 4, 0, m->stream>>>(m->part, ctas, m->gsum, m->words);
+    k_mlp_adam<<<NWEIGHT / 128, 128, 0, m->stream>>>(m->gsum, m->w, m->m1, m->m2, m->grad, m->wbf, m->cfg.lr, b1, b2, 1e-8f, m->state, m->words);
+    return cudaGetLastError() == cudaSuccess ? RC_OK : mfail(m, RC_ERR_CUDA, "launch");
 }
 
 rc_status rc_mlp_infer(rc_mlp* m, const float* d_pos4, const float* d_nrm4, const float* d_aux4, int n, float* d_out, int ostride) {
@@ -860,8 +877,7 @@ rc_status rc_mlp_infer(rc_mlp* m, const float* d_pos4, const float* d_nrm4, cons
     a.out = d_out;
     a.ostride = ostride;
     const int ntiles = (n + 127) / 128;
-    k_mlp_forward<false, INFER_GROUPS><<<std::min((ntiles + INFER_GROUPS - 1) / INFER_GROUPS, m->sms), FWD_THREADS * INFER_GROUPS,
-                                         FWD_SMEM_INFER, m->stream>>>(a);
+    k_mlp_infer<<<std::min((ntiles + INFER_GROUPS - 1) / INFER_GROUPS, m->sms), FWD_THREADS * INFER_GROUPS, INFER_SMEM, m->stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? RC_OK : mfail(m, RC_ERR_CUDA, "launch");
 }
 

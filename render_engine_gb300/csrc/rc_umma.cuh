@@ -7,6 +7,10 @@
 // apart, along the rows SBO bytes apart.  Element (r, k) lives at
 //     (r / 8) * SBO + (k / 8) * LBO + (r % 8) * 16 + (k % 8) * 2.
 // Here LBO = 128 (a K-row of core matrices is contiguous) and SBO = 128 * K / 8.
+//
+// The same bytes are an operand with the other index as K (MN-major): a core matrix holds 8 values
+// of the tile's rows, now K, by 16 bytes of its columns, now M or N.  Core matrices adjacent along
+// M or N are then SBO apart and those adjacent along K LBO apart: SBO = 128, LBO = 128 * K / 8.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -33,10 +37,11 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
     return d;
 }
 
-// Instruction descriptor of kind::f16: bf16 A and B (both K-major), FP32 accumulator,
-// M x N tile.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// Instruction descriptor of kind::f16: bf16 A and B (K-major, or MN-major where a_mn / b_mn),
+// FP32 accumulator, M x N tile.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool a_mn = false, bool b_mn = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) |
+           ((uint32_t)(M >> 4) << 24);
 }
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

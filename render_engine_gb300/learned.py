@@ -75,8 +75,7 @@ class LearnedCache:
         self.gen = torch.Generator(device=dev)
         self.gen.manual_seed(seed)
         self.dev = dev
-        # one index buffer refilled every step: the training step's arguments stay the same, so
-        # the library replays its captured graph of the step
+        # one index buffer refilled every step
         self.idx = torch.empty(batch, dtype=torch.int32, device=dev)
 
     def begin(self, state: int, seed: int):
