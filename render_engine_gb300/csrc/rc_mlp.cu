@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstdint>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/rc_mlp.h"
@@ -135,9 +136,11 @@ __device__ __forceinline__ void st_bf16(uint8_t* base, uint32_t off, float v) {
 // albedo and a constant.  Produced eight at a time (one 16-byte group of the K-major tile);
 // emit(group, f) stores them.  Two threads share a point: half 0 produces groups 0..8 (the
 // position octaves), half 1 groups 9..21 (about the same work).
+struct EncIn { float4 P, N, X; };   // position, normal, (albedo, direct light)
+__device__ __forceinline__ EncIn encode_load(const MlpArgs& a, int pt) { return {a.P[pt], a.N[pt], a.aux[pt]}; }
 template <class Emit>
-__device__ __forceinline__ void encode(const MlpArgs& a, int pt, int half, Emit&& emit) {
-    const float4 P = a.P[pt], Nn = a.N[pt];
+__device__ __forceinline__ void encode(const MlpArgs& a, const EncIn& in, int half, Emit&& emit) {
+    const float4 P = in.P, Nn = in.N, X = in.X;
     const float p[3] = {fminf(fmaxf((P.x - a.lo[0]) * a.inv_ext[0], 0.f), 1.f), fminf(fmaxf((P.y - a.lo[1]) * a.inv_ext[1], 0.f), 1.f),
                         fminf(fmaxf((P.z - a.lo[2]) * a.inv_ext[2], 0.f), 1.f)};
     const float nv[3] = {Nn.x, Nn.y, Nn.z};
@@ -167,7 +170,6 @@ __device__ __forceinline__ void encode(const MlpArgs& a, int pt, int half, Emit&
         }
         return;
     }
-    const float4 X = a.aux[pt];
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {   // 72 + 8 ax: sin / cos of 2^o pi n
         octaves(3.14159265f * nv[ax]);
@@ -202,15 +204,27 @@ __device__ __forceinline__ void encode(const MlpArgs& a, int pt, int half, Emit&
     emit(21, f);
 }
 
-// Inference over tiles of 128 queries.  A CTA holds the bf16 weights once and runs GROUPS
-// tiles at a time, each on its own group of two warpgroups (thread t of a group works on query
-// row t % 128; the two threads of a row split the input features and the columns of each
-// accumulator, warp w reading the tensor-memory lanes of its quarter w % 4), with its own
-// activation tile, mbarrier, named barrier and 64 tensor-memory columns; the groups overlap
-// one tile's products with another's encoding and epilogues.
-constexpr int FWD_THREADS = 256;                               // threads of one group
-constexpr int INFER_GROUPS = 4;                                // tiles in flight per CTA
-constexpr size_t GROUP_SMEM = (size_t)128 * K0 * 2;            // activation tile
+// Inference over tiles of 128 queries, one persistent CTA per SM over the tiles blockIdx.x,
+// blockIdx.x + gridDim.x, ...: tile k of the CTA is encoded by encoder group k % 2 (256 threads, two
+// per query) into that group's X0 buffer and taken through the layers by chain k % 4 (128 threads,
+// one per query) with its own activation buffer and 64 tensor-memory columns.  A chain gives the X0
+// buffer back as soon as the first layer's product has read it, so two of them keep four chains
+// busy, and encoding, products and epilogues of up to six tiles run at once.
+//
+// Bound by instruction issue and the chains' latency together.  1,082,802 queries: 92 us; as four
+// groups of 256 threads that each encoded a tile and then took it through the layers, 141 us.  One
+// tile alone: 8.7 us.
+constexpr int IN_CHAINS = 4, IN_ENCODERS = 2;
+constexpr int IN_CHAIN_T = 128, IN_ENC_T = 256;
+constexpr int IN_THREADS = IN_CHAINS * IN_CHAIN_T + IN_ENCODERS * IN_ENC_T;
+constexpr int IS_X = WF_BYTES;                              // X0 buffers, 128 x 176
+constexpr int IS_H = IS_X + IN_ENCODERS * 128 * K0 * 2;     // activation buffers, 128 x 64
+constexpr size_t INFER_SMEM = (size_t)IS_H + IN_CHAINS * 128 * HID * 2;
+static_assert(INFER_SMEM > 114 * 1024 && INFER_SMEM <= 226 * 1024, "one inference CTA per SM");
+// named barriers: X0 full (one per chain), X0 empty (one per buffer), a chain's own
+enum InferBar { IB_FULL = 1, IB_EMPTY = IB_FULL + IN_CHAINS, IB_CHAIN = IB_EMPTY + IN_ENCODERS };
+static_assert(IN_THREADS <= 1024 && IB_CHAIN + IN_CHAINS <= 16, "threads and barriers of an inference CTA");
+
 // 16 accumulator columns -> ReLU -> bf16, as two 16-byte pieces of a K-major tile
 __device__ __forceinline__ void relu_pack(const float (&v)[16], uint4& lo4, uint4& hi4) {
     lo4.x = pack_bf16(fmaxf(v[0], 0.f), fmaxf(v[1], 0.f));
@@ -225,91 +239,120 @@ __device__ __forceinline__ void relu_pack(const float (&v)[16], uint4& lo4, uint
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
     return make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
 }
-__global__ void __launch_bounds__(FWD_THREADS * INFER_GROUPS) k_mlp_infer(const MlpArgs a) {
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+__global__ void __launch_bounds__(IN_THREADS) k_mlp_infer(const MlpArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t mbar[INFER_GROUPS];
+    __shared__ uint64_t mbar[IN_CHAINS];
     __shared__ uint32_t tmem_base;
-    __shared__ int gflag[INFER_GROUPS];
-    constexpr uint32_t TCOLS = 64u * INFER_GROUPS;
-    uint8_t* sw = smem;                               // weight tiles, WF_BYTES
-    const int grp = threadIdx.x / FWD_THREADS, tid = threadIdx.x % FWD_THREADS;
-    // this group's activation tile: X0 (128 x 176) and then each H_l (128 x 64) in its place,
-    // H_{l+1} written once the product that reads H_l has completed
-    uint8_t* sx = smem + WF_BYTES + (size_t)grp * GROUP_SMEM;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int row = tid & 127, half = tid >> 7, quarter = warp & 3;
-    for (int i = threadIdx.x; i < WF_BYTES / 16; i += FWD_THREADS * INFER_GROUPS)
-        reinterpret_cast<uint4*>(sw)[i] = reinterpret_cast<const uint4*>(a.wbf)[i];
-    if (threadIdx.x < INFER_GROUPS) mbar_init(&mbar[threadIdx.x], 1);
-    if (threadIdx.x < 32) tmem_alloc(&tmem_base, TCOLS);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int i = tid; i < WF_BYTES / 16; i += IN_THREADS) reinterpret_cast<uint4*>(smem)[i] = reinterpret_cast<const uint4*>(a.wbf)[i];
+    if (tid < IN_CHAINS) mbar_init(&mbar[tid], 1);
+    if (warp == 0) tmem_alloc(&tmem_base, 64u * IN_CHAINS);
     fence_proxy_async();
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    const uint32_t tmem = tmem_base + 64u * (uint32_t)grp;
-    // the group's barrier (named barrier 1 + group; barrier 0 is the whole CTA's)
-    auto gsync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(FWD_THREADS) : "memory"); };
-    uint32_t phase = 0;
-    bool ok = true;
     const int ntiles = (a.n + 127) / 128;
-    for (int tile = blockIdx.x * INFER_GROUPS + grp; tile < ntiles && ok; tile += gridDim.x * INFER_GROUPS) {
-        const int s = tile * 128 + row;
-        const bool live = s < a.n;
-        const int pt = live ? (a.idx ? a.idx[s] : s) : 0;
-        encode(a, pt, half, [&](int k8, const float (&f)[8]) {
-            *reinterpret_cast<uint4*>(sx + kmajor_offset(row, 8 * k8, K0)) = pack8(f);
-        });
-        fence_proxy_async();
-        gsync();
-        for (int l = 0; l < NLAYER && ok; ++l) {
-            const int K = in_dim(l), N = out_dim(l);
-            if (tid == 0) {
-                const uint32_t a0 = smem_u32(sx), b0 = smem_u32(sw + wf_off(l));
-                for (int kk = 0; kk < K / 16; ++kk)
-                    mma_bf16(tmem, smem_desc(a0 + 256u * kk, 128u, 16u * K), smem_desc(b0 + 256u * kk, 128u, 16u * K),
-                             idesc_bf16_f32(128, N), kk > 0);
-                mma_commit(&mbar[grp]);
-            }
-            // one warp watches the barrier; the others wait at the group barrier without issuing
-            // (the fence orders the products before the barrier for every thread of the group)
-            if (warp == 0) {
-                ok = mbar_wait(&mbar[grp], phase, WAIT_LIMIT);
+    const int count = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // tiles of this CTA
+    auto first_row = [&](int k) { return ((int)blockIdx.x + k * (int)gridDim.x) * 128; };
+    if (warp >= IN_CHAINS * IN_CHAIN_T / 32) {
+        const int g = (tid - IN_CHAINS * IN_CHAIN_T) / IN_ENC_T, et = tid % IN_ENC_T, row = et & 127, half = et >> 7;
+        uint8_t* sx = smem + IS_X + g * (128 * K0 * 2);
+        auto inputs = [&](int k) {
+            const int s = first_row(k) + row, q = s < a.n ? s : 0;
+            return encode_load(a, a.idx ? a.idx[q] : q);
+        };
+        EncIn next = inputs(g < count ? g : 0);
+        for (int k = g; k < count; k += IN_ENCODERS) {
+            const EncIn in = next;
+            if (k + IN_ENCODERS < count) next = inputs(k + IN_ENCODERS);
+            if (k >= IN_ENCODERS) bar_sync(IB_EMPTY + g, IN_CHAIN_T + IN_ENC_T);
+            encode(a, in, half, [&](int k8, const float (&f)[8]) {
+                *reinterpret_cast<uint4*>(sx + kmajor_offset(row, 8 * k8, K0)) = pack8(f);
+            });
+            fence_proxy_async();
+            bar_arrive(IB_FULL + k % IN_CHAINS, IN_CHAIN_T + IN_ENC_T);
+        }
+    } else {
+        const int c = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+        const uint32_t sm0 = smem_u32(smem), tmem = tmem_base + 64u * (uint32_t)c, acc = tmem + ((uint32_t)(quarter * 32) << 16);
+        uint8_t* sh = smem + IS_H + c * (128 * HID * 2);
+        uint32_t phase = 0;
+        bool ok = true;
+        // One warp of the chain watches the barrier, the others wait for it without issuing (all warps
+        // polling took 229 us where this took 141).  A wait that gives up is the last one: the chain
+        // goes on through its barriers, so that nobody waits for it, and stores no more outputs.
+        auto wait = [&]() {
+            if (quarter == 0) {
+                if (ok && !mbar_wait(&mbar[c], phase, WAIT_LIMIT)) {
+                    ok = false;
+                    if (lane == 0) atomicOr(a.err, 1u);
+                }
                 fence_before_sync();
-                if (lane == 0) gflag[grp] = ok ? 1 : 0;
             }
             phase ^= 1u;
-            gsync();
-            ok = gflag[grp] != 0;   // the whole group leaves together
-            if (!ok) {
-                if (tid == 0) atomicOr(a.err, 1u);
-                break;
-            }
+            bar_sync(IB_CHAIN + c, IN_CHAIN_T);
             fence_after_sync();
-            // columns of this thread: one half of a hidden layer; all 16 outputs for half 0
-            const int c0 = l < NLAYER - 1 ? half * (N / 2) : 0;
-            const int c1 = l < NLAYER - 1 ? c0 + N / 2 : (half == 0 ? N : 0);
-            for (int c = c0; c < c1; c += 16) {
-                float v[16];
-                tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c, v);
-                tmem_wait_ld();
-                if (l < NLAYER - 1) {
-                    uint4 lo4, hi4;
-                    relu_pack(v, lo4, hi4);
-                    *reinterpret_cast<uint4*>(sx + kmajor_offset(row, c, HID)) = lo4;
-                    *reinterpret_cast<uint4*>(sx + kmajor_offset(row, c + 8, HID)) = hi4;
-                } else if (live) {
-                    for (int j = 0; j < a.n_out; ++j) a.out[(size_t)s * a.ostride + j] = v[j];
+        };
+        auto issue = [&](uint32_t a0, uint32_t b0, auto kc, uint32_t idesc) {
+            constexpr int K = decltype(kc)::value;
+            if (quarter == 0 && lane == 0 && ok) {
+#pragma unroll
+                for (int kk = 0; kk < K / 16; ++kk)
+                    mma_bf16(tmem, smem_desc(a0 + 256u * kk, 128u, 16u * K), smem_desc(b0 + 256u * kk, 128u, 16u * K), idesc, kk > 0);
+                mma_commit(&mbar[c]);
+            }
+            __syncwarp();
+        };
+        for (int k = c; k < count; k += IN_CHAINS) {
+            const int b = k % IN_ENCODERS, s = first_row(k) + row;
+            bar_sync(IB_FULL + c, IN_CHAIN_T + IN_ENC_T);
+            issue(sm0 + IS_X + b * (128 * K0 * 2), sm0, std::integral_constant<int, K0>{}, idesc_bf16_f32(128, HID));
+            wait();
+            if (k + IN_ENCODERS < count) bar_arrive(IB_EMPTY + b, IN_CHAIN_T + IN_ENC_T);
+#pragma unroll 1
+            for (int l = 1; l < NLAYER; ++l) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    float v[2][16];
+                    tmem_ld16(acc + 32u * q, v[0]);
+                    tmem_ld16(acc + 32u * q + 16u, v[1]);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint4 lo4, hi4;
+                        relu_pack(v[h], lo4, hi4);
+                        uint8_t* dst = sh + kmajor_offset(row, 32 * q + 16 * h, HID);
+                        *reinterpret_cast<uint4*>(dst) = lo4;
+                        *reinterpret_cast<uint4*>(dst + 128) = hi4;
+                    }
                 }
+                fence_before_sync();
+                fence_proxy_async();
+                bar_sync(IB_CHAIN + c, IN_CHAIN_T);
+                fence_after_sync();
+                issue(smem_u32(sh), sm0 + wf_off(l), std::integral_constant<int, HID>{}, idesc_bf16_f32(128, out_dim(l)));
+                wait();
+            }
+            float v[16];
+            tmem_ld16(acc, v);
+            tmem_wait_ld();
+            if (s < a.n && ok) {
+                float* o = a.out + (size_t)s * a.ostride;
+#pragma unroll
+                for (int j = 0; j < OUTP; ++j)
+                    if (j < a.n_out) o[j] = v[j];
             }
             fence_before_sync();
-            fence_proxy_async();
-            gsync();
+            bar_sync(IB_CHAIN + c, IN_CHAIN_T);   // the accumulator has been read
             fence_after_sync();
         }
+        fence_before_sync();
     }
-    fence_before_sync();
     __syncthreads();
-    if (threadIdx.x < 32) tmem_dealloc(tmem_base, TCOLS);
+    if (warp == 0) tmem_dealloc(tmem_base, 64u * IN_CHAINS);
 }
 
 // 16-byte asynchronous copies global -> shared (no register staging)
@@ -377,9 +420,6 @@ static_assert(TRAIN_SMEM > 114 * 1024 && TRAIN_SMEM <= 226 * 1024, "one training
 // named barriers: an operand handed over by the chain; an X0 buffer full, empty (one of each per buffer)
 enum TrainBar { TB_CHAIN = 1, TB_FULL = 2, TB_EMPTY = 4 };
 
-__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-
 __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int ntiles) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar;
@@ -434,12 +474,17 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int n
         }
     } else if (warp >= W_ENCODE) {
         const int et = tid - TR_CHAIN, row = et & 127, half = et >> 7;
-        for (int it = 0; it < count; ++it) {
+        auto inputs = [&](int it) {
             const int s = ((int)blockIdx.x + it * (int)gridDim.x) * 128 + row;
-            const int pt = a.idx ? a.idx[s] : s;
+            return encode_load(a, a.idx ? a.idx[s] : s);
+        };
+        EncIn next = inputs(0);
+        for (int it = 0; it < count; ++it) {
+            const EncIn in = next;
             uint8_t* sx = smem + xbuf(it);
+            if (it + 1 < count) next = inputs(it + 1);
             if (it >= 2) bar_sync(TB_EMPTY + (it & 1), TR_CHAIN + TR_ENCODE);
-            encode(a, pt, half, [&](int k8, const float (&f)[8]) {
+            encode(a, in, half, [&](int k8, const float (&f)[8]) {
                 *reinterpret_cast<uint4*>(sx + kmajor_offset(row, 8 * k8, K0)) = pack8(f);
             });
             fence_proxy_async();
@@ -689,7 +734,6 @@ __global__ void __launch_bounds__(128) k_mlp_adam(const float* __restrict__ gsum
     *reinterpret_cast<float4*>(st) = n;
 }
 
-constexpr size_t INFER_SMEM = (size_t)WF_BYTES + INFER_GROUPS * GROUP_SMEM;   // 224 KB: one CTA per SM
 }  // namespace
 
 extern "C" rc_status rc_mlp_tile_product(const uint16_t* d_a, const uint16_t* d_b, float* d_d, int K, int N, unsigned* d_err,
@@ -877,7 +921,7 @@ rc_status rc_mlp_infer(rc_mlp* m, const float* d_pos4, const float* d_nrm4, cons
     a.out = d_out;
     a.ostride = ostride;
     const int ntiles = (n + 127) / 128;
-    k_mlp_infer<<<std::min((ntiles + INFER_GROUPS - 1) / INFER_GROUPS, m->sms), FWD_THREADS * INFER_GROUPS, INFER_SMEM, m->stream>>>(a);
+    k_mlp_infer<<<std::min(ntiles, m->sms), IN_THREADS, INFER_SMEM, m->stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? RC_OK : mfail(m, RC_ERR_CUDA, "launch");
 }
 

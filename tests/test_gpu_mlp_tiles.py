@@ -1,4 +1,4 @@
-"""The training step's persistent tiles: the gradient of n samples equals the sum of the gradients of
+"""The training step's and the inference's persistent tiles.  Training: the gradient of n samples equals the sum of the gradients of
 its parts, whatever the number of 128-sample tiles per CTA (none to four, whole and partial rounds)
 and of outputs.  With the learning rate at zero the weights stay put; the loss gradient is scaled by
 1 / (n n_out), so a part of n / k samples weighs 1 / k.  Both sides are FP32 sums of the same bf16
@@ -39,4 +39,27 @@ def test_gradient_is_the_sum_of_its_halves(tiles, n_out):
     # bf16 rounding of the scaled gradients is the same for both (a power of two apart), so what is left
     # is FP32 summation: n terms, errors growing as their square root
     assert np.abs(whole - halves).max() <= 64 * 2.0 ** -24 * np.sqrt(n) * max(scale, np.abs(whole).max())
+    net.close()
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 128 * 152, 128 * 153 + 1, 128 * 305, 128 * 608 - 5, 128 * 611 + 77, 128 * 1000])
+@pytest.mark.parametrize("n_out", [1, 3, 16])
+def test_outputs_do_not_depend_on_the_batch(n, n_out):
+    """A query's outputs are its own: the same bits in a batch of one tile and in one of many
+    tiles per CTA, and nothing beyond the batch or its outputs is written."""
+    P, N, aux = _inputs(n, n)
+    net = mlp.Mlp(n_out=n_out, seed=4)
+    whole = torch.full((n + 1, n_out + 1), -7.0, device="cuda")
+    torch.cuda.synchronize()
+    net.infer_raw(P, N, aux, n, whole.data_ptr(), n_out + 1)
+    assert net.error_flags() == 0
+    assert (whole[n] == -7).all() and (whole[:, n_out] == -7).all()
+    for at in sorted({0, max(0, n - 128), 128 * (n // 256)}):
+        m = min(128, n - at)
+        part = torch.zeros(m, n_out, device="cuda")
+        p, q, x = P[at:at + m].contiguous(), N[at:at + m].contiguous(), aux[at:at + m].contiguous()
+        torch.cuda.synchronize()
+        net.infer(p, q, x, part)
+        assert net.error_flags() == 0
+        assert torch.equal(part, whole[at:at + m, :n_out])
     net.close()
