@@ -28,6 +28,8 @@ namespace adj {
 namespace {
 
 constexpr int B = 256;
+constexpr long long FOLLOW_RAYS = 1 << 21;          // rays from which the sweeps' counts are followed (a sweep of 10 us)
+constexpr int FEW_BELOW = 10;
 constexpr int SCAN_ITEMS = 8;                       // per thread
 constexpr int SCAN_TILE = B * SCAN_ITEMS;           // 2048 per block
 
@@ -96,23 +98,19 @@ __global__ void k_fill(const int* __restrict__ hits, long long n, const int* __r
 }
 
 // the segment of every entry sorted by ray index (rank = entries of the segment with a smaller
-// ray index; ray indices are unique), stored as the ray's source point
-__global__ void k_rank(const int* __restrict__ off, int Np, const int* __restrict__ unordered, int K, long long cap,
+// ray index; ray indices are unique), stored as the ray's source point.  The entry's segment is
+// its ray's hit point.  17.3 M rays: 462 us with a search of the offsets and an atomic maximum per
+// segment on one address, 221 us
+__global__ void k_rank(const int* __restrict__ hits, const int* __restrict__ off, int Np, const int* __restrict__ unordered, int K, long long cap,
                        int* __restrict__ src, int* maxseg) {
     const long long total = off[Np];
     for (long long q = blockIdx.x * (long long)B + threadIdx.x; q < total && q < cap; q += (long long)gridDim.x * B) {
-        int lo = 0, hi = Np;   // largest j with off[j] <= q
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (off[mid] <= q) lo = mid;
-            else hi = mid;
-        }
-        const int a = off[lo], b = off[lo + 1];
-        const int e = unordered[q];
+        const int e = unordered[q], j = hits[e];
+        const int a = off[j], b = off[j + 1];
         int rank = 0;
         for (int t = a; t < b; ++t) rank += unordered[t] < e;
         src[a + rank] = e / K;
-        if (q == a) atomicMax(maxseg, b - a);
+        if (q == a && b - a > *(volatile int*)maxseg) atomicMax(maxseg, b - a);   // (one address: few need the atomic)
     }
 }
 
@@ -135,40 +133,76 @@ __global__ void k_prep(const float* __restrict__ AE, const float* __restrict__ A
     g0[j] = ae[0] * (d + 0.f);
 }
 
-// forward sweep: L_i = (1/K) sum over i's counted rays, in ray order, of g_j = A_j (d_j + L_j)
-// from the previous sweep; writes L and the next sweep's g.  Hit lists are read four rays at a
-// time when K is a multiple of 4 (rows of 16 K bytes stay 16-byte aligned).
+// The value of point i from the previous sweep's gathered values, its counted rays in ray order.
+// Hit lists are read four rays at a time when K is a multiple of 4 (rows of 16 K bytes stay 16-byte
+// aligned).
+__device__ __forceinline__ float fwd_value(const int* __restrict__ hits, int K, int i, const float* __restrict__ gin) {
+    float sum = 0.f;
+    const int* h = hits + (size_t)i * K;
+    if ((K & 3) == 0) {
+        const int4* h4 = reinterpret_cast<const int4*>(h);
+        for (int r = 0; r < K / 4; ++r) {
+            const int4 q = __ldg(h4 + r);
+            const float a = q.x >= 0 ? __ldcg(gin + q.x) : 0.f, b = q.y >= 0 ? __ldcg(gin + q.y) : 0.f;
+            const float c = q.z >= 0 ? __ldcg(gin + q.z) : 0.f, d = q.w >= 0 ? __ldcg(gin + q.w) : 0.f;
+            if (q.x >= 0) sum += a;
+            if (q.y >= 0) sum += b;
+            if (q.z >= 0) sum += c;
+            if (q.w >= 0) sum += d;
+        }
+    } else {
+        for (int r = 0; r < K; ++r) {
+            const int j = __ldg(h + r);
+            if (j >= 0) sum += __ldcg(gin + j);
+        }
+    }
+    return sum / (float)K;
+}
+// w_j + (A_j / K) sum over the rays reaching j, in ray order, of uin[source] (four sources fetched at
+// a time)
+__device__ __forceinline__ float bwd_value(const int* __restrict__ src, int a, int b, int K, float A, float w, const float* __restrict__ uin) {
+    float sum = 0.f;
+    int q = a;
+    for (; q + 4 <= b; q += 4) {
+        const int s0 = __ldg(src + q), s1 = __ldg(src + q + 1), s2 = __ldg(src + q + 2), s3 = __ldg(src + q + 3);
+        const float x0 = __ldcg(uin + s0), x1 = __ldcg(uin + s1), x2 = __ldcg(uin + s2), x3 = __ldcg(uin + s3);
+        sum += x0;
+        sum += x1;
+        sum += x2;
+        sum += x3;
+    }
+    for (; q < b; ++q) sum += __ldcg(uin + __ldg(src + q));
+    return w + A * sum / (float)K;
+}
+__device__ __forceinline__ bool differ(float a, float b) { return __float_as_uint(a) != __float_as_uint(b); }
+
+// The sweeps write, besides the iterate, one bit per point, set when the value that the next sweep
+// gathers is not the one this sweep gathered (a warp's 32 points are a word), and add up the bits.
+// bits is null where nobody asks.
+__device__ __forceinline__ void note_bits(bool changed, int i, int Np, uint32_t* __restrict__ bits, unsigned* __restrict__ count) {
+    const unsigned m = __ballot_sync(0xffffffffu, changed);
+    if ((threadIdx.x & 31) == 0 && i < Np) bits[i >> 5] = m;
+    const int n = __syncthreads_count(changed);
+    if (threadIdx.x == 0 && n) atomicAdd(count, (unsigned)n);
+}
+
+// forward sweep: L_i from the previous sweep's g; writes L and the next sweep's g = A (d + L)
 __global__ void __launch_bounds__(B) k_fwd(const int* __restrict__ hits, int K, int Np, const float2* __restrict__ da,
                                            const float* __restrict__ gin, const float* __restrict__ Lprev, float* __restrict__ Lout,
-                                           float* __restrict__ gout, unsigned* chg) {
+                                           float* __restrict__ gout, uint32_t* __restrict__ bits, unsigned* __restrict__ count, unsigned* chg) {
     const int i = blockIdx.x * B + threadIdx.x;
     float v = 0.f, dv = 0.f;
+    bool changed = false;
     if (i < Np) {
-        float sum = 0.f;
-        const int* h = hits + (size_t)i * K;
-        if ((K & 3) == 0) {
-            const int4* h4 = reinterpret_cast<const int4*>(h);
-            for (int r = 0; r < K / 4; ++r) {
-                const int4 q = __ldg(h4 + r);
-                const float a = q.x >= 0 ? __ldcg(gin + q.x) : 0.f, b = q.y >= 0 ? __ldcg(gin + q.y) : 0.f;
-                const float c = q.z >= 0 ? __ldcg(gin + q.z) : 0.f, d = q.w >= 0 ? __ldcg(gin + q.w) : 0.f;
-                if (q.x >= 0) sum += a;
-                if (q.y >= 0) sum += b;
-                if (q.z >= 0) sum += c;
-                if (q.w >= 0) sum += d;
-            }
-        } else {
-            for (int r = 0; r < K; ++r) {
-                const int j = __ldg(h + r);
-                if (j >= 0) sum += __ldcg(gin + j);
-            }
-        }
-        v = sum / (float)K;
+        v = fwd_value(hits, K, i, gin);
         Lout[i] = v;
         const float2 x = da[i];
-        gout[i] = x.y * (x.x + v);
+        const float g = x.y * (x.x + v);
+        gout[i] = g;
+        if (bits) changed = differ(g, gin[i]);
         dv = fabsf(v - Lprev[i]);
     }
+    if (bits) note_bits(changed, i, Np, bits, count);
     if (chg) {   // change of the sweep, and the largest value (non-negative floats order as their bits)
         const unsigned a = warp_max(__float_as_uint(dv)), b = warp_max(__float_as_uint(fabsf(v)));
         if ((threadIdx.x & 31) == 0) {
@@ -178,30 +212,21 @@ __global__ void __launch_bounds__(B) k_fwd(const int* __restrict__ hits, int K, 
     }
 }
 
-// adjoint sweep: uout[j] = w_j + (A_j / K) sum over the rays reaching j, in ray order, of
-// uin[source] (four sources fetched at a time)
+// adjoint sweep
 __global__ void __launch_bounds__(B) k_bwd(const int* __restrict__ off, const int* __restrict__ src, int K, int Np,
-                                           const float2* __restrict__ da, const float* __restrict__ w,
-                                           const float* __restrict__ uin, float* __restrict__ uout, unsigned* chg) {
+                                           const float2* __restrict__ da, const float* __restrict__ w, const float* __restrict__ uin,
+                                           float* __restrict__ uout, uint32_t* __restrict__ bits, unsigned* __restrict__ count, unsigned* chg) {
     const int j = blockIdx.x * B + threadIdx.x;
     float v = 0.f, dv = 0.f;
+    bool changed = false;
     if (j < Np) {
-        float sum = 0.f;
-        const int a = off[j], b = off[j + 1];
-        int q = a;
-        for (; q + 4 <= b; q += 4) {
-            const int s0 = __ldg(src + q), s1 = __ldg(src + q + 1), s2 = __ldg(src + q + 2), s3 = __ldg(src + q + 3);
-            const float x0 = __ldcg(uin + s0), x1 = __ldcg(uin + s1), x2 = __ldcg(uin + s2), x3 = __ldcg(uin + s3);
-            sum += x0;
-            sum += x1;
-            sum += x2;
-            sum += x3;
-        }
-        for (; q < b; ++q) sum += __ldcg(uin + __ldg(src + q));
-        v = w[j] + da[j].y * sum / (float)K;
+        v = bwd_value(src, off[j], off[j + 1], K, da[j].y, w[j], uin);
         uout[j] = v;
-        dv = fabsf(v - uin[j]);
+        const float u = uin[j];
+        changed = differ(v, u);
+        dv = fabsf(v - u);
     }
+    if (bits) note_bits(changed, j, Np, bits, count);
     if (chg) {
         const unsigned a = warp_max(__float_as_uint(dv)), b = warp_max(__float_as_uint(fabsf(v)));
         if ((threadIdx.x & 31) == 0) {
@@ -211,24 +236,108 @@ __global__ void __launch_bounds__(B) k_bwd(const int* __restrict__ off, const in
     }
 }
 
-// Column c < NL: sum_j (u_j - w_j) G_c[j]; column NL: sum_j w_j L_j.  Block x of column c sums
-// a fixed slice of points (thread-strided, then a fixed tree), so the order never changes.
+// The same sweeps once few values still change.  A point none of whose gathered values changed in the
+// last sweep keeps its value to the last bit.  k_touch marks the points that do gather a changed value
+// (of a changed g_j the sources of the rays reaching j, of a changed u_i the points that its rays
+// reach), at a cost that falls with the changes; the sweep recomputes those, copies the others, and
+// leaves the marks cleared.  1.08 M points, K = 16: 9 to 30 us behind 3 to 17 us of marks, where a full
+// sweep takes 67 (forward) or 70 us (adjoint): those are bound by the L1, which takes one random
+// sector per clock and SM.  A lookup of the gathered values' bits in shared memory instead of the marks
+// cost 43 and 64 us.
+__global__ void __launch_bounds__(B) k_touch(const uint32_t* __restrict__ bits, int words, const int* __restrict__ off, const int* __restrict__ list,
+                                             int K, uint32_t* __restrict__ marks) {
+    // four lanes to a word of 32 points; point j's list is [off[j], off[j + 1]), or [j K, j K + K) without off
+    const int t = blockIdx.x * B + threadIdx.x, wd = t >> 2;
+    if (wd >= words) return;
+    for (uint32_t m = bits[wd]; m; m &= m - 1u) {
+        const int j = 32 * wd + __ffs((int)m) - 1;
+        const int a = off ? off[j] : j * K, b = off ? off[j + 1] : a + K;
+        for (int q = a + (t & 3); q < b; q += 4) {
+            const int i = __ldg(list + q);
+            if (i >= 0) atomicOr(marks + (i >> 5), 1u << (i & 31));
+        }
+    }
+}
+__global__ void __launch_bounds__(B) k_fwd_few(const int* __restrict__ hits, int K, int Np, const float2* __restrict__ da,
+                                               const float* __restrict__ gin, const float* __restrict__ Lprev, float* __restrict__ Lout,
+                                               float* __restrict__ gout, uint32_t* __restrict__ marks, uint32_t* __restrict__ bits,
+                                               unsigned* __restrict__ count) {
+    const int i = blockIdx.x * B + threadIdx.x;
+    const uint32_t word = i < Np ? marks[i >> 5] : 0u;
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0 && word) marks[i >> 5] = 0u;
+    bool changed = false;
+    if (i < Np) {
+        const float g0 = gin[i];
+        float v = Lprev[i], g = g0;
+        if (word >> (i & 31) & 1u) {
+            v = fwd_value(hits, K, i, gin);
+            const float2 x = da[i];
+            g = x.y * (x.x + v);
+            changed = differ(g, g0);
+        }
+        Lout[i] = v;
+        gout[i] = g;
+    }
+    note_bits(changed, i, Np, bits, count);
+}
+__global__ void __launch_bounds__(B) k_bwd_few(const int* __restrict__ off, const int* __restrict__ src, int K, int Np,
+                                               const float2* __restrict__ da, const float* __restrict__ w, const float* __restrict__ uin,
+                                               float* __restrict__ uout, uint32_t* __restrict__ marks, uint32_t* __restrict__ bits,
+                                               unsigned* __restrict__ count) {
+    const int j = blockIdx.x * B + threadIdx.x;
+    const uint32_t word = j < Np ? marks[j >> 5] : 0u;
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0 && word) marks[j >> 5] = 0u;
+    bool changed = false;
+    if (j < Np) {
+        const float u = uin[j];
+        float v = u;
+        if (word >> (j & 31) & 1u) {
+            v = bwd_value(src, off[j], off[j + 1], K, da[j].y, w[j], uin);
+            changed = differ(v, u);
+        }
+        uout[j] = v;
+    }
+    note_bits(changed, j, Np, bits, count);
+}
+
+// Column c < NL: sum_j (u_j - w_j) G_c[j]; column NL: sum_j w_j L_j.  Block x sums a fixed slice of
+// points (thread-strided, then a fixed tree), so the order never changes; it takes COLS columns at
+// once, so that a point's record is read once or twice and not once per column (17 columns of 1.08 M
+// points: 309 -> 134 us).
+constexpr int COLS = 6;
 __global__ void __launch_bounds__(B) k_grad_part(const float* __restrict__ AEu, int aes, int NL, int Np, const float* __restrict__ u,
                                                  const float* __restrict__ w, const float* __restrict__ L, double* __restrict__ part) {
     __shared__ double sh[B];
-    const int c = blockIdx.y;
+    const int c0 = blockIdx.y * COLS;
     const long long per = ((long long)Np + gridDim.x - 1) / gridDim.x;
     const long long j0 = per * blockIdx.x, j1 = min((long long)Np, j0 + per);
-    double s = 0.0;
-    for (long long j = j0 + threadIdx.x; j < j1; j += B)
-        s += c < NL ? ((double)u[j] - (double)w[j]) * (double)AEu[(size_t)aes * j + 1 + c] : (double)w[j] * (double)L[j];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = B / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
+    double s[COLS];
+#pragma unroll
+    for (int k = 0; k < COLS; ++k) s[k] = 0.0;
+    for (long long j = j0 + threadIdx.x; j < j1; j += B) {
+        const float uj = u[j], wj = w[j];
+        const double d = (double)uj - (double)wj;
+        const float* G = AEu + (size_t)aes * j + 1 + c0;
+#pragma unroll
+        for (int k = 0; k < COLS; ++k) {
+            if (c0 + k < NL) s[k] += d * (double)G[k];
+            else if (c0 + k == NL) s[k] += (double)wj * (double)L[j];
+        }
     }
-    if (threadIdx.x == 0) part[(size_t)c * gridDim.x + blockIdx.x] = sh[0];
+#pragma unroll
+    for (int k = 0; k < COLS; ++k) {
+        if (c0 + k > NL) break;
+        __syncthreads();
+        sh[threadIdx.x] = s[k];
+        __syncthreads();
+        for (int o = B / 2; o > 0; o >>= 1) {
+            if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) part[(size_t)(c0 + k) * gridDim.x + blockIdx.x] = sh[0];
+    }
 }
 
 __global__ void __launch_bounds__(B) k_grad_final(const double* __restrict__ part, int G, double* __restrict__ out) {
@@ -261,6 +370,8 @@ cudaError_t scan_exclusive(const int* in, int* out, int n, int* scratch, cudaStr
 
 }  // namespace
 
+size_t bit_words(int Np) { return ((size_t)Np + 31) / 32; }
+
 size_t scan_scratch_ints(long long n) {
     size_t s = 0;
     while (n > 1) {
@@ -279,7 +390,7 @@ cudaError_t build_transpose(const Bufs& b, int Np, int K, cudaStream_t st) {
     k_count<<<stride_blocks(n), B, 0, st>>>(b.hits, n, b.cnt, &b.stats->back);
     if ((e = scan_exclusive(b.cnt, b.off, Np + 1, b.scratch, st)) != cudaSuccess) return e;
     k_fill<<<stride_blocks(n), B, 0, st>>>(b.hits, n, b.off, b.fill, b.unordered);
-    k_rank<<<stride_blocks(n), B, 0, st>>>(b.off, Np, b.unordered, K, n, b.src, &b.stats->max_incoming);
+    k_rank<<<stride_blocks(n), B, 0, st>>>(b.hits, b.off, Np, b.unordered, K, n, b.src, &b.stats->max_incoming);
     return cudaGetLastError();
 }
 
@@ -290,15 +401,54 @@ cudaError_t solve(Bufs* bp, int Np, int K, int NL, int aes, const float* AE, con
     k_prep<<<blocks_for(Np), B, 0, st>>>(AE, AEu, em, aes, NL, Np, b.da, b.g[0]);
     if ((e = cudaMemsetAsync(b.L[0], 0, sizeof(float) * (size_t)Np, st)) != cudaSuccess) return e;
     if ((e = cudaMemcpyAsync(b.u[0], b.w, sizeof(float) * (size_t)Np, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
+    // The sweeps.  On large problems the host follows, two sweeps behind, how many values still change:
+    // below Np / FEW_BELOW of them the sweeps look first what to recompute (with K = 16, 10 % changing
+    // values leave a fifth of the points alone, 1 % leave 85 %), and once none changes in two counted
+    // sweeps, both buffers hold the fixed point and the sweeps up to the last have nothing to change.
+    // The last sweep is always a full one: it measures the change.
+    const bool follow = (long long)Np * K >= FOLLOW_RAYS && iters > 4;
+    const int words = (Np + 31) / 32, touch_blocks = blocks_for(4LL * words);
+    if (follow && ((e = cudaMemsetAsync(b.counts, 0, 2 * sizeof(unsigned) * (size_t)iters, st)) != cudaSuccess ||
+                   (e = cudaMemsetAsync(b.marks, 0, sizeof(uint32_t) * (size_t)words, st)) != cudaSuccess))
+        return e;
+    bool few[2] = {false, false}, still[2] = {false, false};
     for (int t = 0; t < iters; ++t) {
         const bool last = t == iters - 1;
-        k_fwd<<<blocks_for(Np), B, 0, st>>>(b.hits, K, Np, b.da, b.g[t & 1], b.L[t & 1], b.L[(t + 1) & 1], b.g[(t + 1) & 1],
-                                            last ? b.stats->chg : nullptr);
-        k_bwd<<<blocks_for(Np), B, 0, st>>>(b.off, b.src, K, Np, b.da, b.w, b.u[t & 1], b.u[(t + 1) & 1], last ? b.stats->chg : nullptr);
+        if (follow && t >= 4 && (t & 1) == 0 && !last) {
+            // the counts of sweep t - 3 and before have been copied behind sweep t - 3
+            if ((e = cudaEventSynchronize(b.seen[(t >> 1) & 1])) != cudaSuccess) return e;
+            for (int k = 0; k < 2; ++k) {
+                const unsigned n = b.host_counts[2 * (t - 3) + k];
+                few[k] = n < (unsigned)Np / FEW_BELOW;
+                still[k] = n == 0 && b.host_counts[2 * (t - 4) + k] == 0;
+            }
+        }
+        unsigned* chg = last ? b.stats->chg : nullptr;
+        uint32_t *bi0 = follow ? b.bits[0][t & 1] : nullptr, *bi1 = follow ? b.bits[1][t & 1] : nullptr;
+        uint32_t *bo0 = follow ? b.bits[0][(t + 1) & 1] : nullptr, *bo1 = follow ? b.bits[1][(t + 1) & 1] : nullptr;
+        unsigned *c0 = follow ? b.counts + 2 * t : nullptr, *c1 = follow ? c0 + 1 : nullptr;
+        if (last || !few[0]) {
+            k_fwd<<<blocks_for(Np), B, 0, st>>>(b.hits, K, Np, b.da, b.g[t & 1], b.L[t & 1], b.L[(t + 1) & 1], b.g[(t + 1) & 1], bo0, c0, chg);
+        } else if (!still[0]) {
+            k_touch<<<touch_blocks, B, 0, st>>>(bi0, words, b.off, b.src, K, b.marks);
+            k_fwd_few<<<blocks_for(Np), B, 0, st>>>(b.hits, K, Np, b.da, b.g[t & 1], b.L[t & 1], b.L[(t + 1) & 1], b.g[(t + 1) & 1], b.marks, bo0, c0);
+        }
+        if (last || !few[1]) {
+            k_bwd<<<blocks_for(Np), B, 0, st>>>(b.off, b.src, K, Np, b.da, b.w, b.u[t & 1], b.u[(t + 1) & 1], bo1, c1, chg);
+        } else if (!still[1]) {
+            k_touch<<<touch_blocks, B, 0, st>>>(bi1, words, nullptr, b.hits, K, b.marks);
+            k_bwd_few<<<blocks_for(Np), B, 0, st>>>(b.off, b.src, K, Np, b.da, b.w, b.u[t & 1], b.u[(t + 1) & 1], b.marks, bo1, c1);
+        }
+        if (follow && (t & 1) && t + 3 < iters - 1) {   // read before sweep t + 3
+            if ((e = cudaMemcpyAsync(b.host_counts + 2 * (t - 1), b.counts + 2 * (t - 1), 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, st)) !=
+                    cudaSuccess ||
+                (e = cudaEventRecord(b.seen[((t + 3) >> 1) & 1], st)) != cudaSuccess)
+                return e;
+        }
     }
     bp->L_final = b.L[iters & 1];
     bp->u_final = b.u[iters & 1];
-    k_grad_part<<<dim3(GRAD_BLOCKS, NL + 1), B, 0, st>>>(AEu, aes, NL, Np, bp->u_final, b.w, bp->L_final, b.part);
+    k_grad_part<<<dim3(GRAD_BLOCKS, (NL + 1 + COLS - 1) / COLS), B, 0, st>>>(AEu, aes, NL, Np, bp->u_final, b.w, bp->L_final, b.part);
     k_grad_final<<<NL + 1, B, 0, st>>>(b.part, GRAD_BLOCKS, b.stats->out);
     return cudaGetLastError();
 }

@@ -33,11 +33,17 @@ struct Bufs {
     const float* L_final;   // the iterate holding the forward solution (set by solve)
     const float* u_final;   // the iterate holding the adjoint solution (set by solve)
     float* w;         // Np weights
+    uint32_t* bits[2][2];   // forward, adjoint: values that changed in a sweep, bit_words(Np) each, ping-pong
+    uint32_t* marks;        // points to recompute, bit_words(Np)
+    unsigned* counts;       // iterations x (forward, adjoint): how many
+    unsigned* host_counts;  // the same in page-locked memory
+    cudaEvent_t seen[2];    // behind the copies of the counts
     double* part;     // GRAD_BLOCKS * (NL + 1)
     Stats* stats;
 };
 
 size_t scan_scratch_ints(long long n);
+size_t bit_words(int Np);   // words of a bit per point
 // transposed ray lists from b.hits (also clears b.stats)
 cudaError_t build_transpose(const Bufs& b, int Np, int K, cudaStream_t st);
 // `iters` forward and adjoint Jacobi sweeps from L = 0, u = w, then the gradient against the

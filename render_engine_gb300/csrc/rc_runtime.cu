@@ -163,7 +163,9 @@ struct rc_ctx {
     cudaEvent_t load_ev = nullptr;              // the load's copies, which the side stream waits for
     std::vector<cudaEvent_t> copies_ev;         // per state: its copies on the side stream are done (RC_FLAG_LOAD_ASYNC)
     int adj_np = 0, adj_k = 0;                  // sizes of the last rc_adjoint (0: none)
-    int adj_cap_np = 0, adj_cap_k = 0, adj_cap_nl = 0;   // sizes the adjoint buffers were allocated for
+    int adj_cap_np = 0, adj_cap_k = 0, adj_cap_nl = 0, adj_cap_it = 0;   // sizes the adjoint buffers were allocated for
+    unsigned* adj_counts = nullptr;                  // page-locked: values that change, per sweep
+    cudaEvent_t adj_seen[2] = {nullptr, nullptr};    // behind the copies into it
     float4* adj_aeu = nullptr;                  // unit-emission direct light of the last adjoint
     int adj_aeu_state = -1;                     // the state adj_aeu holds (-1: none)
     const float* adj_ones = nullptr;
@@ -1586,6 +1588,9 @@ void rc_destroy(rc_ctx* ctx) {
     if (ctx->cam.ready) cudaEventDestroy(ctx->cam.ready);
     if (ctx->flags_dev) cudaFree(ctx->flags_dev);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    if (ctx->adj_counts) cudaFreeHost(ctx->adj_counts);
+    for (cudaEvent_t e : ctx->adj_seen)
+        if (e) cudaEventDestroy(e);
     if (ctx->stage) cudaFree(ctx->stage);
     if (ctx->img) cudaFree(ctx->img);
     for (auto& e : ctx->ev) if (e) cudaEventDestroy(e);
@@ -2220,13 +2225,28 @@ rc_status rc_adjoint(rc_ctx* ctx, const rc_adjoint_params* prm, const float* wei
     adj::Bufs b = ctx->adj;
     rc_status s;
     // buffers kept from call to call while the point count, K and the light count stay
-    if (ctx->adj_cap_np != S.Np || ctx->adj_cap_k != prm->K || ctx->adj_cap_nl != NL) {
+    if (ctx->adj_cap_np != S.Np || ctx->adj_cap_k != prm->K || ctx->adj_cap_nl != NL || ctx->adj_cap_it < iters) {
         CKR(cudaStreamSynchronize(st));
         free_pool(ctx->adj_bufs);
         ctx->adj_np = ctx->adj_k = 0;
         ctx->adj_cap_np = ctx->adj_cap_k = ctx->adj_cap_nl = 0;
         auto& pool = ctx->adj_bufs;
+        const int cap_it = std::max(iters, 64);
+        if (ctx->adj_counts) cudaFreeHost(ctx->adj_counts);
+        ctx->adj_counts = nullptr;
+        ctx->adj_cap_it = 0;
+        CKR(cudaMallocHost(&ctx->adj_counts, 2 * sizeof(unsigned) * (size_t)cap_it));
+        for (cudaEvent_t& e : ctx->adj_seen)
+            if (!e) CKR(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         b = adj::Bufs{};
+        b.host_counts = ctx->adj_counts;
+        b.seen[0] = ctx->adj_seen[0];
+        b.seen[1] = ctx->adj_seen[1];
+        const size_t nbits = adj::bit_words(S.Np);
+        for (auto& pair : b.bits)
+            for (uint32_t*& w : pair)
+                if ((s = dalloc(ctx, pool, &w, nbits))) return s;
+        if ((s = dalloc(ctx, pool, &b.marks, nbits)) || (s = dalloc(ctx, pool, &b.counts, 2 * (size_t)cap_it))) return s;
         float4* AEu = nullptr;
         const float* ones = nullptr;
         if ((s = dalloc(ctx, pool, &b.hits, Np * K)) || (s = dalloc(ctx, pool, &b.cnt, Np + 1)) || (s = dalloc(ctx, pool, &b.off, Np + 1)) ||
@@ -2244,6 +2264,7 @@ rc_status rc_adjoint(rc_ctx* ctx, const rc_adjoint_params* prm, const float* wei
         ctx->adj_cap_np = S.Np;
         ctx->adj_cap_k = prm->K;
         ctx->adj_cap_nl = NL;
+        ctx->adj_cap_it = cap_it;
     }
     float4* AEu = ctx->adj_aeu;
     const float* ones = ctx->adj_ones;
