@@ -186,52 +186,54 @@ __device__ __forceinline__ void note_bits(bool changed, int i, int Np, uint32_t*
     if (threadIdx.x == 0 && n) atomicAdd(count, (unsigned)n);
 }
 
-// forward sweep: L_i from the previous sweep's g; writes L and the next sweep's g = A (d + L)
-__global__ void __launch_bounds__(B) k_fwd(const int* __restrict__ hits, int K, int Np, const float2* __restrict__ da,
-                                           const float* __restrict__ gin, const float* __restrict__ Lprev, float* __restrict__ Lout,
-                                           float* __restrict__ gout, uint32_t* __restrict__ bits, unsigned* __restrict__ count, unsigned* chg) {
-    const int i = blockIdx.x * B + threadIdx.x;
+struct Fwd {   // a forward sweep: L_i from the previous sweep's g; writes L and the next sweep's g = A (d + L)
+    const int* hits;
+    const float2* da;
+    const float *gin, *Lprev;
+    float *Lout, *gout;
+    uint32_t* bits;
+    unsigned* count;
+};
+struct Bwd {   // an adjoint sweep
+    const int *off, *src;
+    const float2* da;
+    const float *w, *uin;
+    float* uout;
+    uint32_t* bits;
+    unsigned* count;
+};
+// Full sweeps: the first nf blocks forward, the others adjoint (the two do not depend on each other, and
+// together they have one tail instead of two: 129 us where the launches of their own took 67 + 70).  chg (may be null): the sweeps' largest changes
+// and values.
+__global__ void __launch_bounds__(B, 8) k_sweep(const Fwd f, const Bwd a, int nf, int K, int Np, unsigned* chg) {
+    const bool fwd = (int)blockIdx.x < nf;
+    const int i = (fwd ? (int)blockIdx.x : (int)blockIdx.x - nf) * B + threadIdx.x;
+    uint32_t* bits = fwd ? f.bits : a.bits;
     float v = 0.f, dv = 0.f;
     bool changed = false;
     if (i < Np) {
-        v = fwd_value(hits, K, i, gin);
-        Lout[i] = v;
-        const float2 x = da[i];
-        const float g = x.y * (x.x + v);
-        gout[i] = g;
-        if (bits) changed = differ(g, gin[i]);
-        dv = fabsf(v - Lprev[i]);
-    }
-    if (bits) note_bits(changed, i, Np, bits, count);
-    if (chg) {   // change of the sweep, and the largest value (non-negative floats order as their bits)
-        const unsigned a = warp_max(__float_as_uint(dv)), b = warp_max(__float_as_uint(fabsf(v)));
-        if ((threadIdx.x & 31) == 0) {
-            atomicMax(&chg[0], a);
-            atomicMax(&chg[1], b);
+        if (fwd) {
+            v = fwd_value(f.hits, K, i, f.gin);
+            f.Lout[i] = v;
+            const float2 x = f.da[i];
+            const float g = x.y * (x.x + v);
+            f.gout[i] = g;
+            if (bits) changed = differ(g, f.gin[i]);
+            dv = fabsf(v - f.Lprev[i]);
+        } else {
+            v = bwd_value(a.src, a.off[i], a.off[i + 1], K, a.da[i].y, a.w[i], a.uin);
+            a.uout[i] = v;
+            const float u = a.uin[i];
+            changed = differ(v, u);
+            dv = fabsf(v - u);
         }
     }
-}
-
-// adjoint sweep
-__global__ void __launch_bounds__(B) k_bwd(const int* __restrict__ off, const int* __restrict__ src, int K, int Np,
-                                           const float2* __restrict__ da, const float* __restrict__ w, const float* __restrict__ uin,
-                                           float* __restrict__ uout, uint32_t* __restrict__ bits, unsigned* __restrict__ count, unsigned* chg) {
-    const int j = blockIdx.x * B + threadIdx.x;
-    float v = 0.f, dv = 0.f;
-    bool changed = false;
-    if (j < Np) {
-        v = bwd_value(src, off[j], off[j + 1], K, da[j].y, w[j], uin);
-        uout[j] = v;
-        const float u = uin[j];
-        changed = differ(v, u);
-        dv = fabsf(v - u);
-    }
-    if (bits) note_bits(changed, j, Np, bits, count);
-    if (chg) {
-        const unsigned a = warp_max(__float_as_uint(dv)), b = warp_max(__float_as_uint(fabsf(v)));
+    if (bits) note_bits(changed, i, Np, bits, fwd ? f.count : a.count);
+    if (chg) {   // change of the sweep, and the largest value (non-negative floats order as their bits)
+        const unsigned x = warp_max(__float_as_uint(dv)), y = warp_max(__float_as_uint(fabsf(v)));
         if ((threadIdx.x & 31) == 0) {
-            atomicMax(&chg[2], a);
-            atomicMax(&chg[3], b);
+            atomicMax(&chg[fwd ? 0 : 2], x);
+            atomicMax(&chg[fwd ? 1 : 3], y);
         }
     }
 }
@@ -258,48 +260,42 @@ __global__ void __launch_bounds__(B) k_touch(const uint32_t* __restrict__ bits, 
         }
     }
 }
-__global__ void __launch_bounds__(B) k_fwd_few(const int* __restrict__ hits, int K, int Np, const float2* __restrict__ da,
-                                               const float* __restrict__ gin, const float* __restrict__ Lprev, float* __restrict__ Lout,
-                                               float* __restrict__ gout, uint32_t* __restrict__ marks, uint32_t* __restrict__ bits,
-                                               unsigned* __restrict__ count) {
+__global__ void __launch_bounds__(B) k_fwd_few(const Fwd f, int K, int Np, uint32_t* __restrict__ marks) {
     const int i = blockIdx.x * B + threadIdx.x;
     const uint32_t word = i < Np ? marks[i >> 5] : 0u;
     __syncwarp();
     if ((threadIdx.x & 31) == 0 && word) marks[i >> 5] = 0u;
     bool changed = false;
     if (i < Np) {
-        const float g0 = gin[i];
-        float v = Lprev[i], g = g0;
+        const float g0 = f.gin[i];
+        float v = f.Lprev[i], g = g0;
         if (word >> (i & 31) & 1u) {
-            v = fwd_value(hits, K, i, gin);
-            const float2 x = da[i];
+            v = fwd_value(f.hits, K, i, f.gin);
+            const float2 x = f.da[i];
             g = x.y * (x.x + v);
             changed = differ(g, g0);
         }
-        Lout[i] = v;
-        gout[i] = g;
+        f.Lout[i] = v;
+        f.gout[i] = g;
     }
-    note_bits(changed, i, Np, bits, count);
+    note_bits(changed, i, Np, f.bits, f.count);
 }
-__global__ void __launch_bounds__(B) k_bwd_few(const int* __restrict__ off, const int* __restrict__ src, int K, int Np,
-                                               const float2* __restrict__ da, const float* __restrict__ w, const float* __restrict__ uin,
-                                               float* __restrict__ uout, uint32_t* __restrict__ marks, uint32_t* __restrict__ bits,
-                                               unsigned* __restrict__ count) {
+__global__ void __launch_bounds__(B) k_bwd_few(const Bwd a, int K, int Np, uint32_t* __restrict__ marks) {
     const int j = blockIdx.x * B + threadIdx.x;
     const uint32_t word = j < Np ? marks[j >> 5] : 0u;
     __syncwarp();
     if ((threadIdx.x & 31) == 0 && word) marks[j >> 5] = 0u;
     bool changed = false;
     if (j < Np) {
-        const float u = uin[j];
+        const float u = a.uin[j];
         float v = u;
         if (word >> (j & 31) & 1u) {
-            v = bwd_value(src, off[j], off[j + 1], K, da[j].y, w[j], uin);
+            v = bwd_value(a.src, a.off[j], a.off[j + 1], K, a.da[j].y, a.w[j], a.uin);
             changed = differ(v, u);
         }
-        uout[j] = v;
+        a.uout[j] = v;
     }
-    note_bits(changed, j, Np, bits, count);
+    note_bits(changed, j, Np, a.bits, a.count);
 }
 
 // Column c < NL: sum_j (u_j - w_j) G_c[j]; column NL: sum_j w_j L_j.  Block x sums a fixed slice of
@@ -427,17 +423,17 @@ cudaError_t solve(Bufs* bp, int Np, int K, int NL, int aes, const float* AE, con
         uint32_t *bi0 = follow ? b.bits[0][t & 1] : nullptr, *bi1 = follow ? b.bits[1][t & 1] : nullptr;
         uint32_t *bo0 = follow ? b.bits[0][(t + 1) & 1] : nullptr, *bo1 = follow ? b.bits[1][(t + 1) & 1] : nullptr;
         unsigned *c0 = follow ? b.counts + 2 * t : nullptr, *c1 = follow ? c0 + 1 : nullptr;
-        if (last || !few[0]) {
-            k_fwd<<<blocks_for(Np), B, 0, st>>>(b.hits, K, Np, b.da, b.g[t & 1], b.L[t & 1], b.L[(t + 1) & 1], b.g[(t + 1) & 1], bo0, c0, chg);
-        } else if (!still[0]) {
+        const Fwd f{b.hits, b.da, b.g[t & 1], b.L[t & 1], b.L[(t + 1) & 1], b.g[(t + 1) & 1], bo0, c0};
+        const Bwd a{b.off, b.src, b.da, b.w, b.u[t & 1], b.u[(t + 1) & 1], bo1, c1};
+        const int nb = blocks_for(Np), nf = last || !few[0] ? nb : 0, na = last || !few[1] ? nb : 0;
+        if (nf + na) k_sweep<<<nf + na, B, 0, st>>>(f, a, nf, K, Np, chg);
+        if (!nf && !still[0]) {
             k_touch<<<touch_blocks, B, 0, st>>>(bi0, words, b.off, b.src, K, b.marks);
-            k_fwd_few<<<blocks_for(Np), B, 0, st>>>(b.hits, K, Np, b.da, b.g[t & 1], b.L[t & 1], b.L[(t + 1) & 1], b.g[(t + 1) & 1], b.marks, bo0, c0);
+            k_fwd_few<<<nb, B, 0, st>>>(f, K, Np, b.marks);
         }
-        if (last || !few[1]) {
-            k_bwd<<<blocks_for(Np), B, 0, st>>>(b.off, b.src, K, Np, b.da, b.w, b.u[t & 1], b.u[(t + 1) & 1], bo1, c1, chg);
-        } else if (!still[1]) {
+        if (!na && !still[1]) {
             k_touch<<<touch_blocks, B, 0, st>>>(bi1, words, nullptr, b.hits, K, b.marks);
-            k_bwd_few<<<blocks_for(Np), B, 0, st>>>(b.off, b.src, K, Np, b.da, b.w, b.u[t & 1], b.u[(t + 1) & 1], b.marks, bo1, c1);
+            k_bwd_few<<<nb, B, 0, st>>>(a, K, Np, b.marks);
         }
         if (follow && (t & 1) && t + 3 < iters - 1) {   // read before sweep t + 3
             if ((e = cudaMemcpyAsync(b.host_counts + 2 * (t - 1), b.counts + 2 * (t - 1), 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, st)) !=
