@@ -907,6 +907,7 @@ __global__ void __launch_bounds__(BLOCK, RC_FRAME_MINB) k_frame(const DState s, 
     stage_smem(sm, s);
     if (threadIdx.x == 0) { prt.acc = 0ull; prt.arrived = 0u; }
     __syncthreads();
+    pdl_wait();
     const TraceSmem tsm = smem_view(sm, s);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int ntiles = (p.Np + BLOCK - 1) / BLOCK;
@@ -1111,6 +1112,8 @@ __global__ void __launch_bounds__(BLOCK, RC_FRAME_MINB) k_frame(const DState s, 
         }
     }
     }
+    pdl_release();
+    if (c.rayctr && blockIdx.x == 0 && threadIdx.x == 0) c.rayctr[1] = 0u;   // for the next frame's k_pretrace
     {
         // ray count of the frame: warp sum, one 64-bit atomic per warp
         const unsigned wk = __reduce_add_sync(0xffffffffu, ray_sum);
@@ -1147,7 +1150,7 @@ __global__ void __launch_bounds__(BLOCK, RC_FRAME_MINB) k_frame(const DState s, 
 // kernel, so more warps hide the latency.  The rays are the frame kernel's (same seed, ray
 // count and directions); the first pre_k of each point are traced, and their hit points and
 // cache points written for the frame kernel to read.  The grid is persistent: each warp takes
-// 32 consecutive points at a time from a counter (c.rayctr[1], zeroed before the launch), so a
+// 32 consecutive points at a time from a counter (c.rayctr[1], zeroed by the frame kernel for the next frame), so a
 // warp whose rays were short takes more points instead of leaving its block's slot idle until
 // the block's slowest warp ends (1.8 % per frame on a 199 k-triangle street).  Which warp
 // traces a point does not change its rays or its hits.
@@ -1160,6 +1163,7 @@ __global__ void __launch_bounds__(BLOCK, RC_PRETRACE_MINB) k_pretrace(const DSta
     extern __shared__ float4 sm[];
     stage_smem(sm, s);
     __syncthreads();
+    pdl_wait();
     const TraceSmem tsm = smem_view(sm, s);
     const int lane = threadIdx.x & 31;
     while (true) {
@@ -1181,6 +1185,7 @@ __global__ void __launch_bounds__(BLOCK, RC_PRETRACE_MINB) k_pretrace(const DSta
             out[(size_t)i * p.pre_k + r] = make_float4(h.H.x, h.H.y, h.H.z, __int_as_float(h.back ? -1 : h.pi));
         }
     }
+    pdl_release();
 }
 
 // ------------------------------------------------------------------ ray-queue traversal
@@ -1403,6 +1408,7 @@ __global__ void __launch_bounds__(BLOCK) k_update(const DState s, const DStatic 
     constexpr int LCS = lcs_of(NL);
     if (threadIdx.x == 0) { prt.acc = 0ull; prt.arrived = 0u; npt.acc = 0ull; npt.arrived = 0u; taild.arrived = 0u; }
     __syncthreads();
+    pdl_wait();
     const int i = blockIdx.x * BLOCK + threadIdx.x;
     float pr_out = 0.f;
     double e_d2 = 0.0, e_rs = 0.0, e_cn = 0.0;
@@ -1482,6 +1488,7 @@ __global__ void __launch_bounds__(BLOCK) k_update(const DState s, const DStatic 
             e_cn = 1.0;
         }
     }
+    pdl_release();
     unsigned long long tot;
     if (u64_tail_reduce(pr_fixed(pr_out), prt, c.pracc, c.ticket, tot)) c.sumpr[p.sum_out] = fixed_to_float(tot);
     if (p.want_err) {
@@ -1516,6 +1523,7 @@ __global__ void __launch_bounds__(BLOCK) k_event(const __grid_constant__ EvProgr
     constexpr int LCS = lcs_of(NL);
     if (threadIdx.x == 0) { prt.acc = 0ull; prt.arrived = 0u; npt.acc = 0ull; npt.arrived = 0u; }
     __syncthreads();
+    pdl_wait();
     const int i = blockIdx.x * BLOCK + threadIdx.x;
     const int Np = ev.Np;
     if (ev.zero_rstat)
@@ -1987,6 +1995,7 @@ __global__ void __launch_bounds__(BLOCK) k_taa_pt(const DState s, const DStatic 
     extern __shared__ float4 sm[];
     stage_smem(sm, s);
     __syncthreads();
+    pdl_wait();
     const TraceSmem tsm = smem_view(sm, s);
     const int i = blockIdx.x * BLOCK + threadIdx.x;
     if (i >= p.Np) return;
@@ -2067,17 +2076,16 @@ static cudaError_t resident_grid(const void* kern, size_t smem, int& out, int th
 template <int NL>
 cudaError_t Ops<NL>::pretrace(const DState& s, const DStatic& g, const Grid& grid, const DevCache& c, const FrameParams& p,
                               float4* out, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(c.rayctr, 0, 2 * sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
     if (!p.wavefront || !c.rayq) {   // one thread per point, persistent warps
         const size_t smem = frame_smem_bytes(s);
         if ((e = prep_smem(k_pretrace<NL>, smem)) != cudaSuccess) return e;
         int resident = 0;
         if ((e = resident_grid((const void*)k_pretrace<NL>, smem, resident, BLOCK)) != cudaSuccess) return e;
-        k_pretrace<NL><<<std::max(1, std::min(resident, grid_of(p.Np))), BLOCK, smem, st>>>(s, g, grid, c, p, out);
-        return cudaGetLastError();
+        return launch_dependent(k_pretrace<NL>, std::max(1, std::min(resident, grid_of(p.Np))), BLOCK, smem, st, s, g, grid, c, p, out);
     }
     // ray queue: compacted rays, then the persistent traversal
+    if ((e = cudaMemsetAsync(c.rayctr, 0, 2 * sizeof(unsigned), st)) != cudaSuccess) return e;
     k_ray_queue<NL><<<grid_of(p.Np), BLOCK, 0, st>>>(s, c, p);
     const size_t smem = trace_queue_smem(s);
     auto kern = g.watertight ? k_trace_queue<true> : k_trace_queue<false>;
@@ -2124,8 +2132,7 @@ cudaError_t Ops<NL>::taa_sample(int NW, bool deps, const DState& s, const DStati
         auto kern = deps ? k_taa_pt<NL, W, true> : k_taa_pt<NL, W, false>;                                     \
         cudaError_t e = prep_smem(kern, smem);                                                                 \
         if (e != cudaSuccess) return e;                                                                        \
-        kern<<<grid_of(p.Np), BLOCK, smem, st>>>(s, g, grid, c, p, x, cur, seed, frame);                       \
-        return cudaGetLastError();                                                                             \
+        return launch_dependent(kern, grid_of(p.Np), BLOCK, smem, st, s, g, grid, c, p, x, cur, seed, frame);  \
     }
     RC_NW_LIST(X)
 #undef X
@@ -2178,9 +2185,7 @@ static cudaError_t frame_t(const DState& s, const DStatic& g, const Grid& grid, 
     if (e != cudaSuccess) return e;
     int resident = 0;
     if ((e = resident_grid((const void*)k_frame<NL, NW, DEPS, FUSED>, smem, resident, BLOCK)) != cudaSuccess) return e;
-    const int blocks = std::min(grid_of(p.Np), resident);
-    k_frame<NL, NW, DEPS, FUSED><<<blocks, BLOCK, smem, st>>>(s, g, grid, c, p);
-    return cudaGetLastError();
+    return launch_dependent(k_frame<NL, NW, DEPS, FUSED>, std::min(grid_of(p.Np), resident), BLOCK, smem, st, s, g, grid, c, p);
 }
 
 template <int NL>
@@ -2200,14 +2205,12 @@ cudaError_t Ops<NL>::frame(int NW, bool deps, bool fused, const DState& s, const
 
 template <int NL>
 cudaError_t Ops<NL>::update(const DState& s, const DStatic& g, const DevCache& c, const FrameParams& p, cudaStream_t st) {
-    k_update<NL><<<grid_of(p.Np), BLOCK, 0, st>>>(s, g, c, p);
-    return cudaGetLastError();
+    return launch_dependent(k_update<NL>, grid_of(p.Np), BLOCK, 0, st, s, g, c, p);
 }
 
 template <int NL>
 cudaError_t Ops<NL>::event(const EvProgram& ev, const DevCache& c, cudaStream_t st) {
-    k_event<NL><<<grid_of(ev.Np), BLOCK, 0, st>>>(ev, c);
-    return cudaGetLastError();
+    return launch_dependent(k_event<NL>, grid_of(ev.Np), BLOCK, 0, st, ev, c);
 }
 
 template <int NL>

@@ -16,11 +16,15 @@
 #include <vector>
 
 #include "../../include/rc_mlp.h"
+#include "rc_internal.h"
 #include "rc_umma.cuh"
 
 namespace {
 
 using namespace rc::umma;
+using rc::launch_dependent;
+using rc::pdl_release;
+using rc::pdl_wait;
 
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
 constexpr int TILE_M = 128;
@@ -426,11 +430,13 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int n
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int W_ENCODE = TR_CHAIN / 32, W_ISSUE = (TR_CHAIN + TR_ENCODE) / 32;
+    pdl_release();
     if (tid == 0) mbar_init(&mbar, 1);
     if (warp == W_ISSUE) tmem_alloc(&tmem_base, TR_COLS);
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
+    pdl_wait();   // the kernel before: the last step's weights, the caller's inputs
     const uint32_t tmem = tmem_base, sm0 = smem_u32(smem);
     const int count = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // tiles of this CTA
     auto hbuf = [](int l) { return (uint32_t)(TS_H + (l - 1) * (128 * HID * 2)); };
@@ -668,6 +674,8 @@ static_assert(NWEIGHT % GWEIGHTS == 0, "whole blocks of weights");
 __global__ void __launch_bounds__(GSLICES * GWEIGHTS / 4) k_mlp_gsum(const float* __restrict__ part, int nctas, float* __restrict__ gsum,
                                                                      unsigned* __restrict__ words) {
     __shared__ float slice[GSLICES][GWEIGHTS];
+    pdl_release();
+    part = pdl_wait(part);
     const int w4 = threadIdx.x % (GWEIGHTS / 4), s = threadIdx.x / (GWEIGHTS / 4);
     const float4* p = reinterpret_cast<const float4*>(part) + blockIdx.x * (GWEIGHTS / 4) + w4;
     float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -697,6 +705,10 @@ __global__ void __launch_bounds__(128) k_mlp_adam(const float* __restrict__ gsum
                                                   float* __restrict__ m2, float* __restrict__ grad, uint8_t* __restrict__ wbf, float lr, float b1,
                                                   float b2, float eps, float* st, unsigned* words) {
     const int i = blockIdx.x * 128 + threadIdx.x;
+    pdl_release();
+    st = pdl_wait(st);
+    gsum = pdl_wait(gsum);
+    words = pdl_wait(words);
     const float4 s = __ldcg(reinterpret_cast<const float4*>(st));
     const bool skip = __ldcg(words + WD_NONFINITE) != 0u;
     const float scale = s.x, t = s.y + 1.f;
@@ -905,10 +917,12 @@ rc_status rc_mlp_train(rc_mlp* m, const float* d_pos4, const float* d_nrm4, cons
     m->step++;
     const float b1 = 0.9f, b2 = 0.99f;
     if (!d_loss && cudaMemsetAsync(m->loss, 0, 4, m->stream) != cudaSuccess) return mfail(m, RC_ERR_CUDA, "clear");
-    k_mlp_train<<<ctas, TR_THREADS, TRAIN_SMEM, m->stream>>>(a, ntiles);
-    k_mlp_gsum<<<NWEIGHT / GWEIGHTS, GSLICES * GWEIGHTS / 4, 0, m->stream>>>(m->part, ctas, m->gsum, m->words);
-    k_mlp_adam<<<NWEIGHT / 128, 128, 0, m->stream>>>(m->gsum, m->w, m->m1, m->m2, m->grad, m->wbf, m->cfg.lr, b1, b2, 1e-8f, m->state, m->words);
-    return cudaGetLastError() == cudaSuccess ? RC_OK : mfail(m, RC_ERR_CUDA, "launch");
+    if (launch_dependent(k_mlp_train, ctas, TR_THREADS, TRAIN_SMEM, m->stream, a, ntiles) != cudaSuccess ||
+        launch_dependent(k_mlp_gsum, NWEIGHT / GWEIGHTS, GSLICES * GWEIGHTS / 4, 0, m->stream, m->part, ctas, m->gsum, m->words) != cudaSuccess ||
+        launch_dependent(k_mlp_adam, NWEIGHT / 128, 128, 0, m->stream, m->gsum, m->w, m->m1, m->m2, m->grad, m->wbf, m->cfg.lr, b1, b2, 1e-8f,
+                         m->state, m->words) != cudaSuccess)
+        return mfail(m, RC_ERR_CUDA, "launch");
+    return RC_OK;
 }
 
 rc_status rc_mlp_infer(rc_mlp* m, const float* d_pos4, const float* d_nrm4, const float* d_aux4, int n, float* d_out, int ostride) {

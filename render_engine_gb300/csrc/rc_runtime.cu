@@ -1719,6 +1719,7 @@ rc_status rc_run_begin(rc_ctx* ctx, const rc_method* m, int s0, uint32_t seed) {
         CKR(cudaMemcpyAsync(c.sumpr, sp, 8, cudaMemcpyHostToDevice, st));
         CKR(cudaMemcpyAsync(c.npend, z2, 8, cudaMemcpyHostToDevice, st));
         CKR(cudaMemsetAsync(c.rays, 0, 8, st));
+        if (c.rayctr) CKR(cudaMemsetAsync(c.rayctr, 0, 2 * sizeof(unsigned), st));
         CKR(cudaStreamSynchronize(st));   // sp and z2 are about to go out of scope
     }
     R.p.seed = seed;
