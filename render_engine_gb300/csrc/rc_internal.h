@@ -18,7 +18,7 @@ namespace rc {
 // kernel's blocks come as room appears and orders nothing.  A frame's kernels release at the end
 // of their tiles: blocks of the next grid that come earlier gather on the multiprocessors that
 // run dry first, which makes the next kernel uneven (213 k points, 8 lights, 12 frames: 509 us
-// against 461, and 485 with plain launches).  16 frames of 4 k points 217 -> 177 us, of 1.08 M
+// against 461, and 485 with plain launches).  16 frames of 10.7 k points 217 -> 177 us, of 1.08 M
 // points 952 -> 906; 4 training steps of 65,536 points 258 -> 245.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // the same wait, with the pointer's loads behind it also where the compiler holds the data constant

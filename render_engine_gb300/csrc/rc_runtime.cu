@@ -117,6 +117,7 @@ struct TaaRun {
     uint8_t* pend = nullptr;
     uint32_t *cur = nullptr, *prev = nullptr;
     double *part = nullptr, *out = nullptr;
+    unsigned* ticket = nullptr;     // blocks of the update that have arrived
     std::vector<const int*> dV;     // event voxels per state pair (device), and their counts
     std::vector<int> nV;
     // per state: the sum of the references over the valid points and their count (the error's
@@ -1497,8 +1498,9 @@ rc_status taa_alloc(rc_ctx* ctx) {
         (s = dalloc(ctx, pool, &t.pend, Np)) || (s = dalloc(ctx, pool, &t.cur, NW * Np)) || (s = dalloc(ctx, pool, &t.prev, NW * Np)) ||
         (s = dalloc(ctx, pool, &t.rs, 3 * (size_t)S.NR)) || (s = dalloc(ctx, pool, &t.cnt, (size_t)S.NR)) ||
         (s = dalloc(ctx, pool, &t.part, 3 * (size_t)taa::post_blocks(S.Np))) || (s = dalloc(ctx, pool, &t.out, 3)) ||
-        (s = dput(ctx, pool, &dq, qid)) || (s = dput(ctx, pool, &dquad, quad)))
+        (s = dalloc(ctx, pool, &t.ticket, 1)) || (s = dput(ctx, pool, &dq, qid)) || (s = dput(ctx, pool, &dquad, quad)))
         return s;
+    CKR(cudaMemsetAsync(t.ticket, 0, sizeof(unsigned), ctx->stream));
     t.qid = const_cast<int*>(dq);
     t.quad = dquad;
     const int NS = S.NS, NL = S.NL;
@@ -2427,17 +2429,16 @@ rc_status rc_taa_frame(rc_ctx* ctx, int state, float* err) {
         t.ref_cnt[state] = h[2];
         t.have_sums[state] = 1;
     }
+    // the squared error arrives in page-locked memory, written by the kernel
+    if (err && !ctx->pinned) CKR(cudaMallocHost(&ctx->pinned, 8 * sizeof(double)));
     CKR(taa::post(t.x, t.qid, t.quad, t.H, t.H2, t.mu, t.sg, t.react, Np, M.alpha, TAA_ALPHA_R, M.gamma, d.ref, d.valid, err ? t.part : nullptr,
-                  t.out, st));
-    kernels += err ? 2 : 1;
+                  t.ticket, ctx->pinned, st));
+    ++kernels;
     std::swap(t.H, t.H2);
     ctx->launches += kernels;
     t.prev_state = state;
     t.f = f + 1;
     if (err) {
-        // the squared error through page-locked memory: one DMA, no staging copy
-        if (!ctx->pinned) CKR(cudaMallocHost(&ctx->pinned, 8 * sizeof(double)));
-        CKR(cudaMemcpyAsync(ctx->pinned, t.out, sizeof(double), cudaMemcpyDeviceToHost, st));
         CKR(cudaStreamSynchronize(st));
         const double d2 = ctx->pinned[0];
         const double rs = t.ref_sum[state], cn = t.ref_cnt[state];

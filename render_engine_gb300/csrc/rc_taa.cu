@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "rc_internal.h"
 #include "rc_taa.h"
 
 namespace rc {
@@ -133,7 +134,9 @@ __device__ __forceinline__ float2 df_add(float2 a, float2 b) {
 // added in warp order the same way (the FP64 pipe of this GPU is a small fraction of its
 // FP32 rate), one conversion to FP64 per block.  The sums of the
 // references and of the valid points, which do not change within a state, come from
-// k_ref_sums.  The 3x3
+// k_ref_sums.  The last block to arrive adds the partials in block order, 256 strided runs and a tree
+// (a kernel of its own took 8.7 us and a launch), and stores the sum where the host reads it, without a
+// copy: a call on 1.08 M points 110 -> 98 us.  The 3x3
 // neighbourhood on the point's quad grid (run_taa_mode's table, poc_gpu.cu:1192-1203) is
 // derived from the point's quad: quad[q] = (first point, nu, nv), neighbours in the table's
 // order (dv outer, du inner), -1 outside the grid; a point of no quad has no neighbours.
@@ -141,8 +144,12 @@ __global__ void __launch_bounds__(B) k_post(const float* __restrict__ x, const i
                                             const float* __restrict__ H,
                                             float* __restrict__ H2, float* __restrict__ mu_out, float* __restrict__ sg_out,
                                             int* __restrict__ react, int Np, float alpha, float alpha_r, float gamma,
-                                            const float* __restrict__ ref, const uint8_t* __restrict__ valid, double* __restrict__ part) {
+                                            const float* __restrict__ ref, const uint8_t* __restrict__ valid, double* part, unsigned* ticket,
+                                            double* out) {
     __shared__ float2 sh[B / 32];
+    __shared__ double fin[B];
+    __shared__ bool last;
+    x = pdl_wait(x);
     const int i = blockIdx.x * B + threadIdx.x;
     float2 d2 = make_float2(0.f, 0.f);
     if (i < Np) {
@@ -206,6 +213,23 @@ __global__ void __launch_bounds__(B) k_post(const float* __restrict__ x, const i
         float2 t = sh[0];
         for (int w = 1; w < B / 32; ++w) t = df_add(t, sh[w]);
         part[3 * (size_t)blockIdx.x] = (double)t.x + (double)t.y;
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double a = 0.0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += B) a += __ldcg(part + 3 * (size_t)k);
+    fin[threadIdx.x] = a;
+    __syncthreads();
+    for (int o = B / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o) fin[threadIdx.x] += fin[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        *out = fin[0];
+        *ticket = 0u;   // for the next frame
     }
 }
 
@@ -269,10 +293,11 @@ cudaError_t zone_decide(const float* rs, const float* cnt, uint8_t* pend, const 
 }
 
 cudaError_t post(const float* x, const int* qid, const int4* quad, const float* H, float* H2, float* mu, float* sg, int* react, int Np,
-                 float alpha, float alpha_r, float gamma, const float* ref, const uint8_t* valid, double* part, double* out, cudaStream_t st) {
-    k_post<<<blocks(Np), B, 0, st>>>(x, qid, quad, H, H2, mu, sg, react, Np, alpha, alpha_r, gamma, ref, valid, part);
-    if (part) k_err_final<<<1, B, 0, st>>>(part, blocks(Np), out);
-    return cudaGetLastError();
+                 float alpha, float alpha_r, float gamma, const float* ref, const uint8_t* valid, double* part, unsigned* ticket, double* out,
+                 cudaStream_t st) {
+    cudaError_t e = launch_dependent(k_post, blocks(Np), B, 0, st, x, qid, quad, H, H2, mu, sg, react, Np, alpha, alpha_r, gamma, ref, valid, part,
+                                     ticket, out);
+    return e;
 }
 
 cudaError_t ref_sums(const float* ref, const uint8_t* valid, int Np, double* part, double* out, cudaStream_t st) {
