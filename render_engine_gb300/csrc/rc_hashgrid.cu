@@ -280,11 +280,8 @@ __device__ __forceinline__ void dep_or(uint4* bank, uint32_t e, uint4 m) {
 // Paths are either contiguous (ps = npaths + 1 offsets) or in fixed slots (ps = NULL, path p is
 // v[p * stride .. p * stride + plen[p])).
 template <bool WIDE>
-__global__ void __launch_bounds__(HG_BLOCK) k_hg_mark(const HgDev c, const rc_hg_vertex* __restrict__ v,
-                                                      const int* __restrict__ ps, const int* __restrict__ plen, int stride, int npaths,
-                                                      uint4* bw, const uint4* b0, const uint4* b1) {
-    const int p = blockIdx.x * HG_BLOCK + threadIdx.x;
-    if (p >= npaths) return;
+__device__ __forceinline__ void mark_path(const HgDev& c, const rc_hg_vertex* __restrict__ v, const int* __restrict__ ps,
+                                          const int* __restrict__ plen, int stride, int p, uint4* bw, const uint4* b0, const uint4* b1) {
     uint32_t idx[RC_HG_MAX_DEPTH];
     int len = 0;
     const int D = c.depth;
@@ -331,6 +328,14 @@ __global__ void __launch_bounds__(HG_BLOCK) k_hg_mark(const HgDev c, const rc_hg
     }
 }
 
+template <bool WIDE>
+__global__ void __launch_bounds__(HG_BLOCK, 4) k_hg_mark(const HgDev c, const rc_hg_vertex* __restrict__ v,
+                                                      const int* __restrict__ ps, const int* __restrict__ plen, int stride, int npaths,
+                                                      uint4* bw, const uint4* b0, const uint4* b1) {
+    const int p = blockIdx.x * HG_BLOCK + threadIdx.x;
+    if (p < npaths) mark_path<WIDE>(c, v, ps, plen, stride, p, bw, b0, b1);
+}
+
 // ------------------------------------------------------------------ per-voxel light masks
 // A res^3 grid over the zone box: voxel of a point per axis int((x - lo) * scale), clamped, with
 // scale = res / (hi - lo) rounded once on the host; explicitly rounded operations.
@@ -364,45 +369,69 @@ __constant__ float c_seg19[20] = {0.f / 19.f,  1.f / 19.f,  2.f / 19.f,  3.f / 1
 // reads (64-bit words of the L2), so ten of them are in flight at a time.  1920 x 1080 paths, three
 // slots each, 128^3 voxels: 336 us with a thread per path and four reads in flight, 293 us (L2 70 % busy).
 template <bool WIDE>
+__device__ __forceinline__ void vox_slot(const HgDev& c, const VoxDev& g, const rc_hg_vertex* __restrict__ v, const int* __restrict__ plen,
+                                         int stride, long long j, unsigned long long* __restrict__ vox) {
+    const int res = g.res;
+            const long long p = j / stride;
+            if (j - p * stride >= plen[p]) return;
+            const rc_hg_vertex x = load_vertex<WIDE>(v + j);
+            if ((x.flags & RC_HG_MISS) || x.light_index < 0 || x.light_index >= 64 || !(x.flags & RC_HG_LIGHT_VISIBLE)) return;
+            const unsigned long long bit = 1ull << x.light_index;
+            const float r = mn(x.light_dist, c.td);
+            float a[3], d[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                a[k] = x.hit[k];
+                d[k] = __fmul_rn(x.to_light[k], r);
+            }
+            unsigned last = ~0u;   // consecutive samples in one voxel mark it once (res <= 256: 24-bit indexes)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                unsigned vi[10];
+                bool on[10];
+                unsigned long long w[10];
+#pragma unroll
+                for (int k = 0; k < 10; ++k) {
+                    const float t = c_seg19[10 * h + k];
+                    const int ix = vox_axis(__fadd_rn(a[0], __fmul_rn(d[0], t)), g.lo[0], g.scale[0], res);
+                    const int iy = vox_axis(__fadd_rn(a[1], __fmul_rn(d[1], t)), g.lo[1], g.scale[1], res);
+                    const int iz = vox_axis(__fadd_rn(a[2], __fmul_rn(d[2], t)), g.lo[2], g.scale[2], res);
+                    vi[k] = (unsigned)((iz * res + iy) * res + ix);
+                    on[k] = vi[k] != last;
+                    last = vi[k];
+                }
+#pragma unroll
+                for (int k = 0; k < 10; ++k) w[k] = on[k] ? __ldcg(vox + vi[k]) : bit;
+#pragma unroll
+                for (int k = 0; k < 10; ++k)
+                    if (!(w[k] & bit)) atomicOr(vox + vi[k], bit);
+            }
+}
+template <bool WIDE>
 __global__ void __launch_bounds__(HG_BLOCK) k_vox_mark(const HgDev c, const VoxDev g, const rc_hg_vertex* __restrict__ v,
                                                        const int* __restrict__ plen, int stride, long long nslots,
                                                        unsigned long long* __restrict__ vox) {
-    const int res = g.res;
-    for (long long j = blockIdx.x * (long long)HG_BLOCK + threadIdx.x; j < nslots; j += (long long)gridDim.x * HG_BLOCK) {
-        const long long p = j / stride;
-        if (j - p * stride >= plen[p]) continue;
-        const rc_hg_vertex x = load_vertex<WIDE>(v + j);
-        if ((x.flags & RC_HG_MISS) || x.light_index < 0 || x.light_index >= 64 || !(x.flags & RC_HG_LIGHT_VISIBLE)) continue;
-        const unsigned long long bit = 1ull << x.light_index;
-        const float r = mn(x.light_dist, c.td);
-        float a[3], d[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            a[k] = x.hit[k];
-            d[k] = __fmul_rn(x.to_light[k], r);
-        }
-        unsigned last = ~0u;   // consecutive samples in one voxel mark it once (res <= 256: 24-bit indexes)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            unsigned vi[10];
-            bool on[10];
-            unsigned long long w[10];
-#pragma unroll
-            for (int k = 0; k < 10; ++k) {
-                const float t = c_seg19[10 * h + k];
-                const int ix = vox_axis(__fadd_rn(a[0], __fmul_rn(d[0], t)), g.lo[0], g.scale[0], res);
-                const int iy = vox_axis(__fadd_rn(a[1], __fmul_rn(d[1], t)), g.lo[1], g.scale[1], res);
-                const int iz = vox_axis(__fadd_rn(a[2], __fmul_rn(d[2], t)), g.lo[2], g.scale[2], res);
-                vi[k] = (unsigned)((iz * res + iy) * res + ix);
-                on[k] = vi[k] != last;
-                last = vi[k];
-            }
-#pragma unroll
-            for (int k = 0; k < 10; ++k) w[k] = on[k] ? __ldcg(vox + vi[k]) : bit;
-#pragma unroll
-            for (int k = 0; k < 10; ++k)
-                if (!(w[k] & bit)) atomicOr(vox + vi[k], bit);
-        }
+    for (long long j = blockIdx.x * (long long)HG_BLOCK + threadIdx.x; j < nslots; j += (long long)gridDim.x * HG_BLOCK)
+        vox_slot<WIDE>(c, g, v, plen, stride, j, vox);
+}
+
+// Both marks of a pass of camera paths: of every 1 + stride blocks the first marks the masks of 256
+// paths, the others the voxels of 256 slots each.  The two do not depend on each other; the first is
+// bound by its instructions, the second by the L2, and side by side on a multiprocessor they take
+// 40 us less of 1920 x 1080 three-vertex paths (1398 us a pass; 1438 with a launch each).  Four blocks an
+// SM (64 registers) for this kernel and for k_hg_mark: 1462 us at three, 1406 at five.  Adding the
+// samples (k_hg_accum) in the same launch: 1414.
+template <bool WIDE>
+__global__ void __launch_bounds__(HG_BLOCK, 4) k_path_marks(const HgDev c, const VoxDev g, const rc_hg_vertex* __restrict__ v,
+                                                         const int* __restrict__ plen, int stride, int npaths, uint4* bw, const uint4* b0,
+                                                         const uint4* b1, unsigned long long* __restrict__ vox) {
+    const int grp = blockIdx.x / (unsigned)(stride + 1), k = blockIdx.x % (unsigned)(stride + 1);
+    if (k == 0) {
+        const int p = grp * HG_BLOCK + threadIdx.x;
+        if (p < npaths) mark_path<WIDE>(c, v, nullptr, plen, stride, p, bw, b0, b1);
+    } else {
+        const long long j = ((long long)grp * stride + (k - 1)) * HG_BLOCK + threadIdx.x;
+        if (j < (long long)npaths * stride) vox_slot<WIDE>(c, g, v, plen, stride, j, vox);
     }
 }
 
@@ -1012,6 +1041,13 @@ bool hg_has_voxels(const rc_hg* hg) { return hg->vres > 0; }
 cudaError_t hg_insert_vertices(rc_hg* hg, const float* pos, const float* nrm, int n, uint32_t* entry, rc_hg_vertex* v) {
     if (n <= 0) return cudaSuccess;
     k_hg_insert<<<grid_for(n, HG_BLOCK), HG_BLOCK, 0, hg->stream>>>(dev_of(hg), pos, nrm, n, hg->keys, entry, v);
+    return cudaGetLastError();
+}
+cudaError_t hg_path_marks(rc_hg* hg, const rc_hg_vertex* v, const int* len, int stride, int npaths) {
+    if (npaths <= 0) return cudaSuccess;
+    auto kern = wide_vertices(v) ? k_path_marks<true> : k_path_marks<false>;
+    kern<<<grid_for(npaths, HG_BLOCK) * (stride + 1), HG_BLOCK, 0, hg->stream>>>(dev_of(hg), vox_dev(hg), v, len, stride, npaths,
+                                                                                 hg->bank[hg->bank_sel], hg->bank[0], hg->bank[1], hg->vox);
     return cudaGetLastError();
 }
 }  // namespace rc

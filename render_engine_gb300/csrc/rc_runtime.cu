@@ -2562,9 +2562,8 @@ rc_status rc_hg_camera_paths(rc_hg* hg, rc_ctx* ctx, int state, const rc_hg_path
     const int n = (int)nslots, np = (int)npix;
     CKR(rc::hg_insert_vertices(hg, C.pos, C.nrm, n, C.entry, C.vtx));
     if ((st = rc_hg_accumulate(hg, C.entry, C.rgb, n))) return fail(ctx, st, "accumulate: %s", rc_hg_last_error(hg));
-    if ((st = rc_hg_mark_paths_strided(hg, C.vtx, C.len, (int)S1, np))) return fail(ctx, st, "mark: %s", rc_hg_last_error(hg));
-    if (rc::hg_has_voxels(hg) && (st = rc_hg_voxels_mark(hg, C.vtx, C.len, (int)S1, np)))
-        return fail(ctx, st, "voxels: %s", rc_hg_last_error(hg));
+    if (rc::hg_has_voxels(hg)) CKR(rc::hg_path_marks(hg, C.vtx, C.len, (int)S1, np));
+    else if ((st = rc_hg_mark_paths_strided(hg, C.vtx, C.len, (int)S1, np))) return fail(ctx, st, "mark: %s", rc_hg_last_error(hg));
     // the context's later work waits for this pass
     CKR(cudaEventRecord(C.ready, hs));
     CKR(cudaStreamWaitEvent(ctx->stream, C.ready, 0));

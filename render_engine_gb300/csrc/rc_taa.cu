@@ -220,7 +220,8 @@ __global__ void __launch_bounds__(B) k_post(const float* __restrict__ x, const i
     if (!last) return;
     __threadfence();
     double a = 0.0;
-    for (unsigned k = threadIdx.x; k < gridDim.x; k += B) a += __ldcg(part + 3 * (size_t)k);
+#pragma unroll 8
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += B) a += __ldcg(part + 3 * (size_t)k);   // eight reads in flight
     fin[threadIdx.x] = a;
     __syncthreads();
     for (int o = B / 2; o > 0; o >>= 1) {
