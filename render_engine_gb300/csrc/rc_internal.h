@@ -192,6 +192,14 @@ struct EvProgram {
 
 // Launch wrappers (rc_kernels.cu), one instantiation per light count, each compiled in its
 // own translation unit (-DRC_NL_ONE=n) so the build runs in parallel.
+// One chain of reference iterations: the last iterate, the next, the sum of the iterates, the counts
+// of close hits (may be null) and the iteration's seed.
+struct RefChain {
+    const float* Lin;
+    float *Lout, *acc, *closec;
+    uint32_t seed;
+};
+
 template <int NL>
 struct Ops {
     static cudaError_t build(int NW, const DState& s, const DStatic& g, const Grid& grid, const float* L, const float* inten,
@@ -211,8 +219,7 @@ struct Ops {
                              const int* pts, int npts, void* recs, int maxrec, int* nrec, cudaStream_t st);
     // one iteration of the converged-reference solve (scene preparation)
     static cudaError_t ref_iter(const DState& s, const DStatic& g, const Grid& grid, const DevCache& c, const FrameParams& p,
-                                const float* Lin, float* Lout, float* acc, float* closec, uint32_t seed, int K, int accumulate,
-                                int count_close, cudaStream_t st);
+                                const RefChain* chains, int nchains, int K, int accumulate, cudaStream_t st);
     // one taa-mode sample per point (x), with deps the rays' dependency masks or-ed into cur
     static cudaError_t taa_sample(int NW, bool deps, const DState& s, const DStatic& g, const Grid& grid, const DevCache& c,
                                   const FrameParams& p, float* x, uint32_t* cur, uint32_t seed, uint32_t frame, cudaStream_t st);

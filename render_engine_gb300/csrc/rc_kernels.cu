@@ -1941,49 +1941,121 @@ __global__ void __launch_bounds__(BLOCK) k_probe(const DState s, const DStatic g
 // each point averages K rays of albedo x (direct light + the previous iterate) at its hit
 // points; the iterate of every light goes to Lout, and is added to acc from the warm-up on.
 // close counts the rays that hit within 0.02 (points mostly hemmed in are not valid for the
-// error metric).  Buffers are padded like the cache (LCS floats per point).
-template <int NL>
-__global__ void __launch_bounds__(BLOCK) k_ref(const DState s, const DStatic g, const Grid grid, const DevCache c, const FrameParams p,
-                                               const float* __restrict__ Lin, float* __restrict__ Lout, float* __restrict__ acc,
-                                               float* __restrict__ closec, uint32_t seed, int K, int accumulate, int count_close) {
+// error metric).  Buffers are padded like the cache (LCS floats per point).  The first nb blocks are
+// the first chain's, the others the second's.
+// S lanes share a point's rays: lane s draws and traces rays s, s + S, .. (its generator skips the
+// others' draws), and the lanes then add the lights of S rays in ray order, so the iterate does not
+// depend on S.  Bound by the trace's latency and issue, so a launch wants the chip full: the two
+// chains, which do not depend on each other, share it, and S = 8 where they do not fill it alone.  43 k
+// points, 3 lights, 32 rays, an iteration of one chain: 64 us with a launch a chain, 50 with both in one, 33
+// with eight lanes too (full chips take 18 ps a ray with one lane a point, 23 with eight: 1 M points).
+constexpr int REF_LANES = 8;
+constexpr int REF_ROW = 36;   // floats of an exchange row: the lights of four rays in different banks
+// n steps of rnd's generator s -> a s + c
+struct Lcg { uint32_t a, c; };
+__host__ __device__ constexpr Lcg lcg_steps(int n) {
+    Lcg r{1u, 0u};
+    for (int k = 0; k < n; ++k) r = {r.a * 747796405u, r.c * 747796405u + 2891336453u};
+    return r;
+}
+template <int NL, int S>
+__global__ void __launch_bounds__(BLOCK, NL <= 8 ? 4 : 2) k_ref(const DState s, const DStatic g, const Grid grid, const DevCache c, const FrameParams p,
+                                                  const RefChain ch0, const RefChain ch1, int nb, int K, int accumulate) {
     extern __shared__ float4 sm[];
     constexpr int LCS = lcs_of(NL), AES = aes_of(NL);
+    pdl_release();
     stage_smem(sm, s);
     __syncthreads();
+    pdl_wait();
     const TraceSmem tsm = smem_view(sm, s);
-    const int i = blockIdx.x * BLOCK + threadIdx.x;
-    if (i >= p.Np) return;
-    uint32_t rs = hash32(seed ^ hash32(i + 1));
+    const bool second = (int)blockIdx.x >= nb;
+    const RefChain ch = second ? ch1 : ch0;
+    const long long t = (long long)((int)blockIdx.x - (second ? nb : 0)) * BLOCK + threadIdx.x;
+    const int i = (int)(t / S);
+    if (i >= p.Np) return;   // all lanes of a point
+    uint32_t rs = hash32(ch.seed ^ hash32(i + 1));
     const f3 P = xyz(s.P4[i]), N = xyz(s.N4[i]), O = P + N * 1e-3f;
-    float sum[NL];
-#pragma unroll
-    for (int l = 0; l < NL; ++l) sum[l] = 0.f;
     int close = 0;
-    for (int r = 0; r < K; ++r) {
+    // one ray: its factor and summands, 0 where it does not count
+    auto ray = [&](float& A, float (&x)[NL]) {
         const float u1 = rnd(rs);
         const float u2 = rnd(rs);
         const f3 D = cosine_dir(N, u1, u2);
         const Hit h = trace_resolve(tsm, s, g, grid, p, c, O, D, i);
         if (h.q != -1 && h.t < 0.02f) close++;
-        if (h.back) continue;
+        A = 0.f;
+#pragma unroll
+        for (int l = 0; l < NL; ++l) x[l] = 0.f;
+        if (h.back) return;
         float4 ae[AES / 4], lc[LCS / 4];
         const float4* aep = s.AE + (size_t)h.pi * (AES / 4);
-        const float4* lcp = reinterpret_cast<const float4*>(Lin) + (size_t)h.pi * (LCS / 4);
+        const float4* lcp = reinterpret_cast<const float4*>(ch.Lin) + (size_t)h.pi * (LCS / 4);
 #pragma unroll
         for (int k4 = 0; k4 < AES / 4; ++k4) ae[k4] = __ldg(aep + k4);
 #pragma unroll
         for (int k4 = 0; k4 < LCS / 4; ++k4) lc[k4] = __ldcg(lcp + k4);
-        const float A = ae[0].x;
+        A = ae[0].x;
 #pragma unroll
-        for (int l = 0; l < NL; ++l) sum[l] += A * (comp(ae, l + 1) + comp(lc, l));
-    }
+        for (int l = 0; l < NL; ++l) x[l] = comp(ae, l + 1) + comp(lc, l);
+    };
+    auto store = [&](int l, float sum) {
+        const float v = sum / K;
+        ch.Lout[(size_t)LCS * i + l] = v;
+        if (accumulate) ch.acc[(size_t)LCS * i + l] += v;
+    };
+    if (S == 1) {
+        float sum[NL];
 #pragma unroll
-    for (int l = 0; l < NL; ++l) {
-        const float v = sum[l] / K;
-        Lout[(size_t)LCS * i + l] = v;
-        if (accumulate) acc[(size_t)LCS * i + l] += v;
+        for (int l = 0; l < NL; ++l) sum[l] = 0.f;
+        for (int r = 0; r < K; ++r) {
+            float A, x[NL];
+            ray(A, x);
+#pragma unroll
+            for (int l = 0; l < NL; ++l) sum[l] = __fmaf_rn(A, x[l], sum[l]);
+        }
+#pragma unroll
+        for (int l = 0; l < NL; ++l) store(l, sum[l]);
+    } else {
+        __shared__ __align__(16) float ex[BLOCK / 32][NL + 1][REF_ROW];
+        constexpr Lcg one = lcg_steps(2), others = lcg_steps(2 * (S - 1));
+        constexpr int M = (NL + S - 1) / S;
+        const int lane = threadIdx.x & 31, sub = lane % S, first = lane - sub;
+        const unsigned group = ((1u << S) - 1u) << first;
+        float(*w)[REF_ROW] = ex[threadIdx.x >> 5];
+        for (int k = 0; k < sub; ++k) rs = rs * one.a + one.c;
+        float sum[M];
+#pragma unroll
+        for (int m = 0; m < M; ++m) sum[m] = 0.f;
+        for (int r0 = 0; r0 < K; r0 += S) {
+            float A = 0.f, x[NL];
+#pragma unroll
+            for (int l = 0; l < NL; ++l) x[l] = 0.f;
+            if (r0 + sub < K) ray(A, x);
+            rs = rs * others.a + others.c;
+            w[0][lane] = A;
+#pragma unroll
+            for (int l = 0; l < NL; ++l) w[l + 1][lane] = x[l];
+            __syncwarp(group);
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int l = sub + m * S;
+                if (l >= NL) break;
+#pragma unroll
+                for (int q = 0; q < S; q += 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(&w[0][first + q]);
+                    const float4 y = *reinterpret_cast<const float4*>(&w[l + 1][first + q]);
+                    sum[m] = __fmaf_rn(a.w, y.w, __fmaf_rn(a.z, y.z, __fmaf_rn(a.y, y.y, __fmaf_rn(a.x, y.x, sum[m]))));
+                }
+            }
+            __syncwarp(group);
+        }
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+            if (sub + m * S < NL) store(sub + m * S, sum[m]);
+        for (int o = S / 2; o > 0; o >>= 1) close += __shfl_xor_sync(group, close, o);
+        if (sub != 0) return;
     }
-    if (count_close) closec[i] += (float)close;
+    if (ch.closec) ch.closec[i] += (float)close;
 }
 
 // One sample per point of the reference's taa mode (k_taa_pt, poc_gpu.cu:1062-1098): one cosine
@@ -2112,13 +2184,21 @@ cudaError_t Ops<NL>::frozen_hits(const DState& s, const DStatic& g, const Grid& 
 
 template <int NL>
 cudaError_t Ops<NL>::ref_iter(const DState& s, const DStatic& g, const Grid& grid, const DevCache& c, const FrameParams& p,
-                              const float* Lin, float* Lout, float* acc, float* closec, uint32_t seed, int K, int accumulate,
-                              int count_close, cudaStream_t st) {
+                              const RefChain* chains, int nchains, int K, int accumulate, cudaStream_t st) {
     const size_t smem = frame_smem_bytes(s);
-    cudaError_t e = prep_smem(k_ref<NL>, smem);
-    if (e != cudaSuccess) return e;
-    k_ref<NL><<<grid_of(p.Np), BLOCK, smem, st>>>(s, g, grid, c, p, Lin, Lout, acc, closec, seed, K, accumulate, count_close);
-    return cudaGetLastError();
+    cudaError_t e;
+    int resident = 0;
+    if ((e = prep_smem(k_ref<NL, 1>, smem)) != cudaSuccess) return e;
+    if ((e = resident_grid((const void*)k_ref<NL, 1>, smem, resident, BLOCK)) != cudaSuccess) return e;
+    // few points, whose blocks would not fill the chip: eight lanes to each (an iteration of a chain of 32 rays
+    // at 60 k points 45 us, 51 with one lane; at 75 k 56 and 51; on 608 resident blocks the two meet near 67 k),
+    // unless a scene of many dynamic triangles leaves no room for the exchange
+    const bool split = K > 1 && 8ll * nchains * grid_of(p.Np) < 7ll * resident &&
+                       smem + sizeof(float) * (BLOCK / 32) * (NL + 1) * REF_ROW <= 160 * 1024;
+    auto kern = split ? k_ref<NL, REF_LANES> : k_ref<NL, 1>;
+    if (split && (e = prep_smem(kern, smem)) != cudaSuccess) return e;
+    const int nb = (int)(((long long)p.Np * (split ? REF_LANES : 1) + BLOCK - 1) / BLOCK);
+    return launch_dependent(kern, nchains * nb, BLOCK, smem, st, s, g, grid, c, p, chains[0], chains[nchains - 1], nb, K, accumulate);
 }
 
 // Mask widths built for every light count (NW = voxels / 32 of the transit grid).
@@ -2286,7 +2366,8 @@ cudaError_t Ops<NL>::preload(int NW) {
     touch((const void*)k_ray_queue<NL>);
     touch((const void*)k_trace_queue<false>);
     touch((const void*)k_trace_queue<true>);
-    touch((const void*)k_ref<NL>);
+    touch((const void*)k_ref<NL, 1>);
+    touch((const void*)k_ref<NL, REF_LANES>);
     touch((const void*)k_error<NL>);
     touch((const void*)k_proj_apply<NL>);
     touch((const void*)k_camera<NL>);

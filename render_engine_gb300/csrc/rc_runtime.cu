@@ -2126,11 +2126,14 @@ rc_status rc_reference_build(rc_ctx* ctx, const rc_ref_params* prm, double* nois
     std::fill(ctx->taa.have_sums.begin(), ctx->taa.have_sums.end(), (char)0);
     std::vector<DevBuf> tmp;
     struct TmpFree { std::vector<DevBuf>& p; ~TmpFree() { free_pool(p); } } tmp_free{tmp};
-    float *chain[2], *acc[2], *out = nullptr, *closec = nullptr;
+    float *chain[2], *acc[2], *out[2], *closec = nullptr;
     rc_status s;
     for (int ch = 0; ch < 2; ++ch)
         if ((s = dalloc(ctx, tmp, &chain[ch], LCS * Np)) || (s = dalloc(ctx, tmp, &acc[ch], LCS * Np))) return s;
-    if ((s = dalloc(ctx, tmp, &out, LCS * Np)) || (s = dalloc(ctx, tmp, &closec, Np))) return s;
+    if ((s = dalloc(ctx, tmp, &out[0], LCS * Np)) || (s = dalloc(ctx, tmp, &closec, Np))) return s;
+    // the two chains side by side in one launch; one after the other where their second buffer finds no room
+    const bool both = dalloc(ctx, tmp, &out[1], LCS * Np) == RC_OK;
+    if (!both) { cudaGetLastError(); out[1] = out[0]; }
     FrameParams p{};
     p.Np = S.Np;
     auto mix = [](unsigned long long x) {   // poc_gpu.cu:260-262
@@ -2152,20 +2155,22 @@ rc_status rc_reference_build(rc_ctx* ctx, const rc_ref_params* prm, double* nois
         std::vector<uint8_t> val(Np);
         while (true) {
             const int n_it = done == 0 ? prm->warmup + prm->block : prm->block;
-            for (int ch = 0; ch < 2; ++ch) {
-                float* a = chain[ch];
-                float* b = out;
+            for (int ch = 0; ch < 2; ch += both ? 2 : 1) {
+                const int nch = both ? 2 : 1;
                 for (int k = 0; k < n_it; ++k) {
                     const int it = done + k;
-                    const uint32_t seed = (uint32_t)mix(0x51ull + 7919ull * (unsigned long long)si + 104729ull * (unsigned long long)ch +
-                                                        31ull * (unsigned long long)it);
-                    CKR(RC_DISPATCH(NL, ref_iter(d, S.g, S.grid, ctx->c, p, a, b, acc[ch], closec, seed, prm->K, it >= prm->warmup,
-                                                 ch == 0, st)));
-                    std::swap(a, b);
+                    RefChain rc[2];
+                    for (int q = 0; q < nch; ++q) {
+                        const int x = ch + q;
+                        const uint32_t seed = (uint32_t)mix(0x51ull + 7919ull * (unsigned long long)si + 104729ull * (unsigned long long)x +
+                                                            31ull * (unsigned long long)it);
+                        rc[q] = {k & 1 ? out[x] : chain[x], k & 1 ? chain[x] : out[x], acc[x], x == 0 ? closec : nullptr, seed};
+                    }
+                    CKR(RC_DISPATCH(NL, ref_iter(d, S.g, S.grid, ctx->c, p, rc, nch, prm->K, it >= prm->warmup, st)));
                 }
-                if (a != chain[ch]) {   // the last iterate is in `out`: keep it as the chain's state
-                    CKR(cudaMemcpyAsync(chain[ch], a, LCS * Np * 4, cudaMemcpyDeviceToDevice, st));
-                }
+                for (int q = 0; q < nch; ++q)
+                    if (n_it & 1)   // the last iterate is in `out`: keep it as the chain's state
+                        CKR(cudaMemcpyAsync(chain[ch + q], out[ch + q], LCS * Np * 4, cudaMemcpyDeviceToDevice, st));
             }
             done += n_it;
             T = done - prm->warmup;
