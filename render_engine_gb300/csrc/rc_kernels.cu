@@ -418,7 +418,10 @@ __device__ __forceinline__ bool trace_boxes(const TraceSmem& sm, const DState& s
 // lanes that reached the call together): each tests every popc(act)-th triangle, and the smallest
 // distance, then the smallest index at that distance, is the scan's answer.  One such ray costs its
 // warp about 200 instructions; on its own lane, through the plane filter, it made the warp the
-// last of a small frame by 8 us (10,728 points: 20 us instead of 12).
+// last of a small frame by 8 us (10,728 points: 20 us instead of 12).  From more than SCAN_LANES such lanes on
+// (rows of points inside or behind a wall) each scans for itself: a room whose walls stand through its
+// enclosing box, 1,082,802 points: 75 us a fused frame one by one, 70 at 4, 68 at 8 and at 14.
+constexpr int SCAN_LANES = 14;
 static __device__ __forceinline__ float2 scan_lanes(const float4* __restrict__ tri, int nt, unsigned act, unsigned need, f3 o, f3 d, float tmin,
                                                  int q) {
     const unsigned lane = threadIdx.x & 31u;
@@ -441,8 +444,10 @@ static __device__ __forceinline__ float2 scan_lanes(const float4* __restrict__ t
     return make_float2(tmin, __int_as_float(q));
 }
 
-// The plane filter over all groups, and the triangles outside any.
-static __device__ __forceinline__ float2 trace_filter(const float4* tri, const float4* grp, const int* misc, int ng, int nmisc, GroupRanges gr,
+// The plane filter over all groups, and the triangles outside any.  Not inlined: beside trace_boxes in
+// one kernel it spilt in its loops (a room with a turned door, 1,082,802 points: 94 us a fused frame, 83 as
+// a call; the box states' tracked frames pay 2 us for it).
+static __device__ __noinline__ float2 trace_filter(const float4* tri, const float4* grp, const int* misc, int ng, int nmisc, GroupRanges gr,
                                                    f3 o, f3 d) {
     float tmin = __int_as_float(0x7f800000);
     int q = -1, jb = 0x7fffffff;
@@ -462,8 +467,9 @@ __device__ __forceinline__ void trace_dyn(const TraceSmem& sm, const DState& s, 
     tmin = __int_as_float(0x7f800000);
     q = -1;
     if (brute || s.ng == 0) {
+        const float4* tri = s.nbox >= 0 ? s.tri : sm.tri;
         int jb = 0x7fffffff;
-        for (int j = 0; j < s.nt; ++j) mt_tri(sm.tri, j, o, d, tmin, q, jb);
+        for (int j = 0; j < s.nt; ++j) mt_tri(tri, j, o, d, tmin, q, jb);
         return;
     }
     float2 r;
@@ -472,6 +478,15 @@ __device__ __forceinline__ void trace_dyn(const TraceSmem& sm, const DState& s, 
         const unsigned act = __activemask();
         const unsigned need = __ballot_sync(act, !ok);
         if (need == 0u) return;
+        if (__popc(need) > SCAN_LANES) {   // many lanes (points in or behind a wall): each its own scan
+            if (!ok) {
+                int jb = 0x7fffffff;
+                tmin = __int_as_float(0x7f800000);
+                q = -1;
+                for (int j = 0; j < s.nt; ++j) mt_tri(s.tri, j, o, d, tmin, q, jb);
+            }
+            return;
+        }
         r = scan_lanes(s.tri, s.nt, act, need, o, d, tmin, q);
     } else {
         r = trace_filter(sm.tri, sm.grp, sm.misc, s.ng, s.nmisc, s.gr, o, d);
@@ -777,18 +792,13 @@ __device__ __forceinline__ TraceSmem smem_view(float4* sm, const DState& s) {
     TraceSmem t;
     const int nt = staged_tri(s), nr = staged_rec(s);
     t.quad = sm + (nr - 2 * s.nquad);
-    if (s.nbox >= 0) {
-        t.box = sm;
-        t.rect = sm + box_float4s(s);
-        t.grp = s.grp;
-        t.tri = s.tri;
-        t.misc = s.misc;
-    } else {
-        t.box = t.rect = nullptr;
-        t.grp = sm;
-        t.tri = sm + nr;
-        t.misc = (const int*)(sm + nr + nt);
-    }
+    // where each is staged (build_boxes: either the boxes and rectangles, or the groups and triangles);
+    // plain offsets, so that the compiler sees shared memory on both paths
+    t.box = sm;
+    t.rect = sm + box_float4s(s);
+    t.grp = sm;
+    t.tri = sm + nr;
+    t.misc = (const int*)(sm + nr + nt);
     return t;
 }
 
