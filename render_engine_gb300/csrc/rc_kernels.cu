@@ -1744,7 +1744,8 @@ __device__ __forceinline__ float shadow_t(const TraceSmem& sm, const DState& s, 
     return q == -1 ? INFINITY : t;
 }
 
-// Four blocks an SM (64 registers; 52 bytes spilt at 3 lights): a 1080p pass of two bounces 1410 us with three, 1380.
+// Four blocks an SM (64 registers; 52 bytes spilt at 3 lights): a 1080p pass of two bounces 1410 us with three,
+// 1380 with four; 1456 since the plane filter is a call, which the two traces of a vertex pay for.
 template <int NL>
 __global__ void __launch_bounds__(BLOCK, 4) k_paths(const DState s, const DStatic g, const Grid grid, const DevCache c, const FrameParams p,
                                                  const CameraD cam, const PathD pd, float* __restrict__ pos, float* __restrict__ nrm,
