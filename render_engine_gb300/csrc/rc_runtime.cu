@@ -1632,8 +1632,9 @@ rc_status rc_scene_load_memory(rc_ctx* ctx, const void* data, size_t nbytes) {
     free_pool(ctx->adj_bufs);
     free_pool(ctx->taa_bufs);
     ctx->taa = TaaRun{};
+    ctx->adj = adj::Bufs{};
     ctx->adj_np = ctx->adj_k = 0;
-    ctx->adj_cap_np = ctx->adj_cap_k = ctx->adj_cap_nl = 0;
+    ctx->adj_cap_np = ctx->adj_cap_k = ctx->adj_cap_nl = ctx->adj_cap_it = 0;
     ctx->have_scene = false;
     ctx->run.active = false;
     ctx->c = DevCache{};
@@ -2225,28 +2226,38 @@ rc_status rc_adjoint(rc_ctx* ctx, const rc_adjoint_params* prm, const float* wei
     if (prm->state < 0 || prm->state >= S.NS) return fail(ctx, RC_ERR_ARG, "state %d out of range", prm->state);
     if ((long long)S.Np * prm->K >= (1ll << 31)) return fail(ctx, RC_ERR_ARG, "Np * K must stay below 2^31");
     if (S.NL + 1 > adj::MAX_COLS) return fail(ctx, RC_ERR_UNSUPPORTED, "%d lights", S.NL);
+    const int NL = S.NL;
+    // the emissions of the forward solve: the state's, or the caller's (looked at before the last
+    // call's results and buffers are touched)
+    std::vector<float> E = S.st[prm->state].inten;
+    if (prm->emission)
+        for (int l = 0; l < NL; ++l) {
+            if (!std::isfinite(prm->emission[l])) return fail(ctx, RC_ERR_ARG, "emission %d not finite", l);
+            E[l] = prm->emission[l];
+        }
     CKR(cudaSetDevice(ctx->cfg.device));
     if (rc_status es = ensure_state(ctx, prm->state)) return es;
     cudaStream_t st = ctx->stream;
     const size_t Np = (size_t)S.Np, K = (size_t)prm->K;
-    const int NL = S.NL, AES = aes_of(NL), iters = prm->iterations ? prm->iterations : 64;
-    adj::Bufs b = ctx->adj;
+    const int AES = aes_of(NL), iters = prm->iterations ? prm->iterations : 64;
     rc_status s;
-    // buffers kept from call to call while the point count, K and the light count stay
+    ctx->adj_np = ctx->adj_k = 0;   // no results until this call has its own
+    // Buffers kept from call to call while the point count, K and the light count stay and the
+    // iterations fit.  ctx->adj and the capacities are set together, when every buffer is there: a call that
+    // ends early in between leaves neither behind.
     if (ctx->adj_cap_np != S.Np || ctx->adj_cap_k != prm->K || ctx->adj_cap_nl != NL || ctx->adj_cap_it < iters) {
         CKR(cudaStreamSynchronize(st));
         free_pool(ctx->adj_bufs);
-        ctx->adj_np = ctx->adj_k = 0;
-        ctx->adj_cap_np = ctx->adj_cap_k = ctx->adj_cap_nl = 0;
+        ctx->adj = adj::Bufs{};
+        ctx->adj_cap_np = ctx->adj_cap_k = ctx->adj_cap_nl = ctx->adj_cap_it = 0;
         auto& pool = ctx->adj_bufs;
         const int cap_it = std::max(iters, 64);
         if (ctx->adj_counts) cudaFreeHost(ctx->adj_counts);
         ctx->adj_counts = nullptr;
-        ctx->adj_cap_it = 0;
         CKR(cudaMallocHost(&ctx->adj_counts, 2 * sizeof(unsigned) * (size_t)cap_it));
         for (cudaEvent_t& e : ctx->adj_seen)
             if (!e) CKR(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        b = adj::Bufs{};
+        adj::Bufs b{};
         b.host_counts = ctx->adj_counts;
         b.seen[0] = ctx->adj_seen[0];
         b.seen[1] = ctx->adj_seen[1];
@@ -2266,6 +2277,7 @@ rc_status rc_adjoint(rc_ctx* ctx, const rc_adjoint_params* prm, const float* wei
             (s = dalloc(ctx, pool, &b.part, (size_t)adj::GRAD_BLOCKS * (NL + 1))) || (s = dalloc(ctx, pool, &b.stats, 1)) ||
             (s = dalloc(ctx, pool, &AEu, (size_t)AES / 4 * Np)) || (s = dput(ctx, pool, &ones, std::vector<float>((size_t)NL, 1.f))))
             return s;
+        ctx->adj = b;
         ctx->adj_aeu = AEu;
         ctx->adj_aeu_state = -1;
         ctx->adj_ones = ones;
@@ -2274,6 +2286,7 @@ rc_status rc_adjoint(rc_ctx* ctx, const rc_adjoint_params* prm, const float* wei
         ctx->adj_cap_nl = NL;
         ctx->adj_cap_it = cap_it;
     }
+    adj::Bufs& b = ctx->adj;
     float4* AEu = ctx->adj_aeu;
     const float* ones = ctx->adj_ones;
     const DState& d = S.st[prm->state].d;
@@ -2290,18 +2303,10 @@ rc_status rc_adjoint(rc_ctx* ctx, const rc_adjoint_params* prm, const float* wei
         launched = 1;
     }
     CKR(adj::build_transpose(b, S.Np, prm->K, st));
-    // the emissions of the forward solve: the state's, or the caller's
-    std::vector<float> E = S.st[prm->state].inten;
     std::vector<DevBuf> tmp;
     struct TmpFree { std::vector<DevBuf>& p; ~TmpFree() { free_pool(p); } } tmp_free{tmp};
     const float* dem = nullptr;
-    if (prm->emission) {
-        for (int l = 0; l < NL; ++l) {
-            if (!std::isfinite(prm->emission[l])) return fail(ctx, RC_ERR_ARG, "emission %d not finite", l);
-            E[l] = prm->emission[l];
-        }
-        if ((s = dput(ctx, tmp, &dem, E))) return s;
-    }
+    if (prm->emission && (s = dput(ctx, tmp, &dem, E))) return s;
     CKR(adj::solve(&b, S.Np, prm->K, NL, AES, reinterpret_cast<const float*>(d.AE), reinterpret_cast<const float*>(AEu), dem, iters,
                    st));
     adj::Stats hs{};
@@ -2323,7 +2328,6 @@ rc_status rc_adjoint(rc_ctx* ctx, const rc_adjoint_params* prm, const float* wei
         res->back = (long long)hs.back;
         res->max_incoming = hs.max_incoming;
     }
-    ctx->adj = b;
     ctx->adj_np = S.Np;
     ctx->adj_k = prm->K;
     return RC_OK;
