@@ -562,8 +562,15 @@ void build_boxes(const std::vector<PlaneGroup>& gs, const std::vector<float>& T,
         float w0, w1;
         memcpy(&w0, &v[0], 4);
         memcpy(&w1, &v[1], 4);
-        out.grp.push_back(make_float4(x.lo[0], x.hi[0], x.lo[1], x.hi[1]));
-        out.grp.push_back(make_float4(x.lo[2], x.hi[2], w0, w1));
+        // A side's plane is its own triangles', not the corner sums of its neighbours: one rounding between
+        // the two (3e-8) moves the crossing of a ray that grazes the plane by that over its slope, past the margin.
+        float lo[3], hi[3];
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = x.face[2 * k] >= 0 ? gs[x.face[2 * k]].c : x.lo[k];
+            hi[k] = x.face[2 * k + 1] >= 0 ? gs[x.face[2 * k + 1]].c : x.hi[k];
+        }
+        out.grp.push_back(make_float4(lo[0], hi[0], lo[1], hi[1]));
+        out.grp.push_back(make_float4(lo[2], hi[2], w0, w1));
     };
     Box empty{};
     for (int f = 0; f < 6; ++f) empty.face[f] = -1;
