@@ -2149,9 +2149,11 @@ __global__ void __launch_bounds__(BLOCK) k_frozen(const DState s, const DStatic 
 
 static int grid_of(int Np) { return (Np + BLOCK - 1) / BLOCK; }
 
+// Dynamic shared memory beyond the 48 KB that a launch may have unasked, which count the kernel's static
+// shared memory too (`fixed`; 1 KB covers the kernels that keep a few reduction words).
 template <typename K>
-static cudaError_t prep_smem(K kern, size_t smem) {
-    if (smem > 48 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+static cudaError_t prep_smem(K kern, size_t smem, size_t fixed = 1024) {
+    if (smem + fixed > 48 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return cudaSuccess;
 }
 
@@ -2204,10 +2206,10 @@ cudaError_t Ops<NL>::ref_iter(const DState& s, const DStatic& g, const Grid& gri
     // few points, whose blocks would not fill the chip: eight lanes to each (an iteration of a chain of 32 rays
     // at 60 k points 45 us, 51 with one lane; at 75 k 56 and 51; on 608 resident blocks the two meet near 67 k),
     // unless a scene of many dynamic triangles leaves no room for the exchange
-    const bool split = K > 1 && 8ll * nchains * grid_of(p.Np) < 7ll * resident &&
-                       smem + sizeof(float) * (BLOCK / 32) * (NL + 1) * REF_ROW <= 160 * 1024;
+    constexpr size_t exchange = sizeof(float) * (BLOCK / 32) * (NL + 1) * REF_ROW;
+    const bool split = K > 1 && 8ll * nchains * grid_of(p.Np) < 7ll * resident && smem + exchange <= 160 * 1024;
     auto kern = split ? k_ref<NL, REF_LANES> : k_ref<NL, 1>;
-    if (split && (e = prep_smem(kern, smem)) != cudaSuccess) return e;
+    if (split && (e = prep_smem(kern, smem, exchange)) != cudaSuccess) return e;
     const int nb = (int)(((long long)p.Np * (split ? REF_LANES : 1) + BLOCK - 1) / BLOCK);
     return launch_dependent(kern, nchains * nb, BLOCK, smem, st, s, g, grid, c, p, chains[0], chains[nchains - 1], nb, K, accumulate);
 }
