@@ -266,13 +266,8 @@ __host__ __device__ inline int box_float4s(const DState& s) {
 __host__ __device__ inline int grp_float4s(const DState& s) {
     return 3 * s.ng + 3 * (s.ng / 2) + box_float4s(s) + (s.nbox < 0 ? 0 : 3 * s.ng) + 2 * s.nquad;
 }
-// What a block stages of it (stage_smem), and the triangles beside it.
-__host__ __device__ inline int staged_rec(const DState& s) {
-    return s.nbox < 0 ? grp_float4s(s) : box_float4s(s) + 3 * s.ng + 2 * s.nquad;
-}
-__host__ __device__ inline int staged_tri(const DState& s) { return s.nbox < 0 ? 3 * s.nt : 0; }
-__host__ __device__ inline size_t frame_smem_bytes(const DState& s) {
-    return sizeof(float4) * (size_t)(staged_rec(s) + staged_tri(s)) + (s.nbox < 0 ? sizeof(int) * (size_t)s.nmisc : 0) + 16;
+__host__ __device__ inline size_t frame_smem_bytes(const DState& s) {   // what a block stages (stage_smem)
+    return sizeof(float4) * (3 * (size_t)s.nt + (size_t)grp_float4s(s)) + sizeof(int) * (size_t)s.nmisc + 16;
 }
 __host__ __device__ constexpr int lcs_of(int NL) { return (NL + 3) / 4 * 4; }
 __host__ __device__ constexpr int aes_of(int NL) { return (NL + 1 + 3) / 4 * 4; }

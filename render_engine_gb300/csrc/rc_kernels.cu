@@ -419,9 +419,11 @@ __device__ __forceinline__ bool trace_boxes(const TraceSmem& sm, const DState& s
 // distance, then the smallest index at that distance, is the scan's answer.  One such ray costs its
 // warp about 200 instructions; on its own lane, through the plane filter, it made the warp the
 // last of a small frame by 8 us (10,728 points: 20 us instead of 12).  From more than SCAN_LANES such lanes on
-// (rows of points inside or behind a wall) each scans for itself: a room whose walls stand through its
-// enclosing box, 1,082,802 points: 75 us a fused frame one by one, 70 at 4, 68 at 8 and at 14.
-constexpr int SCAN_LANES = 14;
+// (rows of points inside, behind or close beside a wall, cameras outside the room) each goes through the plane
+// filter.  20 frames of a room whose walls stand through its enclosing box, 1,082,802 points: 1174 us; 1355
+// when the triangles came from the L2 and more than 14 lanes scanned each for itself; 1430 with the plane filter
+// alone.  A room of 0.8 x 0.4 x 0.3, 200,000 points: 334, 619 and 425.
+constexpr int SCAN_LANES = 8;
 static __device__ __forceinline__ float2 scan_lanes(const float4* __restrict__ tri, int nt, unsigned act, unsigned need, f3 o, f3 d, float tmin,
                                                  int q) {
     const unsigned lane = threadIdx.x & 31u;
@@ -446,7 +448,8 @@ static __device__ __forceinline__ float2 scan_lanes(const float4* __restrict__ t
 
 // The plane filter over all groups, and the triangles outside any.  Not inlined: beside trace_boxes in
 // one kernel it spilt in its loops (a room with a turned door, 1,082,802 points: 94 us a fused frame, 83 as
-// a call; the box states' tracked frames pay 2 us for it).
+// a call; the box states' tracked frames pay 2 us for it).  One call site, on what the block has staged: a second
+// one, for box states on the triangles in global memory, cost 3 % of every frame, pointers to either 12 %.
 static __device__ __noinline__ float2 trace_filter(const float4* tri, const float4* grp, const int* misc, int ng, int nmisc, GroupRanges gr,
                                                    f3 o, f3 d) {
     float tmin = __int_as_float(0x7f800000);
@@ -459,7 +462,7 @@ static __device__ __noinline__ float2 trace_filter(const float4* tri, const floa
 
 // Closest dynamic-triangle hit, equal to the reference's in-order scan (poc_gpu.cu:199-220).
 // States made of boxes go through trace_boxes, and the few rays that it cannot decide through the
-// scan itself.  The plane filter takes other states: pass 1 marks the groups whose plane crossing
+// scan itself.  The plane filter takes other states, and warps with many undecided rays: pass 1 marks the groups whose plane crossing
 // falls in their outer box; pass 2 visits the marked groups nearest first, runs the exact
 // Möller-Trumbore on their triangles, and stops once the next crossing lies beyond the best exact
 // hit by more than the filter's error.
@@ -467,9 +470,8 @@ __device__ __forceinline__ void trace_dyn(const TraceSmem& sm, const DState& s, 
     tmin = __int_as_float(0x7f800000);
     q = -1;
     if (brute || s.ng == 0) {
-        const float4* tri = s.nbox >= 0 ? s.tri : sm.tri;
         int jb = 0x7fffffff;
-        for (int j = 0; j < s.nt; ++j) mt_tri(tri, j, o, d, tmin, q, jb);
+        for (int j = 0; j < s.nt; ++j) mt_tri(sm.tri, j, o, d, tmin, q, jb);
         return;
     }
     float2 r;
@@ -478,19 +480,15 @@ __device__ __forceinline__ void trace_dyn(const TraceSmem& sm, const DState& s, 
         const unsigned act = __activemask();
         const unsigned need = __ballot_sync(act, !ok);
         if (need == 0u) return;
-        if (__popc(need) > SCAN_LANES) {   // many lanes (points in or behind a wall): each its own scan
-            if (!ok) {
-                int jb = 0x7fffffff;
-                tmin = __int_as_float(0x7f800000);
-                q = -1;
-                for (int j = 0; j < s.nt; ++j) mt_tri(s.tri, j, o, d, tmin, q, jb);
-            }
+        if (__popc(need) <= SCAN_LANES) {
+            r = scan_lanes(sm.tri, s.nt, act, need, o, d, tmin, q);
+            tmin = r.x;
+            q = __float_as_int(r.y);
             return;
         }
-        r = scan_lanes(s.tri, s.nt, act, need, o, d, tmin, q);
-    } else {
-        r = trace_filter(sm.tri, sm.grp, sm.misc, s.ng, s.nmisc, s.gr, o, d);
+        if (ok) return;
     }
+    r = trace_filter(sm.tri, sm.grp, sm.misc, s.ng, s.nmisc, s.gr, o, d);
     tmin = r.x;
     q = __float_as_int(r.y);
 }
@@ -777,26 +775,24 @@ __device__ __forceinline__ Hit trace_resolve(const TraceSmem& sm, const DState& 
     return h;
 }
 
-// What the trace reads of a state's geometry goes to shared memory once per block: with boxes their
-// records alone (the full scan takes few rays and reads the triangles through L1), otherwise the triangles, the groups and the triangles outside any; the quad records with both.
+// What the trace reads of a state's geometry goes to shared memory once per block: the group buffer,
+// the triangles and the triangles outside any group.  (Box states need groups and triangles for undecided rays
+// only; 5 KB of a 31-rectangle room.  They cost 8 lights' frames 3 %, in L1 capacity, and 3 lights' 1 %; without them the
+// undecided rays' loads wait for the L2, see SCAN_LANES.)
 __device__ __forceinline__ void stage_smem(float4* sm, const DState& s) {
-    const int nt = staged_tri(s), nr = staged_rec(s);
-    const float4* rec = s.grp + (grp_float4s(s) - nr);
-    for (int j = threadIdx.x; j < nr; j += blockDim.x) sm[j] = rec[j];
+    const int nt = 3 * s.nt, nr = grp_float4s(s);
+    for (int j = threadIdx.x; j < nr; j += blockDim.x) sm[j] = s.grp[j];
     for (int j = threadIdx.x; j < nt; j += blockDim.x) sm[nr + j] = s.tri[j];
     int* smi = (int*)(sm + nr + nt);
-    if (s.nbox < 0)
-        for (int j = threadIdx.x; j < s.nmisc; j += blockDim.x) smi[j] = s.misc[j];
+    for (int j = threadIdx.x; j < s.nmisc; j += blockDim.x) smi[j] = s.misc[j];
 }
 __device__ __forceinline__ TraceSmem smem_view(float4* sm, const DState& s) {
     TraceSmem t;
-    const int nt = staged_tri(s), nr = staged_rec(s);
-    t.quad = sm + (nr - 2 * s.nquad);
-    // where each is staged (build_boxes: either the boxes and rectangles, or the groups and triangles);
-    // plain offsets, so that the compiler sees shared memory on both paths
-    t.box = sm;
-    t.rect = sm + box_float4s(s);
+    const int nt = 3 * s.nt, nr = grp_float4s(s);
     t.grp = sm;
+    t.box = sm + 3 * s.ng + 3 * (s.ng / 2);
+    t.rect = t.box + box_float4s(s);
+    t.quad = sm + (nr - 2 * s.nquad);
     t.tri = sm + nr;
     t.misc = (const int*)(sm + nr + nt);
     return t;
@@ -2073,8 +2069,9 @@ __global__ void __launch_bounds__(BLOCK, NL <= 8 ? 4 : 2) k_ref(const DState s, 
 // ray; the radiance at its hit point = A x (direct light summed over lights + the converged
 // reference), 0 when the ray does not count; with DEPS the ray's dependency mask (the hit's
 // shadow voxels and the ray's own transit voxels) is or-ed into cur.
+// Five blocks an SM (48 registers): 24 frames of 1,082,802 points 2348 us, 2402 with four.
 template <int NL, int NW, bool DEPS>
-__global__ void __launch_bounds__(BLOCK) k_taa_pt(const DState s, const DStatic g, const Grid grid, const DevCache c, const FrameParams p,
+__global__ void __launch_bounds__(BLOCK, 5) k_taa_pt(const DState s, const DStatic g, const Grid grid, const DevCache c, const FrameParams p,
                                                   float* __restrict__ x, uint32_t* __restrict__ cur, uint32_t seed, uint32_t frame) {
     extern __shared__ float4 sm[];
     stage_smem(sm, s);
