@@ -414,6 +414,11 @@ void build_boxes(const std::vector<PlaneGroup>& gs, const std::vector<float>& T,
         full(g, lo, hi);
         for (int k = 0; k < 3; ++k) scale = std::max(scale, std::max(fabsf(lo[k]), fabsf(hi[k])));
     }
+    // Rays start 1e-3 off their surface: where the margin nears that, no origin would be certain to lie
+    // outside its own wall, and every ray would go to the undecided ones' path (a room of 800 m: 1151 us for 20
+    // frames of 200,000 points, 375 with the plane filter).
+    const float m = 1e-5f + 2e-6f * scale;
+    if (!(m <= 5e-4f)) return;
     const float tol = 1e-6f * scale;
     auto same = [&](float a, float b) { return fabsf(a - b) <= tol; };
     // sides of box b among the unused groups (face[2 k + side])
@@ -495,7 +500,6 @@ void build_boxes(const std::vector<PlaneGroup>& gs, const std::vector<float>& T,
         boxes.push_back(f);
     }
     if (boxes.size() > (size_t)n / 2 || boxes.size() > (size_t)MAX_BOXES || !out.misc.empty()) return;
-    const float m = 1e-5f + 2e-6f * scale;
     out.nbox = ((int)boxes.size() + 1) / 2 * 2;
     out.outer = have_outer ? 1 : 0;
     out.box_scale = 4.f * scale;

@@ -64,3 +64,8 @@ def _compare(scale):
 def test_rows_of_undecided_rays():
     """A room of 0.8 x 0.4 x 0.3: its points lie 2 mm apart, and whole rows of them beside the boxes' edges."""
     _compare(0.1)
+
+
+def test_large_units():
+    """A room of 800 x 400 x 300: the slabs' margin passes the 1e-3 that rays start off their surface."""
+    _compare(100.0)
