@@ -399,20 +399,22 @@ struct PlaneGroup { int axis, j0, cnt; float c, lo[2], hi[2]; float line[4]; };
 void build_boxes(const std::vector<PlaneGroup>& gs, const std::vector<float>& T, const std::vector<int>& TQ, float scene_scale,
                  Groups& out) {
     struct Box { float lo[3], hi[3]; int face[6]; bool flat; };
+    struct Rect { float lo[3], hi[3]; };
+    if (!out.misc.empty()) return;
     const int n = (int)gs.size();
     float scale = scene_scale;
-    auto ax = [](int k, int u) { return u == 0 ? (k == 0 ? 1 : 0) : (k == 2 ? 1 : 2); };
-    auto full = [&](int g, float lo[3], float hi[3]) {   // the rectangle as a box of no thickness
-        const int k = gs[g].axis;
-        lo[k] = hi[k] = gs[g].c;
-        for (int u = 0; u < 2; ++u) { lo[ax(k, u)] = gs[g].lo[u]; hi[ax(k, u)] = gs[g].hi[u]; }
-    };
     std::vector<char> used(n, 0);
+    std::vector<Rect> rc(n);   // the groups' rectangles as boxes of no thickness
     for (int g = 0; g < n; ++g) {
         if (gs[g].cnt == 0) { used[g] = 1; continue; }   // padding
-        float lo[3], hi[3];
-        full(g, lo, hi);
-        for (int k = 0; k < 3; ++k) scale = std::max(scale, std::max(fabsf(lo[k]), fabsf(hi[k])));
+        const int k = gs[g].axis;
+        rc[g].lo[k] = rc[g].hi[k] = gs[g].c;
+        for (int u = 0; u < 2; ++u) {
+            const int a = u == 0 ? (k == 0 ? 1 : 0) : (k == 2 ? 1 : 2);
+            rc[g].lo[a] = gs[g].lo[u];
+            rc[g].hi[a] = gs[g].hi[u];
+        }
+        for (int a = 0; a < 3; ++a) scale = std::max(scale, std::max(fabsf(rc[g].lo[a]), fabsf(rc[g].hi[a])));
     }
     // Rays start 1e-3 off their surface: where the margin nears that, no origin would be certain to lie
     // outside its own wall, and every ray would go to the undecided ones' path (a room of 800 m: 1151 us for 20
@@ -421,54 +423,95 @@ void build_boxes(const std::vector<PlaneGroup>& gs, const std::vector<float>& T,
     if (!(m <= 5e-4f)) return;
     const float tol = 1e-6f * scale;
     auto same = [&](float a, float b) { return fabsf(a - b) <= tol; };
-    // sides of box b among the unused groups (face[2 k + side])
-    auto sides = [&](Box& b) {
+    auto equal = [](const Rect& a, const Rect& b) {
+        return a.lo[0] == b.lo[0] && a.hi[0] == b.hi[0] && a.lo[1] == b.lo[1] && a.hi[1] == b.hi[1] && a.lo[2] == b.lo[2] && a.hi[2] == b.hi[2];
+    };
+    // The boxes that two groups of different axes span with a common edge, each with the groups that
+    // are sides of it (in their order; face[2 k + side]): found once, while the choice below
+    // goes over the pairs again and again (9 boxes in a room, 56 groups: 107 us a state when each turn compared
+    // all groups anew, 14 us).
+    struct Side { int g, f; };
+    struct Span { Rect b; double vol; int s0, s1, found, turn; };   // its sides are side[s0 .. s1)
+    struct Pair { int x, y, span; };
+    std::vector<Span> spans;
+    std::vector<Pair> pairs;
+    std::vector<Side> side;
+    spans.reserve(64);
+    pairs.reserve(256);
+    side.reserve(256);
+    const GroupRanges& gr = out.gr;   // the groups are in the order of their axes
+    for (int x = 0; x < gr.g0[2]; ++x) {
+        if (used[x]) continue;
+        const Rect p = rc[x];
+        const int kx = gs[x].axis;
+        for (int y = gr.g0[kx + 1]; y < n; ++y) {
+            const int ky = gs[y].axis, kz = 3 - kx - ky;
+            const Rect& q = rc[y];
+            if (used[y]) continue;
+            if (!same(p.lo[kz], q.lo[kz]) || !same(p.hi[kz], q.hi[kz])) continue;
+            if (!(same(p.lo[kx], q.lo[kx]) || same(p.lo[kx], q.hi[kx])) || !(same(q.lo[ky], p.lo[ky]) || same(q.lo[ky], p.hi[ky]))) continue;
+            Rect b;
+            for (int a = 0; a < 3; ++a) { b.lo[a] = std::min(p.lo[a], q.lo[a]); b.hi[a] = std::max(p.hi[a], q.hi[a]); }
+            int at = 0;
+            while (at < (int)spans.size() && !equal(spans[at].b, b)) ++at;
+            if (at == (int)spans.size()) {
+                const int s0 = (int)side.size();
+                for (int k = 0; k < 3; ++k) {
+                    const int u = k == 0 ? 1 : 0, v = k == 2 ? 1 : 2;
+                    for (int g = gr.g0[k]; g < gr.g0[k + 1]; ++g) {
+                        const Rect& r = rc[g];
+                        const bool low = same(r.lo[k], b.lo[k]);
+                        if (!(low || same(r.lo[k], b.hi[k])) || used[g]) continue;
+                        if (same(r.lo[u], b.lo[u]) && same(r.hi[u], b.hi[u]) && same(r.lo[v], b.lo[v]) && same(r.hi[v], b.hi[v]))
+                            side.push_back({g, 2 * k + (low ? 0 : 1)});
+                    }
+                }
+                spans.push_back({b, (double)(b.hi[0] - b.lo[0]) * (b.hi[1] - b.lo[1]) * (b.hi[2] - b.lo[2]), s0, (int)side.size(), 0, -1});
+            }
+            pairs.push_back({x, y, at});
+        }
+    }
+    // the sides of a span among the unused groups
+    auto sides = [&](const Span& sp, Box& b) {
         int found = 0;
         for (int f = 0; f < 6; ++f) b.face[f] = -1;
-        for (int g = 0; g < n; ++g) {
-            if (used[g]) continue;
-            float lo[3], hi[3];
-            full(g, lo, hi);
-            const int k = gs[g].axis;
-            bool fit = true;
-            for (int a = 0; a < 3; ++a)
-                if (a != k) fit = fit && same(lo[a], b.lo[a]) && same(hi[a], b.hi[a]);
-            if (!fit) continue;
-            const int f = same(lo[k], b.lo[k]) ? 2 * k : (same(lo[k], b.hi[k]) ? 2 * k + 1 : -1);
-            if (f < 0 || b.face[f] >= 0) continue;
-            b.face[f] = g;
-            ++found;
-        }
+        for (int q = sp.s0; q < sp.s1; ++q)
+            if (!used[side[q].g] && b.face[side[q].f] < 0) {
+                b.face[side[q].f] = side[q].g;
+                ++found;
+            }
         return found;
     };
     // the best box that two unused groups of different axes span
+    int turn = 0;
     auto best = [&](bool enclosing, Box& res) {
-        int most = 1;
+        int most = 1, pick = -1;
         double vol = -1.0;
-        for (int x = 0; x < n; ++x)
-            for (int y = x + 1; y < n; ++y) {
-                if (used[x] || used[y] || gs[x].axis == gs[y].axis) continue;
+        for (const Pair& pr : pairs) {
+            if (used[pr.x] || used[pr.y]) continue;
+            Span& sp = spans[pr.span];
+            if (sp.turn != turn) {
                 Box b{};
-                float l0[3], h0[3], l1[3], h1[3];
-                full(x, l0, h0);
-                full(y, l1, h1);
-                const int kx = gs[x].axis, ky = gs[y].axis, kz = 3 - kx - ky;
-                if (!same(l0[kz], l1[kz]) || !same(h0[kz], h1[kz])) continue;
-                if (!(same(l0[kx], l1[kx]) || same(l0[kx], h1[kx])) || !(same(l1[ky], l0[ky]) || same(l1[ky], h0[ky]))) continue;
-                for (int a = 0; a < 3; ++a) { b.lo[a] = std::min(l0[a], l1[a]); b.hi[a] = std::max(h0[a], h1[a]); }
-                const int f = sides(b);
-                const double v = (double)(b.hi[0] - b.lo[0]) * (b.hi[1] - b.lo[1]) * (b.hi[2] - b.lo[2]);
-                if (enclosing ? (f == 6 && v > vol) : (f > most || (f == most && v > vol && f > 1))) {
-                    most = f;
-                    vol = v;
-                    res = b;
-                }
+                sp.found = sides(sp, b);
+                sp.turn = turn;
             }
-        return enclosing ? vol > 0.0 : most > 1;
+            const int f = sp.found;
+            if (enclosing ? (f == 6 && sp.vol > vol) : (f > most || (f == most && sp.vol > vol && f > 1))) {
+                most = f;
+                vol = sp.vol;
+                pick = pr.span;
+            }
+        }
+        if (enclosing ? !(vol > 0.0) : most <= 1) return false;
+        memcpy(res.lo, spans[pick].b.lo, sizeof res.lo);
+        memcpy(res.hi, spans[pick].b.hi, sizeof res.hi);
+        sides(spans[pick], res);
+        return true;
     };
     auto take = [&](const Box& b) {
         for (int f = 0; f < 6; ++f)
             if (b.face[f] >= 0) used[b.face[f]] = 1;
+        ++turn;
     };
     Box outer{};
     bool have_outer = best(true, outer);
@@ -493,13 +536,14 @@ void build_boxes(const std::vector<PlaneGroup>& gs, const std::vector<float>& T,
     for (int g = 0; g < n; ++g) {
         if (used[g]) continue;
         Box f{};
-        full(g, f.lo, f.hi);
+        memcpy(f.lo, rc[g].lo, sizeof f.lo);
+        memcpy(f.hi, rc[g].hi, sizeof f.hi);
         for (int k = 0; k < 6; ++k) f.face[k] = -1;
         f.face[2 * gs[g].axis] = f.face[2 * gs[g].axis + 1] = g;
         f.flat = true;
         boxes.push_back(f);
     }
-    if (boxes.size() > (size_t)n / 2 || boxes.size() > (size_t)MAX_BOXES || !out.misc.empty()) return;
+    if (boxes.size() > (size_t)n / 2 || boxes.size() > (size_t)MAX_BOXES) return;
     out.nbox = ((int)boxes.size() + 1) / 2 * 2;
     out.outer = have_outer ? 1 : 0;
     out.box_scale = 4.f * scale;
@@ -859,6 +903,8 @@ rc_status load_scene(rc_ctx* ctx, const uint8_t* data, size_t n) {
     // once the global arrays are checked; the caller keeps its buffer until rc_sync)
     const bool async = (ctx->cfg.flags & RC_FLAG_LOAD_ASYNC) != 0;
     if (async && (s = ensure_side(ctx, S.NS))) return s;
+    struct Grouped { std::vector<float> T; std::vector<int> TQ; Groups G; };
+    std::vector<Grouped> grouped;
     for (int k = 0; k < S.NS; ++k) {
         HostState& hs = S.st[k];
         hs.inten = r.vec<float>(NL);
@@ -889,7 +935,17 @@ rc_status load_scene(rc_ctx* ctx, const uint8_t* data, size_t n) {
         float scene_scale = 0.f;
         for (int a = 0; a < 3; ++a)
             scene_scale = std::max(scene_scale, std::max(fabsf(S.grid.lo[a]), fabsf(S.grid.lo[a] + S.grid.ext[a])));
-        Groups G = build_groups(T, TQ, S.Nt, scene_scale);
+        // states often share their triangles (a lamp switched): grouped once
+        size_t same = 0;
+        auto equal = [&](const Grouped& x) {
+            return S.Nt == 0 || (memcmp(x.T.data(), T.data(), 4 * T.size()) == 0 && memcmp(x.TQ.data(), TQ.data(), 4 * TQ.size()) == 0);
+        };
+        while (same < grouped.size() && !equal(grouped[same])) ++same;
+        if (same == grouped.size()) {
+            grouped.push_back({T, TQ, {}});
+            grouped.back().G = build_groups(T, TQ, S.Nt, scene_scale);
+        }
+        Groups G = grouped[same].G;
         DState& d = hs.d;
         memset(&d, 0, sizeof d);
         d.nquad = build_quads(Q, dims, off, G.grp);
