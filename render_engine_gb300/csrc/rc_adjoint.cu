@@ -353,13 +353,15 @@ __global__ void __launch_bounds__(B) k_grad_final(const double* __restrict__ par
 int blocks_for(long long n) { return (int)((n + B - 1) / B); }
 int stride_blocks(long long n) { return (int)(std::min)((n + B - 1) / B, 152LL * 16); }
 
-cudaError_t scan_exclusive(const int* in, int* out, int n, int* scratch, cudaStream_t st) {
+cudaError_t scan_exclusive(const int* in, int* out, int n, int* scratch, cudaStream_t st, long long& launches) {
     const int nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     k_scan_tile<<<nb, B, 0, st>>>(in, out, n, scratch);
+    ++launches;
     if (nb > 1) {
-        cudaError_t e = scan_exclusive(scratch, scratch, nb, scratch + nb, st);
+        cudaError_t e = scan_exclusive(scratch, scratch, nb, scratch + nb, st, launches);
         if (e != cudaSuccess) return e;
         k_scan_add<<<blocks_for(n), B, 0, st>>>(out, n, scratch);
+        ++launches;
     }
     return cudaGetLastError();
 }
@@ -377,21 +379,22 @@ size_t scan_scratch_ints(long long n) {
     return s + 1;
 }
 
-cudaError_t build_transpose(const Bufs& b, int Np, int K, cudaStream_t st) {
+cudaError_t build_transpose(const Bufs& b, int Np, int K, cudaStream_t st, long long& launches) {
     const long long n = (long long)Np * K;
     cudaError_t e;
     if ((e = cudaMemsetAsync(b.cnt, 0, sizeof(int) * ((size_t)Np + 1), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(b.fill, 0, sizeof(int) * (size_t)Np, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(b.stats, 0, sizeof(Stats), st)) != cudaSuccess) return e;
     k_count<<<stride_blocks(n), B, 0, st>>>(b.hits, n, b.cnt, &b.stats->back);
-    if ((e = scan_exclusive(b.cnt, b.off, Np + 1, b.scratch, st)) != cudaSuccess) return e;
+    if ((e = scan_exclusive(b.cnt, b.off, Np + 1, b.scratch, st, launches)) != cudaSuccess) return e;
     k_fill<<<stride_blocks(n), B, 0, st>>>(b.hits, n, b.off, b.fill, b.unordered);
     k_rank<<<stride_blocks(n), B, 0, st>>>(b.hits, b.off, Np, b.unordered, K, n, b.src, &b.stats->max_incoming);
+    launches += 3;
     return cudaGetLastError();
 }
 
 cudaError_t solve(Bufs* bp, int Np, int K, int NL, int aes, const float* AE, const float* AEu, const float* em, int iters,
-                  cudaStream_t st) {
+                  cudaStream_t st, long long& launches) {
     const Bufs& b = *bp;
     cudaError_t e;
     k_prep<<<blocks_for(Np), B, 0, st>>>(AE, AEu, em, aes, NL, Np, b.da, b.g[0]);
@@ -426,14 +429,19 @@ cudaError_t solve(Bufs* bp, int Np, int K, int NL, int aes, const float* AE, con
         const Fwd f{b.hits, b.da, b.g[t & 1], b.L[t & 1], b.L[(t + 1) & 1], b.g[(t + 1) & 1], bo0, c0};
         const Bwd a{b.off, b.src, b.da, b.w, b.u[t & 1], b.u[(t + 1) & 1], bo1, c1};
         const int nb = blocks_for(Np), nf = last || !few[0] ? nb : 0, na = last || !few[1] ? nb : 0;
-        if (nf + na) k_sweep<<<nf + na, B, 0, st>>>(f, a, nf, K, Np, chg);
+        if (nf + na) {
+            k_sweep<<<nf + na, B, 0, st>>>(f, a, nf, K, Np, chg);
+            ++launches;
+        }
         if (!nf && !still[0]) {
             k_touch<<<touch_blocks, B, 0, st>>>(bi0, words, b.off, b.src, K, b.marks);
             k_fwd_few<<<nb, B, 0, st>>>(f, K, Np, b.marks);
+            launches += 2;
         }
         if (!na && !still[1]) {
             k_touch<<<touch_blocks, B, 0, st>>>(bi1, words, nullptr, b.hits, K, b.marks);
             k_bwd_few<<<nb, B, 0, st>>>(a, K, Np, b.marks);
+            launches += 2;
         }
         if (follow && (t & 1) && t + 3 < iters - 1) {   // read before sweep t + 3
             if ((e = cudaMemcpyAsync(b.host_counts + 2 * (t - 1), b.counts + 2 * (t - 1), 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, st)) !=
@@ -446,6 +454,7 @@ cudaError_t solve(Bufs* bp, int Np, int K, int NL, int aes, const float* AE, con
     bp->u_final = b.u[iters & 1];
     k_grad_part<<<dim3(GRAD_BLOCKS, (NL + 1 + COLS - 1) / COLS), B, 0, st>>>(AEu, aes, NL, Np, bp->u_final, b.w, bp->L_final, b.part);
     k_grad_final<<<NL + 1, B, 0, st>>>(b.part, GRAD_BLOCKS, b.stats->out);
+    launches += 3;   // with k_prep
     return cudaGetLastError();
 }
 

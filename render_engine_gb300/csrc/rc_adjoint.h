@@ -44,12 +44,12 @@ struct Bufs {
 
 size_t scan_scratch_ints(long long n);
 size_t bit_words(int Np);   // words of a bit per point
-// transposed ray lists from b.hits (also clears b.stats)
-cudaError_t build_transpose(const Bufs& b, int Np, int K, cudaStream_t st);
+// transposed ray lists from b.hits (also clears b.stats); adds the kernels launched to `launches`, as solve does
+cudaError_t build_transpose(const Bufs& b, int Np, int K, cudaStream_t st, long long& launches);
 // `iters` forward and adjoint Jacobi sweeps from L = 0, u = w, then the gradient against the
 // unit-emission direct light AEu (same gather-record layout as AE, `aes` floats per point)
 cudaError_t solve(Bufs* b, int Np, int K, int NL, int aes, const float* AE, const float* AEu, const float* em, int iters,
-                  cudaStream_t st);
+                  cudaStream_t st, long long& launches);
 
 }  // namespace adj
 }  // namespace rc

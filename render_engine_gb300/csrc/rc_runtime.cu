@@ -2361,25 +2361,24 @@ rc_status rc_adjoint(rc_ctx* ctx, const rc_adjoint_params* prm, const float* wei
     p.Np = S.Np;
     CKR(cudaMemcpyAsync(b.w, weights, Np * 4, cudaMemcpyHostToDevice, st));
     CKR(RC_DISPATCH(NL, frozen_hits(d, S.g, S.grid, ctx->c, p, prm->seed, prm->K, b.hits, st)));
-    int launched = 0;
+    ++ctx->launches;
     if (ctx->adj_aeu_state != prm->state) {
         // G_l, the direct light of every light at unit emission, depends only on the state's
         // geometry and the light positions: built once per state (no voxel masks)
         CKR(RC_DISPATCH(NL, build(ctx->NW, d, S.g, S.grid, S.L, ones, AEu, nullptr, S.Np, ctx->flags_dev, st)));
         ctx->adj_aeu_state = prm->state;
-        launched = 1;
+        ++ctx->launches;
     }
-    CKR(adj::build_transpose(b, S.Np, prm->K, st));
+    CKR(adj::build_transpose(b, S.Np, prm->K, st, ctx->launches));
     std::vector<DevBuf> tmp;
     struct TmpFree { std::vector<DevBuf>& p; ~TmpFree() { free_pool(p); } } tmp_free{tmp};
     const float* dem = nullptr;
     if (prm->emission && (s = dput(ctx, tmp, &dem, E))) return s;
     CKR(adj::solve(&b, S.Np, prm->K, NL, AES, reinterpret_cast<const float*>(d.AE), reinterpret_cast<const float*>(AEu), dem, iters,
-                   st));
+                   st, ctx->launches));
     adj::Stats hs{};
     CKR(cudaMemcpyAsync(&hs, b.stats, sizeof hs, cudaMemcpyDeviceToHost, st));
     CKR(cudaStreamSynchronize(st));
-    ctx->launches += 9 + launched + 2 * iters;
     double jg = 0.0;
     for (int l = 0; l < NL; ++l) {
         dJ_dE[l] = (float)hs.out[l];
@@ -2645,7 +2644,7 @@ rc_status rc_hg_camera_paths(rc_hg* hg, rc_ctx* ctx, int state, const rc_hg_path
     CKR(cudaStreamWaitEvent(ctx->stream, C.ready, 0));
     C.stride = (int)S1;
     C.npaths = np;
-    ctx->launches += rc::hg_has_voxels(hg) ? 5 : 4;
+    ctx->launches += 4;
     return RC_OK;
 }
 
