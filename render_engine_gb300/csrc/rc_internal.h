@@ -21,7 +21,10 @@ namespace rc {
 // against 461, and 485 with plain launches).  16 frames of 10.7 k points 217 -> 177 us, of 1.08 M
 // points 952 -> 906; 4 training steps of 65,536 points 258 -> 245.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// the same wait, with the pointer's loads behind it also where the compiler holds the data constant
+// The same wait, with the pointer's loads behind it also where the compiler holds the data constant or knows
+// that the asm cannot reach it: a __restrict__ parameter.  What a kernel of the chain writes is read through
+// such a pointer, and never through the non-coherent path (__ldg), which takes data that nobody writes during
+// the kernel's life, and that life begins before the wait.
 template <typename T>
 __device__ __forceinline__ T* pdl_wait(T* p) {
     asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");

@@ -2076,7 +2076,7 @@ __global__ void __launch_bounds__(BLOCK, 5) k_taa_pt(const DState s, const DStat
     extern __shared__ float4 sm[];
     stage_smem(sm, s);
     __syncthreads();
-    pdl_wait();
+    cur = pdl_wait(cur);
     const TraceSmem tsm = smem_view(sm, s);
     const int i = blockIdx.x * BLOCK + threadIdx.x;
     if (i >= p.Np) return;

@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int n
         };
         for (int i = tid; i < WF_BYTES / 16; i += TR_CHAIN) cp_async16(smem + 16 * i, a.wbf + 16 * i);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const float sc = __ldg(a.scale);   // loss scale (a power of two)
+        const float sc = __ldcg(pdl_wait(a.scale));   // loss scale (a power of two), written by the last step's Adam kernel
         auto point = [&](int it) {
             const int s = ((int)blockIdx.x + it * (int)gridDim.x) * 128 + row;
             return a.idx ? a.idx[s] : s;
@@ -709,6 +709,9 @@ __global__ void __launch_bounds__(128) k_mlp_adam(const float* __restrict__ gsum
     st = pdl_wait(st);
     gsum = pdl_wait(gsum);
     words = pdl_wait(words);
+    w = pdl_wait(w);
+    m1 = pdl_wait(m1);
+    m2 = pdl_wait(m2);
     const float4 s = __ldcg(reinterpret_cast<const float4*>(st));
     const bool skip = __ldcg(words + WD_NONFINITE) != 0u;
     const float scale = s.x, t = s.y + 1.f;

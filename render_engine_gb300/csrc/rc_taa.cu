@@ -150,12 +150,18 @@ __global__ void __launch_bounds__(B) k_post(const float* __restrict__ x, const i
     __shared__ double fin[B];
     __shared__ bool last;
     x = pdl_wait(x);
+    H = pdl_wait(H);
+    react = pdl_wait(react);
+    ref = pdl_wait(ref);
     const int i = blockIdx.x * B + threadIdx.x;
     float2 d2 = make_float2(0.f, 0.f);
     if (i < Np) {
         float s1 = 0.f, s2 = 0.f;
         int n = 0;
-        const int q = qid[i];
+        const int q = qid[i], rc = react[i];
+        float h = H[i];
+        const bool counted = ref && valid[i];
+        const float want = counted ? ref[i] : 0.f;
         if (q >= 0) {
             const int4 g = quad[q];   // first point, nu, nv
             const int r = i - g.x, iu = r % g.y, iv = r / g.y;
@@ -182,13 +188,11 @@ __global__ void __launch_bounds__(B) k_post(const float* __restrict__ x, const i
         const float sg = sqrtf(fmaxf(s2 / n - mu * mu, 0.f));
         mu_out[i] = mu;
         sg_out[i] = sg;
-        float h = H[i];
         if (gamma > 0.f) {
             const float lo = mu - gamma * sg, hi = mu + gamma * sg;
             h = fminf(fmaxf(h, lo), hi);
         }
         float a = alpha, target = x[i];
-        const int rc = react[i];
         if (rc > 0) {
             a = alpha_r;
             react[i] = rc - 1;
@@ -196,8 +200,8 @@ __global__ void __launch_bounds__(B) k_post(const float* __restrict__ x, const i
         }
         const float hn = h + a * (target - h);
         H2[i] = hn;
-        if (ref && valid[i]) {
-            const float e = hn - ref[i];
+        if (counted) {
+            const float e = hn - want;
             const float hi = __fmul_rn(e, e);
             d2 = make_float2(hi, __fmaf_rn(e, e, -hi));   // e^2 = hi + lo exactly
         }
