@@ -81,8 +81,15 @@ rc_status rc_mlp_weights(rc_mlp* m, float* host, size_t n, int to_device);
 /* The summed gradient of the last training step, same layout.  Synchronises the stream. */
 rc_status rc_mlp_gradients(rc_mlp* m, float* host, size_t n);
 
-/* Bit 0: a completion wait gave up.  Synchronises the stream. */
+/* Bit 0: a completion wait gave up.  Such a training step leaves the weights, the gradients and the loss
+ * scale as they were; an inference leaves the outputs of the tiles from there on unwritten.
+ * Synchronises the stream. */
 rc_status rc_mlp_error_flags(rc_mlp* m, unsigned* flags);
+
+/* Polls of a completion wait before it gives up, for the calls that follow; at most 2^24, the default.
+ * With 0 every wait gives up at once (and then waits for the product in flight all the same), a drill
+ * for the caller's handling of the error flag. */
+rc_status rc_mlp_wait_limit(rc_mlp* m, uint32_t polls);
 
 #ifdef __cplusplus
 }

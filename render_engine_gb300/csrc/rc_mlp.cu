@@ -106,6 +106,11 @@ constexpr int NWEIGHT = HID * K0 + 3 * HID * HID + OUTP * HID;   // 24,576
 __host__ __device__ constexpr int wf_off(int l) { return 2 * master_off(l); }   // byte offset of W_l's tile
 constexpr int WF_BYTES = 2 * NWEIGHT;                                           // 49,152
 
+// Words beside the training state: why this step's gradients must not be applied; blocks that have read
+// the state.
+enum MlpWord { WD_FAILED = 0, WD_TICKET, WD_COUNT };
+constexpr unsigned STEP_NONFINITE = 1u, STEP_GAVE_UP = 2u;   // a gradient is not finite; a wait gave up
+
 struct MlpArgs {
     const uint8_t* wbf;        // bf16 weight tiles
     const float4* P;           // point position (xyz)
@@ -123,6 +128,8 @@ struct MlpArgs {
     float* loss;               // training: sum of the relative L2 loss (for reporting)
     float loss_scale;          // 1 / (samples x n_out)
     const float* scale;        // training: the loss scale of this step (device, MlpState::SCALE)
+    unsigned* words;           // training: MlpWord
+    uint32_t polls;            // polls of a completion wait before it gives up
     unsigned* err;
 };
 
@@ -249,10 +256,14 @@ __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.ar
 __global__ void __launch_bounds__(IN_THREADS) k_mlp_infer(const MlpArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar[IN_CHAINS];
+    __shared__ volatile int gave_up[IN_CHAINS];
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int i = tid; i < WF_BYTES / 16; i += IN_THREADS) reinterpret_cast<uint4*>(smem)[i] = reinterpret_cast<const uint4*>(a.wbf)[i];
-    if (tid < IN_CHAINS) mbar_init(&mbar[tid], 1);
+    if (tid < IN_CHAINS) {
+        mbar_init(&mbar[tid], 1);
+        gave_up[tid] = 0;
+    }
     if (warp == 0) tmem_alloc(&tmem_base, 64u * IN_CHAINS);
     fence_proxy_async();
     fence_before_sync();
@@ -286,13 +297,16 @@ __global__ void __launch_bounds__(IN_THREADS) k_mlp_infer(const MlpArgs a) {
         uint32_t phase = 0;
         bool ok = true;
         // One warp of the chain watches the barrier, the others wait for it without issuing (all warps
-        // polling took 229 us where this took 141).  A wait that gives up is the last one: the chain
-        // goes on through its barriers, so that nobody waits for it, and stores no more outputs.
+        // polling took 229 us where this took 141).  A wait that gives up raises the error flag, and the
+        // chain stores no more outputs (its warps read that behind the barrier).  The product in flight is
+        // waited for once more, so that nothing is overwritten or freed under it; if that gives up too,
+        // no more products are issued, and the chain goes on through its barriers, so that nobody waits for it.
         auto wait = [&]() {
             if (quarter == 0) {
-                if (ok && !mbar_wait(&mbar[c], phase, WAIT_LIMIT)) {
-                    ok = false;
-                    if (lane == 0) atomicOr(a.err, 1u);
+                if (ok && !mbar_wait(&mbar[c], phase, a.polls)) {
+                    gave_up[c] = 1;
+                    atomicOr(a.err, 1u);
+                    ok = mbar_wait(&mbar[c], phase, WAIT_LIMIT);
                 }
                 fence_before_sync();
             }
@@ -343,7 +357,7 @@ __global__ void __launch_bounds__(IN_THREADS) k_mlp_infer(const MlpArgs a) {
             float v[16];
             tmem_ld16(acc, v);
             tmem_wait_ld();
-            if (s < a.n && ok) {
+            if (s < a.n && !gave_up[c]) {
                 float* o = a.out + (size_t)s * a.ostride;
 #pragma unroll
                 for (int j = 0; j < OUTP; ++j)
@@ -427,11 +441,15 @@ enum TrainBar { TB_CHAIN = 1, TB_FULL = 2, TB_EMPTY = 4 };
 __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int ntiles) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar;
+    __shared__ volatile int gave_up, lost;
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int W_ENCODE = TR_CHAIN / 32, W_ISSUE = (TR_CHAIN + TR_ENCODE) / 32;
     pdl_release();
-    if (tid == 0) mbar_init(&mbar, 1);
+    if (tid == 0) {
+        mbar_init(&mbar, 1);
+        gave_up = lost = 0;
+    }
     if (warp == W_ISSUE) tmem_alloc(&tmem_base, TR_COLS);
     fence_before_sync();
     __syncthreads();
@@ -448,9 +466,10 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int n
             bar_sync(TB_FULL + (it & 1), TR_ENCODE + 32);
 #pragma unroll 1
             for (int l = 0; l < NLAYER; ++l) {
+                const bool stop = lost;   // (read while it would wait anyway; at most one product more is issued)
                 if (l > 0) bar_sync(TB_CHAIN, TR_CHAIN + 32);
                 fence_after_sync();
-                if (lane == 0) {
+                if (lane == 0 && !stop) {
                     const uint32_t K = (uint32_t)in_dim(l);
                     mma_chain(tmem + TR_DA, smem_desc(sm0 + (l == 0 ? xbuf(it) : hbuf(l)), 128u, 16u * K), 256u,
                               smem_desc(sm0 + wf_off(l), 128u, 16u * K), 256u, (int)K / 16, idesc_bf16_f32(128, out_dim(l)), true);
@@ -460,9 +479,10 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int n
             }
 #pragma unroll 1
             for (int l = NLAYER - 1; l >= 0; --l) {
+                const bool stop = lost;
                 bar_sync(TB_CHAIN, TR_CHAIN + 32);
                 fence_after_sync();
-                if (lane == 0) {
+                if (lane == 0 && !stop) {
                     const uint32_t Kin = (uint32_t)in_dim(l), Nout = (uint32_t)out_dim(l);
                     const uint32_t z = sm0 + (l == 4 ? (uint32_t)TS_DY : (l == 3 ? (uint32_t)TS_E : hbuf(l + 2)));
                     if (l >= 1) {
@@ -501,12 +521,18 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int n
         const uint32_t acc = tmem + TR_DA + ((uint32_t)(quarter * 32) << 16);
         uint32_t phase = 0;
         bool ok = true;
-        // Every warp watches the barrier itself.  A wait that gives up is the last one: the chain goes
-        // on through its barriers, so that nobody waits for it, and the error flag stays set.
+        // Every warp watches the barrier itself.  A wait that gives up raises the error flag and marks the
+        // step failed: no gradients leave this CTA, and Adam leaves weights and state alone.  The product in
+        // flight is waited for once more, so that nothing is overwritten or freed under it; if that gives up
+        // too, no more products are issued, and the chain goes on through its barriers, so that nobody
+        // waits for it.
         auto wait = [&]() {
-            if (ok && !mbar_wait(&mbar, phase, WAIT_LIMIT)) {
-                ok = false;
-                if (lane == 0) atomicOr(a.err, 1u);
+            if (ok && !mbar_wait(&mbar, phase, a.polls)) {
+                gave_up = 1;
+                atomicOr(a.err, 1u);
+                atomicOr(a.words + WD_FAILED, STEP_GAVE_UP);
+                ok = mbar_wait(&mbar, phase, WAIT_LIMIT);
+                if (!ok) lost = 1;
             }
             phase ^= 1u;
             fence_after_sync();
@@ -579,7 +605,7 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int n
                     handover();
                     if (half == 0) {
                         for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-                        if (lane == 0 && lsum != 0.f) atomicAdd(a.loss, lsum);
+                        if (lane == 0 && ok && lsum != 0.f) atomicAdd(a.loss, lsum);
                     }
                 }
             }
@@ -616,7 +642,7 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(const MlpArgs a, int n
     __syncthreads();
     fence_after_sync();
     // the CTA's weight gradients: rows = outputs 0..63, in the lanes of the warps 0 and 1 of each four
-    if (warp < W_ISSUE && (warp & 3) < 2) {
+    if (warp < W_ISSUE && (warp & 3) < 2 && !gave_up) {
         const int row = (warp & 3) * 32 + lane;
         float* dw = a.dwpart + (size_t)blockIdx.x * NWEIGHT;
         int piece = 0;
@@ -662,9 +688,6 @@ __global__ void k_mlp_pack(const float* __restrict__ w, uint8_t* __restrict__ wb
 enum MlpState { ST_SCALE = 0, ST_STEPS, ST_RUN, ST_SKIPPED, ST_COUNT };
 constexpr float SCALE_MAX = 65536.f;
 constexpr int SCALE_RUN = 1000;
-// words beside the state: a gradient of this step is not finite; blocks that have read the state
-enum MlpWord { WD_NONFINITE = 0, WD_TICKET, WD_COUNT };
-
 // Gradient of each weight = the CTAs' gradients added in a fixed order (reproducible): slice s
 // of GSLICES adds CTAs s, s + GSLICES, ... in order, then the slices are added in order.  A block
 // sums 64 weights, one thread per four weights and slice, all of a thread's loads in flight.
@@ -694,10 +717,11 @@ __global__ void __launch_bounds__(GSLICES * GWEIGHTS / 4) k_mlp_gsum(const float
 #pragma unroll
     for (int k = 0; k < GSLICES; ++k) sum += slice[k][threadIdx.x];
     gsum[blockIdx.x * GWEIGHTS + threadIdx.x] = sum;
-    if (!isfinite(sum)) atomicOr(words + WD_NONFINITE, 1u);
+    if (!isfinite(sum)) atomicOr(words + WD_FAILED, STEP_NONFINITE);
 }
 
-// One Adam step on the FP32 master weights, and their bf16 copies; the loss scale's step.  Every
+// One Adam step on the FP32 master weights, and their bf16 copies; the loss scale's step.  A step of which
+// a wait gave up changes nothing.  Every
 // thread reads the state of before the step and forms Adam's bias corrections 1 / (1 - b^t) itself,
 // in FP32 (a double pow is a long chain of the GPU's slow FP64 operations); the last block to have
 // read the state writes the next one.
@@ -713,7 +737,8 @@ __global__ void __launch_bounds__(128) k_mlp_adam(const float* __restrict__ gsum
     m1 = pdl_wait(m1);
     m2 = pdl_wait(m2);
     const float4 s = __ldcg(reinterpret_cast<const float4*>(st));
-    const bool skip = __ldcg(words + WD_NONFINITE) != 0u;
+    const unsigned failed = __ldcg(words + WD_FAILED);
+    const bool skip = failed != 0u;
     const float scale = s.x, t = s.y + 1.f;
     if (i < NWEIGHT && !skip) {
         const float c1 = 1.f / (1.f - powf(b1, t)), c2 = 1.f / (1.f - powf(b2, t));
@@ -732,9 +757,11 @@ __global__ void __launch_bounds__(128) k_mlp_adam(const float* __restrict__ gsum
     __threadfence();
     if (atomicAdd(words + WD_TICKET, 1u) != gridDim.x - 1) return;
     words[WD_TICKET] = 0u;
-    words[WD_NONFINITE] = 0u;   // ready for the next step
+    words[WD_FAILED] = 0u;   // ready for the next step
     float4 n = s;
-    if (skip) {
+    if (failed & STEP_GAVE_UP) {
+        // (not a matter of the scale)
+    } else if (skip) {
         n.x = fmaxf(scale * 0.5f, 1.f);
         n.z = 0.f;
         n.w += 1.f;
@@ -780,6 +807,7 @@ struct rc_mlp {
     unsigned* err = nullptr;
     unsigned* words = nullptr;  // MlpWord
     int cap_tiles = 0, sms = 0;
+    uint32_t polls = WAIT_LIMIT;
     long long step = 0;
     std::string msg;
 };
@@ -800,6 +828,7 @@ MlpArgs args_of(const rc_mlp* m) {
         a.inv_ext[k] = 1.f / (m->cfg.box_hi[k] - m->cfg.box_lo[k]);
     }
     a.err = m->err;
+    a.polls = m->polls;
     return a;
 }
 
@@ -916,6 +945,7 @@ rc_status rc_mlp_train(rc_mlp* m, const float* d_pos4, const float* d_nrm4, cons
     a.loss = d_loss ? d_loss : m->loss;
     a.loss_scale = 1.f / ((float)n * (float)m->cfg.n_out);
     a.scale = m->state + ST_SCALE;
+    a.words = m->words;
     const int ntiles = n / 128, ctas = std::min(ntiles, m->sms);
     m->step++;
     const float b1 = 0.9f, b2 = 0.99f;
@@ -951,6 +981,12 @@ rc_status rc_mlp_loss_scale(rc_mlp* m, float* scale, long long* steps, long long
     if (scale) *scale = st[ST_SCALE];
     if (steps) *steps = (long long)st[ST_STEPS];
     if (skipped) *skipped = (long long)st[ST_SKIPPED];
+    return RC_OK;
+}
+
+rc_status rc_mlp_wait_limit(rc_mlp* m, uint32_t polls) {
+    if (!m || polls > WAIT_LIMIT) return mfail(m, RC_ERR_ARG, "wait limit: at most 2^24 polls");
+    m->polls = polls;
     return RC_OK;
 }
 

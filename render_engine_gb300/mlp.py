@@ -12,7 +12,7 @@ import numpy as np
 from . import native
 
 EXPORTS = ["rc_mlp_tile_product", "rc_mlp_wait_check", "rc_mlp_create", "rc_mlp_destroy", "rc_mlp_last_error", "rc_mlp_train", "rc_mlp_infer",
-           "rc_mlp_weights", "rc_mlp_gradients", "rc_mlp_error_flags", "rc_mlp_loss_scale"]
+           "rc_mlp_weights", "rc_mlp_gradients", "rc_mlp_error_flags", "rc_mlp_wait_limit", "rc_mlp_loss_scale"]
 NWEIGHT = 24576
 LAYERS = [(176, 64), (64, 64), (64, 64), (64, 64), (64, 16)]   # (inputs, outputs)
 
@@ -43,6 +43,7 @@ def _lib():
         L.rc_mlp_weights.argtypes = [vp, vp, ctypes.c_size_t, i]
         L.rc_mlp_gradients.argtypes = [vp, vp, ctypes.c_size_t]
         L.rc_mlp_error_flags.argtypes = [vp, ctypes.POINTER(ctypes.c_uint)]
+        L.rc_mlp_wait_limit.argtypes = [vp, ctypes.c_uint32]
         L.rc_mlp_loss_scale.argtypes = [vp, ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_longlong),
                                         ctypes.POINTER(ctypes.c_longlong)]
         _bound = True
@@ -142,6 +143,10 @@ class Mlp:
         g = np.empty(NWEIGHT, np.float32)
         self._chk(self.L.rc_mlp_gradients(self.h, g.ctypes.data_as(ctypes.c_void_p), g.size))
         return g
+
+    def wait_limit(self, polls: int):
+        """Polls of a completion wait before it gives up, for the calls that follow (at most 2^24, the default)."""
+        self._chk(self.L.rc_mlp_wait_limit(self.h, polls))
 
     def error_flags(self) -> int:
         f = ctypes.c_uint()
