@@ -986,6 +986,10 @@ rc_status load_scene(rc_ctx* ctx, const uint8_t* data, size_t n) {
         d.nmisc = (int)G.misc.size();
         d.gr = G.gr;
         size_t smem = frame_smem_bytes(d);
+        if (smem > 200 * 1024 && d.nquad) {   // the quads' records are an aid that many triangles leave no room for
+            d.nquad = 0;
+            smem = frame_smem_bytes(d);
+        }
         if (smem > 200 * 1024) return fail(ctx, RC_ERR_UNSUPPORTED, "%d dynamic triangles exceed shared memory", S.Nt);
         if (k == 0) {
             // state 0's build (where runs usually begin) starts on the side stream as soon as its
