@@ -206,7 +206,7 @@ __device__ __forceinline__ void mark_segment(const HgDev& c, uint32_t (&m)[3], c
     const uint32_t M = fixed ? (uint32_t)(mg * ONE) + 1u : 0u, lim = fixed ? M << 6 : 0xffffffffu;
     uint32_t late0 = 0u, late1 = 0u;   // the samples left to the exact evaluation, n <= 48
     uint32_t i0 = 0u;
-    if (START_MARKED && tmin == 0.f) {
+    if (START_MARKED && fixed && tmin == 0.f) {   // (an infinite d: a + d 0 is not a)
         i0 = 1u;
         z[0] += dz[0];
         z[1] += dz[1];
