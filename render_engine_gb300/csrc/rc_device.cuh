@@ -180,21 +180,31 @@ __device__ __forceinline__ f3 cosine_dir(f3 N, float u1, float u2) {
 // Möller-Trumbore of one triangle, the reference's expression order (poc_gpu.cu:203-217).
 // Accepts when t is smaller, or equal with a smaller triangle index: over any visiting order
 // this selects what the reference's in-order scan selects.
+//
+// Every operation is written with its rounding, as the compiler contracts the plain expressions in the full
+// scan: several kernels hold several copies of this test (the scan, the filter's exact test, the shared
+// scan), and a ray through an edge or a diagonal, where u, v or u + v lies within a rounding of 0 or 1,
+// must get the same answer from each of them.
+__device__ __forceinline__ float mt_cross1(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }   // a b - c d
+__device__ __forceinline__ f3 mt_cross(f3 a, f3 b) {
+    return mk(mt_cross1(a.y, b.z, a.z, b.y), mt_cross1(a.z, b.x, a.x, b.z), mt_cross1(a.x, b.y, a.y, b.x));
+}
+__device__ __forceinline__ float mt_dot(f3 a, f3 b) { return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y))); }
 __device__ __forceinline__ void mt_tri(const float4* __restrict__ tri, int j, f3 o, f3 d,
                                        float& tmin, int& q, int& jbest) {
     const float4 A = tri[3 * j], B = tri[3 * j + 1], C = tri[3 * j + 2];
     const f3 v0 = xyz(A), e1 = xyz(B), e2 = xyz(C);
-    f3 p = cross(d, e2);
-    float det = dot(e1, p);
+    const f3 p = mt_cross(d, e2);
+    const float det = mt_dot(e1, p);
     if (fabsf(det) <= 1e-9f) return;
-    float inv = 1.f / det;
-    f3 tv = o - v0;
-    float u = dot(tv, p) * inv;
+    const float inv = __fdiv_rn(1.f, det);
+    const f3 tv = mk(__fsub_rn(o.x, v0.x), __fsub_rn(o.y, v0.y), __fsub_rn(o.z, v0.z));
+    const float u = __fmul_rn(__fmaf_rn(tv.z, p.z, __fmaf_rn(tv.y, p.y, __fmul_rn(tv.x, p.x))), inv);
     if (u < 0.f) return;
-    f3 qv = cross(tv, e1);
-    float v = dot(d, qv) * inv;
-    if (v < 0.f || u + v > 1.f) return;
-    float t = dot(e2, qv) * inv;
+    const f3 qv = mt_cross(tv, e1);
+    const float v = __fmul_rn(mt_dot(d, qv), inv);
+    if (v < 0.f || __fadd_rn(u, v) > 1.f) return;
+    const float t = __fmul_rn(mt_dot(e2, qv), inv);
     if (t > 1e-4f && (t < tmin || (t == tmin && j < jbest))) { tmin = t; q = __float_as_int(A.w); jbest = j; }
 }
 
