@@ -197,7 +197,7 @@ __device__ __forceinline__ void mt_tri(const float4* __restrict__ tri, int j, f3
     const f3 p = mt_cross(d, e2);
     const float det = mt_dot(e1, p);
     if (fabsf(det) <= 1e-9f) return;
-    const float inv = __fdiv_rn(1.f, det);
+    const float inv = __frcp_rn(det);
     const f3 tv = mk(__fsub_rn(o.x, v0.x), __fsub_rn(o.y, v0.y), __fsub_rn(o.z, v0.z));
     const float u = __fmul_rn(__fmaf_rn(tv.z, p.z, __fmaf_rn(tv.y, p.y, __fmul_rn(tv.x, p.x))), inv);
     if (u < 0.f) return;

@@ -291,6 +291,7 @@ __device__ __forceinline__ void trace_groups(const float4* __restrict__ tri, con
             if (sd > GL.w) jend = j + 1;
             else if (sd < -GL.w) j = j + 1;
         }
+#pragma unroll 1
         for (; j < jend; ++j) mt_tri(tri, j, o, d, tmin, q, jb);
         thr = tmin * 1.0001f + 1e-5f;
     }
@@ -435,6 +436,7 @@ static __device__ __forceinline__ float2 scan_lanes(const float4* __restrict__ t
         const f3 sd = mk(__shfl_sync(act, d.x, src), __shfl_sync(act, d.y, src), __shfl_sync(act, d.z, src));
         float t = __int_as_float(0x7f800000);
         int tq = -1, j1 = 0x7fffffff;
+#pragma unroll 1
         for (int j = rank; j < nt; j += n) mt_tri(tri, j, so, sd, t, tq, j1);
         const unsigned best = __reduce_min_sync(act, __float_as_uint(t));
         const unsigned at = __reduce_min_sync(act, __float_as_uint(t) == best ? (unsigned)j1 : 0x7fffffffu);
@@ -454,12 +456,16 @@ static __device__ __noinline__ float2 trace_filter(const float4* tri, const floa
                                                    f3 o, f3 d) {
     float tmin = __int_as_float(0x7f800000);
     int q = -1, jb = 0x7fffffff;
+#pragma unroll 1
     for (int k = 0; k < nmisc; ++k) mt_tri(tri, misc[k], o, d, tmin, q, jb);
     if (ng <= 32) trace_groups<unsigned>(tri, grp, ng, gr, o, d, tmin, q, jb);
     else trace_groups<unsigned long long>(tri, grp, ng, gr, o, d, tmin, q, jb);
     return make_float2(tmin, __int_as_float(q));
 }
 
+// The loops over triangles around the exact test are kept rolled: most rays make a turn or two of one of them,
+// and unrolled their loads cost the kernels' hot paths registers (fused frames of 1,082,802 points, 3 lights: 52
+// bytes spilt and 945 us for 16, rolled 12 and 898; a turned door's filter 68 bytes and 4).
 // Closest dynamic-triangle hit, equal to the reference's in-order scan (poc_gpu.cu:199-220).
 // States made of boxes go through trace_boxes, and the few rays that it cannot decide through the
 // scan itself.  The plane filter takes other states, and warps with many undecided rays: pass 1 marks the groups whose plane crossing
@@ -471,6 +477,7 @@ __device__ __forceinline__ void trace_dyn(const TraceSmem& sm, const DState& s, 
     q = -1;
     if (brute || s.ng == 0) {
         int jb = 0x7fffffff;
+#pragma unroll 1
         for (int j = 0; j < s.nt; ++j) mt_tri(sm.tri, j, o, d, tmin, q, jb);
         return;
     }
@@ -777,8 +784,8 @@ __device__ __forceinline__ Hit trace_resolve(const TraceSmem& sm, const DState& 
 
 // What the trace reads of a state's geometry goes to shared memory once per block: the group buffer,
 // the triangles and the triangles outside any group.  (Box states need groups and triangles for undecided rays
-// only; 5 KB of a 31-rectangle room.  They cost 8 lights' frames 3 %, in L1 capacity, and 3 lights' 1 %; without them the
-// undecided rays' loads wait for the L2, see SCAN_LANES.)
+// only: 5 KB of a 31-rectangle room, 1 to 3 % of a frame in L1 capacity.  Without them the undecided rays' loads
+// wait for the L2, see SCAN_LANES.)
 __device__ __forceinline__ void stage_smem(float4* sm, const DState& s) {
     const int nt = 3 * s.nt, nr = grp_float4s(s);
     for (int j = threadIdx.x; j < nr; j += blockDim.x) sm[j] = s.grp[j];
@@ -1740,8 +1747,8 @@ __device__ __forceinline__ float shadow_t(const TraceSmem& sm, const DState& s, 
     return q == -1 ? INFINITY : t;
 }
 
-// Four blocks an SM (64 registers; 52 bytes spilt at 3 lights): a 1080p pass of two bounces 1410 us with three,
-// 1380 with four; 1456 since the plane filter is a call, which the two traces of a vertex pay for.
+// Four blocks an SM (64 registers; 88 bytes spilt at 3 lights): a 1080p pass of two bounces 1410 us with three,
+// 1380 with four; 1394 since the plane filter is a call, which the two traces of a vertex pay for.
 template <int NL>
 __global__ void __launch_bounds__(BLOCK, 4) k_paths(const DState s, const DStatic g, const Grid grid, const DevCache c, const FrameParams p,
                                                  const CameraD cam, const PathD pd, float* __restrict__ pos, float* __restrict__ nrm,
