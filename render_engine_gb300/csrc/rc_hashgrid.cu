@@ -372,40 +372,40 @@ template <bool WIDE>
 __device__ __forceinline__ void vox_slot(const HgDev& c, const VoxDev& g, const rc_hg_vertex* __restrict__ v, const int* __restrict__ plen,
                                          int stride, long long j, unsigned long long* __restrict__ vox) {
     const int res = g.res;
-            const long long p = j / stride;
-            if (j - p * stride >= plen[p]) return;
-            const rc_hg_vertex x = load_vertex<WIDE>(v + j);
-            if ((x.flags & RC_HG_MISS) || x.light_index < 0 || x.light_index >= 64 || !(x.flags & RC_HG_LIGHT_VISIBLE)) return;
-            const unsigned long long bit = 1ull << x.light_index;
-            const float r = mn(x.light_dist, c.td);
-            float a[3], d[3];
+    const long long p = j / stride;
+    if (j - p * stride >= plen[p]) return;
+    const rc_hg_vertex x = load_vertex<WIDE>(v + j);
+    if ((x.flags & RC_HG_MISS) || x.light_index < 0 || x.light_index >= 64 || !(x.flags & RC_HG_LIGHT_VISIBLE)) return;
+    const unsigned long long bit = 1ull << x.light_index;
+    const float r = mn(x.light_dist, c.td);
+    float a[3], d[3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                a[k] = x.hit[k];
-                d[k] = __fmul_rn(x.to_light[k], r);
-            }
-            unsigned last = ~0u;   // consecutive samples in one voxel mark it once (res <= 256: 24-bit indexes)
+    for (int k = 0; k < 3; ++k) {
+        a[k] = x.hit[k];
+        d[k] = __fmul_rn(x.to_light[k], r);
+    }
+    unsigned last = ~0u;   // consecutive samples in one voxel mark it once (res <= 256: 24-bit indexes)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                unsigned vi[10];
-                bool on[10];
-                unsigned long long w[10];
+    for (int h = 0; h < 2; ++h) {
+        unsigned vi[10];
+        bool on[10];
+        unsigned long long w[10];
 #pragma unroll
-                for (int k = 0; k < 10; ++k) {
-                    const float t = c_seg19[10 * h + k];
-                    const int ix = vox_axis(__fadd_rn(a[0], __fmul_rn(d[0], t)), g.lo[0], g.scale[0], res);
-                    const int iy = vox_axis(__fadd_rn(a[1], __fmul_rn(d[1], t)), g.lo[1], g.scale[1], res);
-                    const int iz = vox_axis(__fadd_rn(a[2], __fmul_rn(d[2], t)), g.lo[2], g.scale[2], res);
-                    vi[k] = (unsigned)((iz * res + iy) * res + ix);
-                    on[k] = vi[k] != last;
-                    last = vi[k];
-                }
+        for (int k = 0; k < 10; ++k) {
+            const float t = c_seg19[10 * h + k];
+            const int ix = vox_axis(__fadd_rn(a[0], __fmul_rn(d[0], t)), g.lo[0], g.scale[0], res);
+            const int iy = vox_axis(__fadd_rn(a[1], __fmul_rn(d[1], t)), g.lo[1], g.scale[1], res);
+            const int iz = vox_axis(__fadd_rn(a[2], __fmul_rn(d[2], t)), g.lo[2], g.scale[2], res);
+            vi[k] = (unsigned)((iz * res + iy) * res + ix);
+            on[k] = vi[k] != last;
+            last = vi[k];
+        }
 #pragma unroll
-                for (int k = 0; k < 10; ++k) w[k] = on[k] ? __ldcg(vox + vi[k]) : bit;
+        for (int k = 0; k < 10; ++k) w[k] = on[k] ? __ldcg(vox + vi[k]) : bit;
 #pragma unroll
-                for (int k = 0; k < 10; ++k)
-                    if (!(w[k] & bit)) atomicOr(vox + vi[k], bit);
-            }
+        for (int k = 0; k < 10; ++k)
+            if (!(w[k] & bit)) atomicOr(vox + vi[k], bit);
+    }
 }
 template <bool WIDE>
 __global__ void __launch_bounds__(HG_BLOCK) k_vox_mark(const HgDev c, const VoxDev g, const rc_hg_vertex* __restrict__ v,
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(HG_BLOCK) k_vox_mark(const HgDev c, const VoxD
 // Both marks of a pass of camera paths: of every 1 + stride blocks the first marks the masks of 256
 // paths, the others the voxels of 256 slots each.  The two do not depend on each other; the first is
 // bound by its instructions, the second by the L2, and side by side on a multiprocessor they take
-// 40 us less of 1920 x 1080 three-vertex paths (1398 us a pass; 1438 with a launch each).  Four blocks an
+// 40 us less of 1920 x 1080 three-vertex paths (1398 us a pass when it was made, 1438 with a launch each).  Four blocks an
 // SM (64 registers) for this kernel and for k_hg_mark: 1462 us at three, 1406 at five.  Adding the
 // samples (k_hg_accum) in the same launch: 1414.
 template <bool WIDE>

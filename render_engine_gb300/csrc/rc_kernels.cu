@@ -421,9 +421,9 @@ __device__ __forceinline__ bool trace_boxes(const TraceSmem& sm, const DState& s
 // warp about 200 instructions; on its own lane, through the plane filter, it made the warp the
 // last of a small frame by 8 us (10,728 points: 20 us instead of 12).  From more than SCAN_LANES such lanes on
 // (rows of points inside, behind or close beside a wall, cameras outside the room) each goes through the plane
-// filter.  20 frames of a room whose walls stand through its enclosing box, 1,082,802 points: 1174 us; 1355
+// filter.  20 frames of a room whose walls stand through its enclosing box, 1,082,802 points: 1135 us; 1360
 // when the triangles came from the L2 and more than 14 lanes scanned each for itself; 1430 with the plane filter
-// alone.  A room of 0.8 x 0.4 x 0.3, 200,000 points: 334, 619 and 425.
+// alone.  A room of 0.8 x 0.4 x 0.3, 200,000 points: 318, 621 and 422.
 constexpr int SCAN_LANES = 8;
 static __device__ __forceinline__ float2 scan_lanes(const float4* __restrict__ tri, int nt, unsigned act, unsigned need, f3 o, f3 d, float tmin,
                                                  int q) {
@@ -2076,7 +2076,7 @@ __global__ void __launch_bounds__(BLOCK, NL <= 8 ? 4 : 2) k_ref(const DState s, 
 // ray; the radiance at its hit point = A x (direct light summed over lights + the converged
 // reference), 0 when the ray does not count; with DEPS the ray's dependency mask (the hit's
 // shadow voxels and the ray's own transit voxels) is or-ed into cur.
-// Five blocks an SM (48 registers): 24 frames of 1,082,802 points 2348 us, 2402 with four.
+// Five blocks an SM (48 registers): 24 frames of 1,082,802 points 2.2 % less than with four.
 template <int NL, int NW, bool DEPS>
 __global__ void __launch_bounds__(BLOCK, 5) k_taa_pt(const DState s, const DStatic g, const Grid grid, const DevCache c, const FrameParams p,
                                                   float* __restrict__ x, uint32_t* __restrict__ cur, uint32_t seed, uint32_t frame) {
